@@ -257,17 +257,53 @@ __global__ void __launch_bounds__(256) k_raygen(const __grid_constant__ Params p
 // Node and triangle visits a lane makes between two refills of the warp's finished lanes.
 constexpr int kTravBudget = 8;
 
-// Warp-aggregated refill from a queue: every lane with busy == false takes the next entry
-// index (one atomic per warp); lanes left without an entry get idx >= n.  `drained` (warp
-// uniform) records that the queue is exhausted.
-__device__ __forceinline__ uint32_t refill(bool busy, uint32_t* cursor, uint32_t n, bool& drained) {
-    const unsigned lane = threadIdx.x & 31u;
+// Where a warp of a persistent traversal launch takes its queue entries from: runs of kRun entries,
+// the first one its own (no atomic: a queue of up to one run per warp is handed out without any),
+// later ones from the launch's cursor with one global atomic each.  Taking entries one refill at a
+// time made every warp of the GPU queue up on the cursor's cache line (about 8 entries per
+// atomic).  Shorter first runs that spread a short queue over more warps shorten a lone launch
+// (46 k rays of a 20 k-triangle mesh: 50 -> 40 us) but cost issue slots when several lanes'
+// launches share the GPU (4.9 M-path pass over 328 k triangles: 4.58 -> 4.82 ms).
+struct Feed {
+    uint32_t cur, end;        // the warp's entries not handed out yet (warp uniform)
+    uint32_t own;             // entries handed out without the cursor
+    bool drained;             // the queue ends at `end`
+};
+constexpr uint32_t kRun = 32;
+__device__ __forceinline__ Feed feed_init(uint32_t n) {
+    const uint32_t w = blockIdx.x * (kTraceBlock / 32u) + (threadIdx.x >> 5);
+    Feed f;
+    f.cur = min(n, w * kRun);
+    f.end = min(n, f.cur + kRun);
+    f.own = gridDim.x * (kTraceBlock / 32u) * kRun;
+    f.drained = f.own >= n;
+    return f;
+}
+// Every lane with busy == false takes an entry; false: none is left for this lane.
+__device__ __forceinline__ bool refill(Feed& f, bool busy, uint32_t* cursor, uint32_t n, uint32_t& idx) {
     const unsigned idle = __ballot_sync(kFull, !busy);
-    uint32_t base = 0;
-    if (lane == 0) base = atomicAdd(cursor, (uint32_t)__popc(idle));
-    base = __shfl_sync(kFull, base, 0);
-    if (base + (uint32_t)__popc(idle) >= n) drained = true;
-    return base + (uint32_t)__popc(idle & lanemask_lt());
+    const uint32_t want = (uint32_t)__popc(idle), have = f.end - f.cur;
+    const uint32_t rank = (uint32_t)__popc(idle & lanemask_lt());
+    idx = f.cur + rank;
+    bool got = rank < have;
+    if (want <= have) {
+        f.cur += want;
+    } else {
+        f.cur = f.end;
+        if (!f.drained) {
+            uint32_t base = 0;
+            if ((threadIdx.x & 31u) == 0) base = f.own + atomicAdd(cursor, kRun);
+            base = min(n, __shfl_sync(kFull, base, 0));
+            f.end = min(n, base + kRun);
+            f.drained = f.end >= n;
+            if (!got) {
+                idx = base + (rank - have);
+                got = idx < f.end;
+            }
+            f.cur = min(f.end, base + (want - have));
+        }
+    }
+    return got && !busy;
 }
 
 // Closest hit of each queued ray.  Persistent warps; a lane whose ray is done takes the next
@@ -282,16 +318,17 @@ __global__ void __launch_bounds__(kTraceBlock, kTraceMinBlocks) k_extend(const _
     const uint32_t* q = p.wave.q[depth & 1];
     uint32_t* cursor = &p.wave.counters[cur_ext(depth)];
     if (blockIdx.x == 0 && threadIdx.x == 0) atomicAdd(&p.wave.stats[0], (unsigned long long)n);
-    bool busy = false, drained = false;
+    bool busy = false;
+    Feed feed = feed_init(n);
     uint32_t slot = 0;
     float tfar = 0.f;
     const SceneDev* sc = &p.scene;
     WRay r;
     Trav st;
     for (;;) {
-        if (!drained && __any_sync(kFull, !busy)) {
-            const uint32_t idx = refill(busy, cursor, n, drained);
-            if (!busy && idx < n) {
+        if ((!feed.drained || feed.cur < feed.end) && __any_sync(kFull, !busy)) {
+            uint32_t idx;
+            if (refill(feed, busy, cursor, n, idx)) {
                 slot = depth == 0 ? idx : q[idx];
                 const FilmDev* film = &p.film;
                 if constexpr (kMulti) {
@@ -328,16 +365,20 @@ __global__ void __launch_bounds__(kTraceBlock, kTraceMinBlocks) k_shadow(const _
     uint32_t* cursor = &p.wave.counters[cur_sh(depth)];
     const size_t rs = p.wave.capacity;          // record stride: records are [bounce][slot]
     if (blockIdx.x == 0 && threadIdx.x == 0) atomicAdd(&p.wave.stats[1], (unsigned long long)n);
-    unsigned long long splats = 0;
-    bool busy = false, drained = false;
+    uint32_t splats = 0;
+    __shared__ uint32_t block_splats;
+    if (threadIdx.x == 0) block_splats = 0;
+    __syncthreads();
+    bool busy = false;
+    Feed feed = feed_init(n);
     uint32_t idx = 0;
     const SceneDev* sc = &p.scene;
     WRay r;
     Trav st;
     for (;;) {
-        if (!drained && __any_sync(kFull, !busy)) {
-            const uint32_t k = refill(busy, cursor, n, drained);
-            if (!busy && k < n) {
+        if ((!feed.drained || feed.cur < feed.end) && __any_sync(kFull, !busy)) {
+            uint32_t k;
+            if (refill(feed, busy, cursor, n, k)) {
                 idx = k;
                 const float4 o = p.wave.sh_o[idx];
                 const float4 d = p.wave.sh_d[idx];
@@ -373,7 +414,12 @@ __global__ void __launch_bounds__(kTraceBlock, kTraceMinBlocks) k_shadow(const _
             busy = false;
         }
     }
-    if (splats) atomicAdd(&p.wave.stats[2], splats);
+    // one 64-bit atomic per block: one per thread (151,552 on one address) took 60 us of the 130 us
+    // that 1 M shadow rays of the 34-triangle room needed
+    splats = __reduce_add_sync(kFull, splats);
+    if ((threadIdx.x & 31u) == 0 && splats) atomicAdd(&block_splats, splats);
+    __syncthreads();
+    if (threadIdx.x == 0 && block_splats) atomicAdd(&p.wave.stats[2], (unsigned long long)block_splats);
 }
 
 // -----------------------------------------------------------------------------------------
@@ -1422,7 +1468,8 @@ __global__ void __launch_bounds__(256) k_connect_compact(const __grid_constant__
         splats += j - n0;
         p.wave.rec_n[slot] = (uint8_t)j;
     }
-    if (splats) atomicAdd(&p.wave.stats[2], splats);
+    for (int o = 16; o; o >>= 1) splats += __shfl_down_sync(kFull, splats, o);
+    if ((threadIdx.x & 31u) == 0 && splats) atomicAdd(&p.wave.stats[2], splats);
 }
 
 // -----------------------------------------------------------------------------------------
