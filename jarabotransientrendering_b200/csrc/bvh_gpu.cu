@@ -547,17 +547,17 @@ __global__ void k_count4(const BinNode* __restrict__ nodes, const uint32_t* q, u
 // order; boxes one ulp outward), its children's indices and triangle offsets for the next level
 __global__ void k_place4(const BinNode* __restrict__ nodes, const uint32_t* __restrict__ ids, const uint32_t* q,
                          uint32_t lo, uint32_t n, const int4* kids, const uint32_t* n4, uint32_t* gidx, uint32_t* toff,
-                         GpuNode* out, uint32_t* order, uint32_t* leaves) {
+                         DevNode* out, uint32_t* order, uint32_t* leaves) {
     const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n) return;
     const uint32_t nd = q[lo + i];
     const int4 c4 = kids[nd];
     const int32_t c[4] = {c4.x, c4.y, c4.z, c4.w};
-    GpuNode g;
+    DevNode g;
     uint32_t gnext = gidx[nd] + 1, t = toff[nd];
     for (int j = 0; j < 4; ++j) {
         if (c[j] < 0) {
-            g.lox[j] = g.hix[j] = g.loy[j] = g.hiy[j] = g.loz[j] = g.hiz[j] = 0.0f;
+            for (int k = 0; k < 3; ++k) g.plane[k][j][0] = g.plane[k][j][1] = 3.402823466e+38f;
             g.child[j] = ~(int32_t)0;           // leaf of 0 triangles: never entered
             continue;
         }
@@ -569,9 +569,7 @@ __global__ void k_place4(const BinNode* __restrict__ nodes, const uint32_t* __re
                 bhi[k] = nextafterf(bhi[k], INFINITY);
             }
         }
-        g.lox[j] = blo[0]; g.hix[j] = bhi[0];
-        g.loy[j] = blo[1]; g.hiy[j] = bhi[1];
-        g.loz[j] = blo[2]; g.hiz[j] = bhi[2];
+        for (int k = 0; k < 3; ++k) { g.plane[k][j][0] = blo[k]; g.plane[k][j][1] = bhi[k]; }
         if (b.left >= 0) {
             g.child[j] = (int32_t)gnext;
             gidx[c[j]] = gnext;
@@ -607,7 +605,7 @@ T* pool_alloc(size_t count, cudaStream_t s, std::vector<void*>& held) {
 // false when the input is invalid (out-of-range index or non-finite vertex: the caller's host
 // builder reports which).  Throws tri::CudaError on CUDA failures.
 bool build_bvh_device(const float* d_v, uint32_t nv, const uint32_t* d_t, uint32_t nt, uint32_t max_leaf,
-                      cudaStream_t s, const std::function<GpuNode*(size_t)>& alloc_nodes, uint32_t* d_order,
+                      cudaStream_t s, const std::function<DevNode*(size_t)>& alloc_nodes, uint32_t* d_order,
                       DeviceBvh& out) {
     const auto t0 = std::chrono::steady_clock::now();
     if (nt == 0 || nt >= (1u << 28)) return false;
@@ -720,7 +718,7 @@ bool build_bvh_device(const float* d_v, uint32_t nv, const uint32_t* d_t, uint32
     uint32_t n4root = 0;
     TR_CUDA(cudaMemcpyAsync(&n4root, n4, sizeof(n4root), cudaMemcpyDeviceToHost, s));
     TR_CUDA(cudaStreamSynchronize(s));
-    GpuNode* dn = alloc_nodes(n4root);
+    DevNode* dn = alloc_nodes(n4root);
     TR_CUDA(cudaMemsetAsync(d.counters + 6, 0, sizeof(uint32_t), s));
     for (int L = 0; L < levels; ++L)
         k_place4<<<(lvl_n[L] + 127) / 128, 128, 0, s>>>(d.nodes, d.ids[cur], q, lvl_lo[L], lvl_n[L], kids, n4,

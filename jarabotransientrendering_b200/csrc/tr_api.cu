@@ -167,7 +167,7 @@ void ensure_wave(tr_ctx* x, uint32_t capacity) {
     w.ray_d = x->alloc<float4>(capacity);
     w.thr = x->alloc<float4>(capacity);
     w.rng = x->alloc<unsigned long long>(capacity);
-    w.hit = x->alloc<float4>(capacity);
+    w.hit = x->alloc<float2>(capacity);
     w.q[0] = x->alloc<uint32_t>(capacity);
     w.q[1] = x->alloc<uint32_t>(capacity);
     w.sh_o = x->alloc<float4>(capacity);
@@ -191,7 +191,7 @@ void ensure_wave(tr_ctx* x, uint32_t capacity) {
         lw.ray_d = x->alloc<float4>(capacity);
         lw.thr = x->alloc<float4>(capacity);
         lw.rng = x->alloc<unsigned long long>(capacity);
-        lw.hit = x->alloc<float4>(capacity);
+        lw.hit = x->alloc<float2>(capacity);
         lw.q[0] = x->alloc<uint32_t>(capacity);
         lw.q[1] = x->alloc<uint32_t>(capacity);
         if (!x->d_lcounters) x->d_lcounters = x->alloc<uint32_t>(trk::kCounters);
@@ -276,7 +276,7 @@ void ensure_lane_wave(tr_ctx* x, int k) {
     w.ray_d = x->alloc<float4>(capacity);
     w.thr = x->alloc<float4>(capacity);
     w.rng = x->alloc<unsigned long long>(capacity);
-    w.hit = x->alloc<float4>(capacity);
+    w.hit = x->alloc<float2>(capacity);
     w.q[0] = x->alloc<uint32_t>(capacity);
     w.q[1] = x->alloc<uint32_t>(capacity);
     w.sh_o = x->alloc<float4>(capacity);
@@ -809,7 +809,7 @@ tr_status tr_create(const tr_scene* s, const tr_camera* c, const tr_film* f, con
         float4* dnodes = nullptr;
         const bool on_device = trh::build_bvh_device(
             d_v, s->num_vertices, d_t, s->num_triangles, 4, x->stream,
-            [&](size_t n) { dnodes = x->alloc<float4>(n * 8); return reinterpret_cast<trh::GpuNode*>(dnodes); },
+            [&](size_t n) { dnodes = x->alloc<float4>(n * 8); return reinterpret_cast<trh::DevNode*>(dnodes); },
             d_o, dbv);
         trh::BvhBuildResult bvh;
         if (!on_device) {
@@ -826,7 +826,21 @@ tr_status tr_create(const tr_scene* s, const tr_camera* c, const tr_film* f, con
             dbv.stack = bvh.stack;
             dbv.build_ms = bvh.build_ms;
             dnodes = x->alloc<float4>(bvh.nodes.size() * 8);
-            upload(dnodes, bvh.nodes.data(), bvh.nodes.size() * sizeof(trh::GpuNode), x->stream);
+            std::vector<trh::DevNode> dev(bvh.nodes.size());
+            for (size_t i = 0; i < dev.size(); ++i) {
+                const trh::GpuNode& n = bvh.nodes[i];
+                for (int j = 0; j < 4; ++j) {
+                    const bool empty = n.child[j] < 0 && ((~n.child[j]) & 7) == 0;
+                    const float lo[3] = {n.lox[j], n.loy[j], n.loz[j]}, hi[3] = {n.hix[j], n.hiy[j], n.hiz[j]};
+                    for (int k = 0; k < 3; ++k) {
+                        dev[i].plane[k][j][0] = empty ? 3.402823466e+38f : lo[k];
+                        dev[i].plane[k][j][1] = empty ? 3.402823466e+38f : hi[k];
+                    }
+                    dev[i].child[j] = n.child[j];
+                    dev[i].pad[j] = 0;
+                }
+            }
+            upload(dnodes, dev.data(), dev.size() * sizeof(trh::DevNode), x->stream);
             TR_CUDA(cudaMemcpyAsync(d_o, bvh.order.data(), sizeof(uint32_t) * ntri, cudaMemcpyHostToDevice, x->stream));
         }
         if (dbv.stack > (uint32_t)trk::kStack) {
@@ -893,7 +907,9 @@ tr_status tr_create(const tr_scene* s, const tr_camera* c, const tr_film* f, con
                     lo[k] = std::min(lo[k], s->vertices[3 * (size_t)i + k]);
                     hi[k] = std::max(hi[k], s->vertices[3 * (size_t)i + k]);
                 }
+            sc.reach = 0.0f;
             for (int k = 0; k < 3; ++k) {
+                sc.reach = std::max(sc.reach, std::max(std::fabs(lo[k]), std::fabs(hi[k])));
                 sc.bmin[k] = lo[k];
                 sc.binv[k] = hi[k] > lo[k] ? 1.0f / (hi[k] - lo[k]) : 1.0f;
             }
@@ -1275,7 +1291,7 @@ extern "C" tr_status tr_render_region_noalloc(tr_ctx* x, uint32_t x0, uint32_t y
         w.ray_o = reinterpret_cast<float4*>(take(sizeof(float4) * kNaSlots));
         w.ray_d = reinterpret_cast<float4*>(take(sizeof(float4) * kNaSlots));
         w.thr = reinterpret_cast<float4*>(take(sizeof(float4) * kNaSlots));
-        w.hit = reinterpret_cast<float4*>(take(sizeof(float4) * kNaSlots));
+        w.hit = reinterpret_cast<float2*>(take(sizeof(float2) * kNaSlots));
         w.sh_o = reinterpret_cast<float4*>(take(sizeof(float4) * kNaSlots));
         w.sh_d = reinterpret_cast<float4*>(take(sizeof(float4) * kNaSlots));
         w.sh_L = reinterpret_cast<float4*>(take(sizeof(float4) * kNaSlots));

@@ -177,7 +177,7 @@ void ensure_lane(tr_batch* b, trk::Wave& w, uint32_t capacity, unsigned long lon
     w.ray_d = b->alloc<float4>(capacity);
     w.thr = b->alloc<float4>(capacity);
     w.rng = b->alloc<unsigned long long>(capacity);
-    w.hit = b->alloc<float4>(capacity);
+    w.hit = b->alloc<float2>(capacity);
     w.q[0] = b->alloc<uint32_t>(capacity);
     w.q[1] = b->alloc<uint32_t>(capacity);
     w.sh_o = b->alloc<float4>(capacity);

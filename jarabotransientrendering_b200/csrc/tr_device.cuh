@@ -144,7 +144,6 @@ struct WRay {
     float tnear;
     int kx, ky, kz;
     float Sx, Sy;
-    f3 inv;       // reciprocal direction for the slab test
 };
 
 __device__ __forceinline__ void wray_setup(WRay& r, f3 o, f3 d, float tnear) {
@@ -159,10 +158,6 @@ __device__ __forceinline__ void wray_setup(WRay& r, f3 o, f3 d, float tnear) {
     r.kx = kx; r.ky = ky; r.kz = kz;
     float dz = comp(d, kz);
     r.Sx = comp(d, kx) / dz; r.Sy = comp(d, ky) / dz;
-    const float e = 1e-30f;
-    r.inv = mk(1.0f / (fabsf(d.x) > e ? d.x : copysignf(e, d.x)),
-               1.0f / (fabsf(d.y) > e ? d.y : copysignf(e, d.y)),
-               1.0f / (fabsf(d.z) > e ? d.z : copysignf(e, d.z)));
 }
 
 __device__ __forceinline__ bool wt_hit(const WRay& r, f3 p0, f3 p1, f3 p2, float tfar,

@@ -262,7 +262,15 @@ tr_status train_on_pool(tr_guide* g, const trk::GuideWave& gw, const uint32_t* p
 }  // namespace tri
 
 namespace trh {
-struct GpuNode;
+// Four-child node as the traversal reads it (128 bytes): per axis and child the box's lower and
+// upper plane side by side, so one packed multiply-add gives both distances, then the child refs
+// as in GpuNode.  An empty slot's planes are all at the largest float: the slab test never passes.
+struct alignas(32) DevNode {
+    float plane[3][4][2];
+    int32_t child[4];
+    int32_t pad[4];
+};
+static_assert(sizeof(DevNode) == 128, "node must be 128 bytes");
 // Figures of a device build (its nodes and leaf order stay on the device).
 struct DeviceBvh {
     uint32_t nodes = 0;          // four-child nodes
@@ -277,6 +285,6 @@ struct DeviceBvh {
 // alloc_nodes(count), the triangle ids in leaf order to d_order [nt].  False on invalid input or
 // a one-leaf scene (the host builder then builds, or reports which index or vertex is wrong).
 bool build_bvh_device(const float* d_vertices, uint32_t nv, const uint32_t* d_triangles, uint32_t nt,
-                      uint32_t max_leaf, cudaStream_t s, const std::function<GpuNode*(size_t)>& alloc_nodes,
+                      uint32_t max_leaf, cudaStream_t s, const std::function<DevNode*(size_t)>& alloc_nodes,
                       uint32_t* d_order, DeviceBvh& out);
 }  // namespace trh

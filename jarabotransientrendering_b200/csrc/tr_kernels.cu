@@ -29,25 +29,77 @@ using namespace trd;
 // triangle test.  Closest hit: smallest t in (tnear, tfar], ties -> lower triangle id (order
 // independent, so the result does not depend on the tree).
 // -----------------------------------------------------------------------------------------
-__device__ __forceinline__ void slab4(float lo_x, float hi_x, float lo_y, float hi_y, float lo_z, float hi_z, int ref,
-                                      float ox, float oy, float oz, float ix, float iy, float iz, float tnear,
-                                      float best, float& key) {
-    const float lx = (lo_x - ox) * ix, hx = (hi_x - ox) * ix;
-    const float ly = (lo_y - oy) * iy, hy = (hi_y - oy) * iy;
-    const float lz = (lo_z - oz) * iz, hz = (hi_z - oz) * iz;
-    const float tmin = fmaxf(fmaxf(fminf(lx, hx), fminf(ly, hy)), fmaxf(fminf(lz, hz), tnear));
-    const float tmax = fminf(fminf(fmaxf(lx, hx), fmaxf(ly, hy)), fminf(fmaxf(lz, hz), best)) * 1.00000036f;
-    // empty slots are leaves of 0 triangles
-    const bool use = ref >= 0 || ((~ref) & 7) != 0;
-    key = (use && tmin <= tmax) ? tmin : __int_as_float(0x7f800000);
+// Two floats in one 64-bit register pair (sm_100 packed FP32 arithmetic).
+typedef unsigned long long f2;
+__device__ __forceinline__ f2 pack2(float lo, float hi) {
+    f2 r;
+    asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(lo), "f"(hi));
+    return r;
+}
+__device__ __forceinline__ void unpack2(f2 v, float& lo, float& hi) {
+    asm("mov.b64 {%0, %1}, %2;" : "=f"(lo), "=f"(hi) : "l"(v));
+}
+__device__ __forceinline__ f2 fma2(f2 a, f2 b, f2 c) {
+    f2 r;
+    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
+    return r;
+}
+__device__ __forceinline__ float max3(float a, float b, float c) {
+    float r;
+    asm("max.f32 %0, %1, %2, %3;" : "=f"(r) : "f"(a), "f"(b), "f"(c));
+    return r;
+}
+__device__ __forceinline__ float min3(float a, float b, float c) {
+    float r;
+    asm("min.f32 %0, %1, %2, %3;" : "=f"(r) : "f"(a), "f"(b), "f"(c));
+    return r;
+}
+
+// The slab test's per-ray constants: per axis, the pairs (for the box's lower plane, for its upper
+// plane) m and a with t = plane * m + a, one packed multiply-add per child and axis.  Against
+// t = (plane - o) * inv the product P = plane * inv and c = o * inv round separately, so the
+// plane the ray meets first gets |m| = |inv| (1 - 8e) and a = -c - 12e|c|, the other one
+// |inv| (1 + 8e) and -c + 12e|c| (e = 2^-24): with the two roundings of the multiply-add the
+// interval holds (1 -+ 6e) times the exact one wherever t > 0.  For t < 0 (a ray with tnear < 0)
+// the slack is taken from the largest |P| a box of the scene can have instead.  |inv| is capped
+// so that c stays finite: a direction component below |o| 2^-100 moves the ray by less than an
+// ulp of o.
+struct SlabRay { f2 mx, my, mz, ax, ay, az; };
+__device__ __forceinline__ void slab_axis(float o, float d, float reach, f2& m, f2& a) {
+    const float ad = fmaxf(fmaxf(fabsf(d), 1e-30f), fabsf(o) * 7.88860905e-31f);
+    const float inv = copysignf(1.0f / ad, d);
+    const float c = o * inv;
+    const float slack = 7.2e-7f * (fabsf(c) + reach * fabsf(inv));
+    const float mn = inv * 0.99999952f, mf = inv * 1.00000048f;
+    const float an = -c - slack, af = slack - c;
+    const bool neg = inv < 0.0f;
+    m = pack2(neg ? mf : mn, neg ? mn : mf);
+    a = pack2(neg ? af : an, neg ? an : af);
+}
+__device__ __forceinline__ SlabRay slab_setup(const SceneDev& sc, f3 o, f3 d, float tnear) {
+    const float reach = tnear < 0.0f ? sc.reach : 0.0f;
+    SlabRay s;
+    slab_axis(o.x, d.x, reach, s.mx, s.ax);
+    slab_axis(o.y, d.y, reach, s.my, s.ay);
+    slab_axis(o.z, d.z, reach, s.mz, s.az);
+    return s;
+}
+// entry distance of a child's box (lower and upper plane of each axis in x, y, z), +inf on a
+// miss; `far` = the closest hit so far, widened for ties
+__device__ __forceinline__ float slab(const SlabRay& s, f2 x, f2 y, f2 z, float tnear, float far) {
+    float lx, hx, ly, hy, lz, hz;
+    unpack2(fma2(x, s.mx, s.ax), lx, hx);
+    unpack2(fma2(y, s.my, s.ay), ly, hy);
+    unpack2(fma2(z, s.mz, s.az), lz, hz);
+    const float tmin = fmaxf(max3(fminf(lx, hx), fminf(ly, hy), fminf(lz, hz)), tnear);
+    const float tmax = fminf(min3(fmaxf(lx, hx), fmaxf(ly, hy), fmaxf(lz, hz)), far);
+    return tmin <= tmax ? tmin : __int_as_float(0x7f800000);
 }
 // 32 bytes in one load (sm_100: 256-bit global loads); p must be 32-byte aligned (the launchers
-// check the node buffer).  A node's bounds arrive in three such loads instead of six 128-bit
-// ones: the divergent lanes of a warp each cost their own L1 request per load instruction.
-__device__ __forceinline__ void ldg256(const float4* p, float4& a, float4& b) {
-    asm("ld.global.nc.v8.f32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
-        : "=f"(a.x), "=f"(a.y), "=f"(a.z), "=f"(a.w), "=f"(b.x), "=f"(b.y), "=f"(b.z), "=f"(b.w)
-        : "l"(p));
+// check the node buffer): the divergent lanes of a warp each cost their own L1 request per load
+// instruction, so a node's bounds arrive in three loads.
+__device__ __forceinline__ void ldg256(const float4* p, f2& a, f2& b, f2& c, f2& d) {
+    asm("ld.global.nc.v4.b64 {%0, %1, %2, %3}, [%4];" : "=l"(a), "=l"(b), "=l"(c), "=l"(d) : "l"(p));
 }
 __device__ __forceinline__ void order2(float& ka, int& ra, float& kb, int& rb) {
     if (kb < ka) {
@@ -60,37 +112,43 @@ __device__ __forceinline__ void order2(float& ka, int& ra, float& kb, int& rb) {
 // leaf), stack depth, closest hit so far.
 struct Trav {
     int node, sp;
-    float best, bu, bv;
+    float best;               // distance of the closest hit so far, the ray's end without one
     uint32_t bid;
 };
+struct Bary { float u, v; };
 __device__ __forceinline__ void trav_init(Trav& st, float tfar) {
-    st.node = 0; st.sp = 0; st.best = tfar; st.bu = 0.f; st.bv = 0.f; st.bid = kInvalid;
+    st.node = 0; st.sp = 0; st.best = tfar; st.bid = kInvalid;
 }
 
 // Runs at most `budget` node or triangle visits of the ray's traversal; returns true once the
 // traversal is complete (closest hit, or any hit with kAnyHit, in st).  The stack lives in
-// shared memory at stack[k * stride].
+// shared memory at stack[k * stride]; uv (optional) receives the closest hit's barycentrics.
+//
+// Bound by the chain of dependent loads of a ray (half of them L1 hits), then by issue slots.  The
+// packed slab test issues 16 % fewer instructions than six subtractions and six products per
+// child (172 M -> 145 M for the 1 M first-bounce rays of a 2 M-path batch over 328 k triangles);
+// with barycentrics and distances that no caller reads left out it fits 72 registers, and
+// six blocks per SM without spills beat seven or eight with them: the 4.9 M-path pass over that
+// mesh takes 4.33 ms (8 blocks 4.52, 5 blocks 4.60; subtract-and-multiply test, 8 blocks: 4.60).
 template <bool kAnyHit>
-__device__ __forceinline__ bool trav_run(const SceneDev& sc, const WRay& r, Trav& st, int* __restrict__ stack,
-                                         int stride, int budget) {
-    const float ox = r.o.x, oy = r.o.y, oz = r.o.z;
-    const float ix = r.inv.x, iy = r.inv.y, iz = r.inv.z;
+__device__ __forceinline__ bool trav_run(const SceneDev& sc, const WRay& r, const SlabRay& s, Trav& st,
+                                         int* __restrict__ stack, int stride, int budget, Bary* uv = nullptr) {
     const float kInf = __int_as_float(0x7f800000);
     for (;;) {
         if (budget-- == 0) return false;
         if (st.node >= 0) {
             const float4* np = sc.nodes + 8 * st.node;
-            float4 lx, hx, ly, hy, lz, hz;
-            ldg256(np, lx, hx);
-            ldg256(np + 2, ly, hy);
-            ldg256(np + 4, lz, hz);
+            f2 x0, x1, x2, x3, y0, y1, y2, y3, z0, z1, z2, z3;
+            ldg256(np, x0, x1, x2, x3);
+            ldg256(np + 2, y0, y1, y2, y3);
+            ldg256(np + 4, z0, z1, z2, z3);
             const int4 ch = __ldg(reinterpret_cast<const int4*>(np + 6));
-            float k0, k1, k2, k3;
             int c0 = ch.x, c1 = ch.y, c2 = ch.z, c3 = ch.w;
-            slab4(lx.x, hx.x, ly.x, hy.x, lz.x, hz.x, c0, ox, oy, oz, ix, iy, iz, r.tnear, st.best, k0);
-            slab4(lx.y, hx.y, ly.y, hy.y, lz.y, hz.y, c1, ox, oy, oz, ix, iy, iz, r.tnear, st.best, k1);
-            slab4(lx.z, hx.z, ly.z, hy.z, lz.z, hz.z, c2, ox, oy, oz, ix, iy, iz, r.tnear, st.best, k2);
-            slab4(lx.w, hx.w, ly.w, hy.w, lz.w, hz.w, c3, ox, oy, oz, ix, iy, iz, r.tnear, st.best, k3);
+            const float far = fmaf(fabsf(st.best), 1e-6f, st.best);
+            float k0 = slab(s, x0, y0, z0, r.tnear, far);
+            float k1 = slab(s, x1, y1, z1, r.tnear, far);
+            float k2 = slab(s, x2, y2, z2, r.tnear, far);
+            float k3 = slab(s, x3, y3, z3, r.tnear, far);
             if constexpr (!kAnyHit) {
                 order2(k0, c0, k1, c1);
                 order2(k2, c2, k3, c3);
@@ -136,7 +194,8 @@ __device__ __forceinline__ bool trav_run(const SceneDev& sc, const WRay& r, Trav
             float t, u, v;
             if (wt_hit(r, f3of(q0), f3of(q1), f3of(q2), st.best, t, u, v)) {
                 if (t < st.best || st.bid == kInvalid || id < st.bid) {
-                    st.best = t; st.bid = id; st.bu = u; st.bv = v;
+                    st.best = t; st.bid = id;
+                    if (uv) *uv = Bary{u, v};
                     if (kAnyHit) return true;
                 }
             }
@@ -149,19 +208,6 @@ __device__ __forceinline__ bool trav_run(const SceneDev& sc, const WRay& r, Trav
         --st.sp;
         st.node = stack[st.sp * stride];
     }
-}
-
-// Whole traversal in one call (used where one thread owns a fixed set of rays).
-template <bool kAnyHit>
-__device__ __forceinline__ uint32_t traverse(const SceneDev& sc, const WRay& r, float tfar,
-                                             float& t_out, float& u_out, float& v_out,
-                                             int* __restrict__ stack, int stride) {
-    Trav st;
-    trav_init(st, tfar);
-    trav_run<kAnyHit>(sc, r, st, stack, stride, 0x7fffffff);
-    t_out = st.bid == kInvalid ? tfar : st.best;
-    u_out = st.bu; v_out = st.bv;
-    return st.bid;
 }
 
 // -----------------------------------------------------------------------------------------
@@ -264,21 +310,15 @@ constexpr int kTravBudget = 8;
 // atomic).  Shorter first runs that spread a short queue over more warps shorten a lone launch
 // (46 k rays of a 20 k-triangle mesh: 50 -> 40 us) but cost issue slots when several lanes'
 // launches share the GPU (4.9 M-path pass over 328 k triangles: 4.58 -> 4.82 ms).
-struct Feed {
-    uint32_t cur, end;        // the warp's entries not handed out yet (warp uniform)
-    uint32_t own;             // entries handed out without the cursor
-    bool drained;             // the queue ends at `end`
-};
+struct Feed { uint32_t cur, end; };     // the warp's entries not handed out yet (warp uniform)
 constexpr uint32_t kRun = 32;
 __device__ __forceinline__ Feed feed_init(uint32_t n) {
     const uint32_t w = blockIdx.x * (kTraceBlock / 32u) + (threadIdx.x >> 5);
-    Feed f;
-    f.cur = min(n, w * kRun);
-    f.end = min(n, f.cur + kRun);
-    f.own = gridDim.x * (kTraceBlock / 32u) * kRun;
-    f.drained = f.own >= n;
-    return f;
+    const uint32_t cur = min(n, w * kRun);
+    return Feed{cur, min(n, cur + kRun)};
 }
+// entries may be left: the warp's own, or beyond its run when that did not end the queue
+__device__ __forceinline__ bool feed_more(const Feed& f, uint32_t n) { return f.cur < f.end || f.end < n; }
 // Every lane with busy == false takes an entry; false: none is left for this lane.
 __device__ __forceinline__ bool refill(Feed& f, bool busy, uint32_t* cursor, uint32_t n, uint32_t& idx) {
     const unsigned idle = __ballot_sync(kFull, !busy);
@@ -290,12 +330,12 @@ __device__ __forceinline__ bool refill(Feed& f, bool busy, uint32_t* cursor, uin
         f.cur += want;
     } else {
         f.cur = f.end;
-        if (!f.drained) {
-            uint32_t base = 0;
-            if ((threadIdx.x & 31u) == 0) base = f.own + atomicAdd(cursor, kRun);
+        if (f.end < n) {
+            // entries past every warp's first run
+            uint32_t base = gridDim.x * (kTraceBlock / 32u) * kRun;
+            if ((threadIdx.x & 31u) == 0) base += atomicAdd(cursor, kRun);
             base = min(n, __shfl_sync(kFull, base, 0));
             f.end = min(n, base + kRun);
-            f.drained = f.end >= n;
             if (!got) {
                 idx = base + (rank - have);
                 got = idx < f.end;
@@ -321,12 +361,12 @@ __global__ void __launch_bounds__(kTraceBlock, kTraceMinBlocks) k_extend(const _
     bool busy = false;
     Feed feed = feed_init(n);
     uint32_t slot = 0;
-    float tfar = 0.f;
     const SceneDev* sc = &p.scene;
     WRay r;
+    SlabRay sr;
     Trav st;
     for (;;) {
-        if ((!feed.drained || feed.cur < feed.end) && __any_sync(kFull, !busy)) {
+        if (feed_more(feed, n) && __any_sync(kFull, !busy)) {
             uint32_t idx;
             if (refill(feed, busy, cursor, n, idx)) {
                 slot = depth == 0 ? idx : q[idx];
@@ -339,18 +379,17 @@ __global__ void __launch_bounds__(kTraceBlock, kTraceMinBlocks) k_extend(const _
                 const float4 o = p.wave.ray_o[slot];
                 const float4 d = p.wave.ray_d[slot];
                 wray_setup(r, mk(o.x, o.y, o.z), mk(d.x, d.y, d.z), kSigmaVis);
+                sr = slab_setup(*sc, r.o, r.d, kSigmaVis);
                 // camera unwarp and the film components need the camera ray's closest surface
                 // at any distance (World::Li's record, World.h:749-766); shade still decides
                 // surface vs medium event by comparing with the sampled distance (o.w)
-                tfar = depth == 0 && (film->unwarp || film->comps) ? __int_as_float(0x7f800000) : o.w;
-                trav_init(st, tfar);
+                trav_init(st, depth == 0 && (film->unwarp || film->comps) ? __int_as_float(0x7f800000) : o.w);
                 busy = true;
             }
         }
         if (!__any_sync(kFull, busy)) break;
-        if (busy && trav_run<false>(*sc, r, st, stack + threadIdx.x, kTraceBlock, kTravBudget)) {
-            const float t = st.bid == kInvalid ? tfar : st.best;
-            p.wave.hit[slot] = make_float4(t, __uint_as_float(st.bid), st.bu, st.bv);
+        if (busy && trav_run<false>(*sc, r, sr, st, stack + threadIdx.x, kTraceBlock, kTravBudget)) {
+            p.wave.hit[slot] = make_float2(st.best, __uint_as_float(st.bid));
             busy = false;
         }
     }
@@ -374,9 +413,10 @@ __global__ void __launch_bounds__(kTraceBlock, kTraceMinBlocks) k_shadow(const _
     uint32_t idx = 0;
     const SceneDev* sc = &p.scene;
     WRay r;
+    SlabRay sr;
     Trav st;
     for (;;) {
-        if ((!feed.drained || feed.cur < feed.end) && __any_sync(kFull, !busy)) {
+        if (feed_more(feed, n) && __any_sync(kFull, !busy)) {
             uint32_t k;
             if (refill(feed, busy, cursor, n, k)) {
                 idx = k;
@@ -385,12 +425,13 @@ __global__ void __launch_bounds__(kTraceBlock, kTraceMinBlocks) k_shadow(const _
                 if constexpr (kMulti)
                     sc = &p.multi.scenes[seg_of_slot(cur_batch(p), __float_as_uint(p.wave.sh_L[idx].w)).scene].scene;
                 wray_setup(r, mk(o.x, o.y, o.z), mk(d.x, d.y, d.z), kSigmaVis);
+                sr = slab_setup(*sc, r.o, r.d, kSigmaVis);
                 trav_init(st, o.w);
                 busy = true;
             }
         }
         if (!__any_sync(kFull, busy)) break;
-        if (busy && trav_run<true>(*sc, r, st, stack + threadIdx.x, kTraceBlock, kTravBudget)) {
+        if (busy && trav_run<true>(*sc, r, sr, st, stack + threadIdx.x, kTraceBlock, kTravBudget)) {
             const float4 d = p.wave.sh_d[idx];
             const uint32_t dw = __float_as_uint(d.w);
             if (dw & kConnRay) {
@@ -551,7 +592,7 @@ __global__ void __launch_bounds__(256, kMulti ? 3 : (kTimeSampling ? 3 : 4))
             const float inv_inc = 1.0f / (float)B.ninc;
             const uint32_t per_pix = B.ns * B.ninc;
             const uint32_t lslot = slot - B.slot_begin;
-            const float4 h = p.wave.hit[slot];
+            const float2 h = p.wave.hit[slot];
             const float4 ro = p.wave.ray_o[slot];
             const float4 rd = p.wave.ray_d[slot];
             const float4 th = p.wave.thr[slot];
@@ -1092,26 +1133,35 @@ __global__ void __launch_bounds__(256) k_bounce_weights(const __grid_constant__ 
 // -----------------------------------------------------------------------------------------
 struct HitOut { float t; uint32_t id; float u, v; };
 
-__global__ void __launch_bounds__(kTraceBlock, kTraceMinBlocks) k_trace_user(SceneDev sc, const float* __restrict__ rays,
-                                                            uint32_t n, int any_hit, HitOut* out,
-                                                            uint32_t* cursor) {
-    extern __shared__ int stack[];     // [bvh depth + 1][kTraceBlock]
-    const unsigned lane = threadIdx.x & 31u;
+template <bool kAnyHit>
+__global__ void __launch_bounds__(kTraceBlock, kTraceMinBlocks) k_trace_user(const __grid_constant__ SceneDev sc,
+                                                                             const float4* __restrict__ rays, uint32_t n,
+                                                                             HitOut* out, uint32_t* cursor) {
+    extern __shared__ int stack[];     // [stack entries][kTraceBlock]
+    bool busy = false;
+    Feed feed = feed_init(n);
+    uint32_t i = 0;
+    WRay r;
+    SlabRay sr;
+    Trav st;
+    Bary uv;
     for (;;) {
-        uint32_t base = 0;
-        if (lane == 0) base = atomicAdd(cursor, 32u);
-        base = __shfl_sync(kFull, base, 0);
-        if (base >= n) break;
-        const uint32_t i = base + lane;
-        if (i < n) {
-            const float4 a = reinterpret_cast<const float4*>(rays)[2 * (size_t)i];
-            const float4 b = reinterpret_cast<const float4*>(rays)[2 * (size_t)i + 1];
-            WRay r;
-            wray_setup(r, mk(a.x, a.y, a.z), mk(b.x, b.y, b.z), a.w);
-            float t, u, v;
-            uint32_t id = any_hit ? traverse<true>(sc, r, b.w, t, u, v, stack + threadIdx.x, kTraceBlock)
-                                  : traverse<false>(sc, r, b.w, t, u, v, stack + threadIdx.x, kTraceBlock);
-            out[i] = HitOut{t, id, u, v};
+        if (feed_more(feed, n) && __any_sync(kFull, !busy)) {
+            uint32_t k;
+            if (refill(feed, busy, cursor, n, k)) {
+                i = k;
+                const float4 a = rays[2 * (size_t)i], b = rays[2 * (size_t)i + 1];
+                wray_setup(r, mk(a.x, a.y, a.z), mk(b.x, b.y, b.z), a.w);
+                sr = slab_setup(sc, r.o, r.d, a.w);
+                trav_init(st, b.w);
+                uv = Bary{0.f, 0.f};
+                busy = true;
+            }
+        }
+        if (!__any_sync(kFull, busy)) break;
+        if (busy && trav_run<kAnyHit>(sc, r, sr, st, stack + threadIdx.x, kTraceBlock, kTravBudget, &uv)) {
+            out[i] = HitOut{st.best, st.bid, uv.u, uv.v};
+            busy = false;
         }
     }
 }
@@ -1234,7 +1284,7 @@ __global__ void __launch_bounds__(256) k_light_shade(const __grid_constant__ Par
         uint32_t slot = 0;
         if (idx < n) {
             slot = depth == 0 ? idx : qin[idx];
-            const float4 h = pl.wave.hit[slot];
+            const float2 h = pl.wave.hit[slot];
             const uint32_t tid = __float_as_uint(h.y);
             if (tid != kInvalid) {
                 const float4 ro = pl.wave.ray_o[slot], rd = pl.wave.ray_d[slot], th = pl.wave.thr[slot];
@@ -1652,8 +1702,10 @@ cudaError_t launch_advance(uint32_t* cur, uint32_t step, cudaStream_t s) {
 cudaError_t launch_trace_user(const SceneDev& sc, const float* rays, uint32_t n, int any_hit, void* out,
                               uint32_t* cursor, int grid, cudaStream_t s) {
     if (reinterpret_cast<uintptr_t>(sc.nodes) & 31u) return cudaErrorMisalignedAddress;
-    k_trace_user<<<grid, kTraceBlock, trace_smem_bytes(sc.bvh_depth), s>>>(sc, rays, n, any_hit,
-                                                                          reinterpret_cast<HitOut*>(out), cursor);
+    const float4* q = reinterpret_cast<const float4*>(rays);
+    HitOut* o = reinterpret_cast<HitOut*>(out);
+    if (any_hit) k_trace_user<true><<<grid, kTraceBlock, trace_smem_bytes(sc.bvh_depth), s>>>(sc, q, n, o, cursor);
+    else k_trace_user<false><<<grid, kTraceBlock, trace_smem_bytes(sc.bvh_depth), s>>>(sc, q, n, o, cursor);
     return cudaGetLastError();
 }
 

@@ -9,14 +9,14 @@ namespace trk {
 
 constexpr int kStack = 96;          // max traversal stack entries per thread (3 per four-child level + 1)
 constexpr int kTraceBlock = 128;    // threads per traversal block
-constexpr int kTraceMinBlocks = 8;  // register budget: 8 traversal blocks per SM
+constexpr int kTraceMinBlocks = 6;  // register budget: 6 traversal blocks per SM
 constexpr int kSplatBlock = 512;    // threads per splat block
 constexpr int kMaxLights = 64;
 constexpr int kMaxMaterials = 256;
 
 // Scene as the kernels see it (device pointers).
 struct SceneDev {
-    const float4* nodes;      // 4 float4 per two-child node
+    const float4* nodes;      // four-child nodes (trh::DevNode, 128 bytes)
     const float4* tris;       // 3 float4 per triangle, leaf order (v0.w = triangle id)
     const float4* tri_ng;     // per triangle id: geometric normal xyz, material index (bits)
     const float4* mats;       // per material: kd.rgb, kind (bits)
@@ -30,6 +30,7 @@ struct SceneDev {
     float g;
     uint32_t bvh_depth;       // traversal stack entries - 1 (3 per four-child level)
     float bmin[3], binv[3];   // scene box (feature normalisation of the learned proposal)
+    float reach;              // largest |coordinate| of the scene
 };
 
 constexpr uint32_t kFlagOrthoFrame = 1u;   // TR_FLAG_ORTHONORMAL_FRAME
@@ -120,7 +121,7 @@ struct Wave {
     float4* ray_d;            // d.xyz, accumulated time
     float4* thr;              // throughput rgb, pending pdf factor (RR prob * direction pdf)
     unsigned long long* rng;  // PCG32 state (increment derived from the camera sample)
-    float4* hit;              // t, triangle id (bits), u, v
+    float2* hit;              // t, triangle id (bits)
     uint32_t* q[2];           // extend queues (ping-pong)
     float4* sh_o;             // shadow: origin, tfar
     float4* sh_d;             // shadow: direction, time bin (bits)
