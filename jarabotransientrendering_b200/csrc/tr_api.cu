@@ -531,8 +531,14 @@ tr_status render_region(tr_ctx* x, uint32_t x0, uint32_t y0, uint32_t x1, uint32
             p.batch.pix_begin = (uint32_t)pb; p.batch.npix = npix;
             p.batch.s0 = s0 + sb; p.batch.ns = ns; p.batch.ninc = ninc;
             p.batch.n_slots = npix * per_pix;
-            TR_CUDA(cudaMemsetAsync(p.wave.counters, 0, trk::kCounters * sizeof(uint32_t), ls));
-            tl(0, [&] { return trk::launch_raygen(p, ls); });
+            // small batches: whole paths in one launch (per-kernel times need the kernels apart)
+            const bool whole = trk::paths_fit(p) && !x->profiling;
+            if (whole) {
+                tl(1, [&] { return trk::launch_paths(p, ls); });
+            } else {
+                TR_CUDA(cudaMemsetAsync(p.wave.counters, 0, trk::kCounters * sizeof(uint32_t), ls));
+                tl(0, [&] { return trk::launch_raygen(p, ls); });
+            }
             if (bidir) {
                 // the light subpaths, on the light wave, from the light points raygen drew.
                 // They share nothing with the eye walks until the connections (own rays,
@@ -555,7 +561,7 @@ tr_status render_region(tr_ctx* x, uint32_t x0, uint32_t y0, uint32_t x1, uint32
                 launches += 1 + 2ull * x->bd.nvert;
                 ext_l += x->bd.nvert;
             }
-            for (uint32_t d = 0; d < x->integ.max_bounces; ++d) {
+            for (uint32_t d = 0; d < (whole ? 0u : x->integ.max_bounces); ++d) {
                 tl(1, [&] { return trk::launch_extend(p, (int)d, x->trace_grid, ls); });
                 if (d > 0) TR_CUDA(order(lsh, ls));
                 if (guided && d < x->guide_depth) {
@@ -573,7 +579,7 @@ tr_status render_region(tr_ctx* x, uint32_t x0, uint32_t y0, uint32_t x1, uint32
                 TR_CUDA(order(ls, lsh));
                 timed_on(3, lsh, [&] { return trk::launch_shadow(p, (int)d, x->trace_grid, lsh); });
             }
-            if (x->integ.max_bounces) TR_CUDA(order(lsh, ls));
+            if (!whole && x->integ.max_bounces) TR_CUDA(order(lsh, ls));
             if (guided && x->guide_pool) {
                 TR_CUDA(trk::launch_train_gather(p, x->pool_state, ls));
                 launches += 2;
@@ -614,9 +620,9 @@ tr_status render_region(tr_ctx* x, uint32_t x0, uint32_t y0, uint32_t x1, uint32
                 tl(4, [&] { return trk::launch_bounce_weights(p, ls); });
                 launches += 1ull + x->film.bounce_films;
             }
-            launches += 2 + 3ull * x->integ.max_bounces;
-            ext_l += x->integ.max_bounces;
-            sh_l += x->integ.max_bounces;
+            launches += 2 + (whole ? 0 : 3ull * x->integ.max_bounces);
+            ext_l += whole ? 1 : x->integ.max_bounces;
+            sh_l += whole ? 0 : x->integ.max_bounces;
             if (sink && sb + ns >= ns_total) {
                 // window = whole frame: the batch's pixels are contiguous film rows
                 const size_t p0 = pb, np = npix;
@@ -1312,11 +1318,15 @@ extern "C" tr_status tr_render_region_noalloc(tr_ctx* x, uint32_t x0, uint32_t y
         p.batch.pix_begin = 0; p.batch.npix = (uint32_t)npix;
         p.batch.s0 = s0; p.batch.ns = ns; p.batch.ninc = x->integ.incoming_samples;
         p.batch.n_slots = (uint32_t)paths;
-        TR_CUDA(trk::launch_raygen(p, strm));
-        for (uint32_t d = 0; d < x->integ.max_bounces; ++d) {
-            TR_CUDA(trk::launch_extend(p, (int)d, x->trace_grid, strm));
-            TR_CUDA(trk::launch_shade(p, (int)d, strm));
-            TR_CUDA(trk::launch_shadow(p, (int)d, x->trace_grid, strm));
+        if (trk::paths_fit(p)) {
+            TR_CUDA(trk::launch_paths(p, strm));
+        } else {
+            TR_CUDA(trk::launch_raygen(p, strm));
+            for (uint32_t d = 0; d < x->integ.max_bounces; ++d) {
+                TR_CUDA(trk::launch_extend(p, (int)d, x->trace_grid, strm));
+                TR_CUDA(trk::launch_shade(p, (int)d, strm));
+                TR_CUDA(trk::launch_shadow(p, (int)d, x->trace_grid, strm));
+            }
         }
         TR_CUDA(trk::launch_splat(p, strm));
         for (uint32_t b = 0; b < x->film.bounce_films; ++b) TR_CUDA(trk::launch_splat(p, strm, (int)b));

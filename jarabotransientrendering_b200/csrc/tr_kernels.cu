@@ -122,7 +122,8 @@ __device__ __forceinline__ void trav_init(Trav& st, float tfar) {
 
 // Runs at most `budget` node or triangle visits of the ray's traversal; returns true once the
 // traversal is complete (closest hit, or any hit with kAnyHit, in st).  The stack lives in
-// shared memory at stack[k * stride]; uv (optional) receives the closest hit's barycentrics.
+// shared memory at stack[k * stride]; uv (optional) receives the closest hit's barycentrics.  kAnyHit
+// leaves the children unsorted; `any` ends the query at its first hit.
 //
 // Bound by the chain of dependent loads of a ray (half of them L1 hits), then by issue slots.  The
 // packed slab test issues 16 % fewer instructions than six subtractions and six products per
@@ -132,7 +133,8 @@ __device__ __forceinline__ void trav_init(Trav& st, float tfar) {
 // mesh takes 4.33 ms (8 blocks 4.52, 5 blocks 4.60; subtract-and-multiply test, 8 blocks: 4.60).
 template <bool kAnyHit>
 __device__ __forceinline__ bool trav_run(const SceneDev& sc, const WRay& r, const SlabRay& s, Trav& st,
-                                         int* __restrict__ stack, int stride, int budget, Bary* uv = nullptr) {
+                                         int* __restrict__ stack, int stride, int budget, Bary* uv = nullptr,
+                                         bool any = kAnyHit) {
     const float kInf = __int_as_float(0x7f800000);
     for (;;) {
         if (budget-- == 0) return false;
@@ -196,7 +198,7 @@ __device__ __forceinline__ bool trav_run(const SceneDev& sc, const WRay& r, cons
                 if (t < st.best || st.bid == kInvalid || id < st.bid) {
                     st.best = t; st.bid = id;
                     if (uv) *uv = Bary{u, v};
-                    if (kAnyHit) return true;
+                    if (any) return true;
                 }
             }
         }
@@ -216,25 +218,13 @@ __device__ __forceinline__ bool trav_run(const SceneDev& sc, const WRay& r, cons
 // (PinholeCamera.h:82-91); per-path PCG32 stream; free flight in a world medium
 // (BidirectionalPathTracing.h:240-268).
 // -----------------------------------------------------------------------------------------
-template <bool kMulti>
-__global__ void __launch_bounds__(256) k_raygen(const __grid_constant__ Params p) {
-    const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-    const Batch* Bp = &p.batch;
-    const SceneSlot* SS = nullptr;
-    if constexpr (kMulti) {
-        const BatchDesc& BD = cur_batch(p);
-        if (i >= BD.n_slots) return;
-        Bp = &seg_of_slot(BD, i);
-        SS = p.multi.scenes + Bp->scene;
-    } else {
-        if (i >= p.batch.n_slots) return;
-    }
-    const Batch& B = *Bp;
-    const FilmDev& film = kMulti ? SS->film : p.film;
-    const CameraDev& c = kMulti ? SS->cam : p.cam;
-    const unsigned long long seed = kMulti ? SS->seed : p.seed;
+struct CameraPath { float4 o, d, target; unsigned long long rng; };
+__device__ __forceinline__ CameraPath camera_path(uint32_t slot, const Batch& B, const FilmDev& film, const CameraDev& c,
+                                                  const SceneDev& sc, unsigned long long seed, uint32_t strata,
+                                                  uint32_t flags) {
+    CameraPath out;
     const uint32_t per_pix = B.ns * B.ninc;
-    const uint32_t li = i - B.slot_begin;
+    const uint32_t li = slot - B.slot_begin;
     const uint32_t pl = li / per_pix;
     const uint32_t rem = li - pl * per_pix;
     const uint32_t sl = rem / B.ninc;
@@ -246,7 +236,6 @@ __global__ void __launch_bounds__(256) k_raygen(const __grid_constant__ Params p
     const uint32_t W = film.W, H = film.H;
     const uint32_t pixel = py * W + px;
 
-    const uint32_t strata = kMulti ? SS->sqrt_spp : p.sqrt_spp;
     const uint32_t spp = strata * strata;
     const uint32_t st = (uint32_t)(s % spp);
     const uint32_t subx = st % strata, suby = st / strata;
@@ -267,10 +256,9 @@ __global__ void __launch_bounds__(256) k_raygen(const __grid_constant__ Params p
     const f3 dd = ((nv * c.fd) + ((uv * 2.0f) * imx)) - ((vv * 2.0f) * imy);
     const f3 d = normalize(dd);
 
-    const SceneDev& sc = kMulti ? SS->scene : p.scene;
     Pcg r;
     pcg_seed(r, seed + (unsigned long long)(j + 1) * kGolden64, cam_id(pixel, s));
-    if ((kMulti ? SS->flags : p.flags) & kFlagTimeSampling) {
+    if (flags & kFlagTimeSampling) {
         // time sampling: one light point per path, the target of the time-angular sampler
         // (World::sample_light + LightSource::sample, BidirectionalPathTracing.h:1107-1113;
         // PointLightSource.h:174-183, RectangularAreaLightSource.h:252-276)
@@ -284,16 +272,40 @@ __global__ void __launch_bounds__(256) k_raygen(const __grid_constant__ Params p
             const float xu = pcg_float(r), xv = pcg_float(r);
             tg = (tg + f3of(__ldg(L + 2)) * xu) + f3of(__ldg(L + 3)) * xv;
         }
-        p.wave.target[i] = make_float4(tg.x, tg.y, tg.z, __uint_as_float(lsel));
+        out.target = make_float4(tg.x, tg.y, tg.z, __uint_as_float(lsel));
     }
-    if (p.bd.ne) p.bd.ne[i] = 0;
     float dsamp = __int_as_float(0x7f800000);
     if (sc.medium) dsamp = -tr_log(pcg_float(r)) / sc.lambda;
 
-    p.wave.ray_o[i] = make_float4(c.pos[0], c.pos[1], c.pos[2], dsamp);
-    p.wave.ray_d[i] = make_float4(d.x, d.y, d.z, 0.0f);
+    out.o = make_float4(c.pos[0], c.pos[1], c.pos[2], dsamp);
+    out.d = make_float4(d.x, d.y, d.z, 0.0f);
+    out.rng = r.state;
+    return out;
+}
+
+template <bool kMulti>
+__global__ void __launch_bounds__(256) k_raygen(const __grid_constant__ Params p) {
+    const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
+    const Batch* Bp = &p.batch;
+    const SceneSlot* SS = nullptr;
+    if constexpr (kMulti) {
+        const BatchDesc& BD = cur_batch(p);
+        if (i >= BD.n_slots) return;
+        Bp = &seg_of_slot(BD, i);
+        SS = p.multi.scenes + Bp->scene;
+    } else {
+        if (i >= p.batch.n_slots) return;
+    }
+    const uint32_t flags = kMulti ? SS->flags : p.flags;
+    const CameraPath cp = camera_path(i, *Bp, kMulti ? SS->film : p.film, kMulti ? SS->cam : p.cam,
+                                      kMulti ? SS->scene : p.scene, kMulti ? SS->seed : p.seed,
+                                      kMulti ? SS->sqrt_spp : p.sqrt_spp, flags);
+    if (flags & kFlagTimeSampling) p.wave.target[i] = cp.target;
+    if (p.bd.ne) p.bd.ne[i] = 0;
+    p.wave.ray_o[i] = cp.o;
+    p.wave.ray_d[i] = cp.d;
     p.wave.thr[i] = make_float4(1.0f, 1.0f, 1.0f, 1.0f);
-    p.wave.rng[i] = r.state;
+    p.wave.rng[i] = cp.rng;
     p.wave.rec_n[i] = 0;
 }
 
@@ -543,12 +555,338 @@ __device__ __noinline__ TaSample time_angular_sample(f3 l, float mod, float r, f
     return o;
 }
 
-// kTimeSampling: compiled with the time-sampling branches (a launch whose context, or some
-// context of whose batch, has TR_FLAG_TIME_SAMPLING; the flag is still read per slot).
+// What a vertex leaves behind: a shadow ray with its contribution, the next ray (handed to the
+// path's state), or a vertex whose direction waits for the learned proposal.
+struct ShadeOut {
+    bool shadow, next, guide;
+    float4 sh_o, sh_d, sh_L;
+    uint4 gv[5];              // guided-vertex record (kGuided only)
+};
+// A path's state between two of its vertices, in the wave's arrays: the incoming ray (origin and
+// free-flight distance, direction and time), throughput and pending pdf factor, PCG32 state, and the
+// slot's camera distance and light point.
+struct WaveState {
+    const Params& p;
+    uint32_t slot, octant;    // octant of the next ray's direction
+    __device__ float4 ray_o() const { return p.wave.ray_o[slot]; }
+    __device__ float4 ray_d() const { return p.wave.ray_d[slot]; }
+    __device__ float4 thr() const { return p.wave.thr[slot]; }
+    __device__ unsigned long long rng() const { return p.wave.rng[slot]; }
+    __device__ float4 target() const { return p.wave.target[slot]; }
+    __device__ float cam_dist() const { return p.wave.cam_dist[slot]; }
+    __device__ void set_cam_dist(float d) { p.wave.cam_dist[slot] = d; }
+    __device__ void next(float4 o, float4 d, float4 t, unsigned long long rng) {
+        p.wave.ray_o[slot] = o;
+        p.wave.ray_d[slot] = d;
+        p.wave.thr[slot] = t;
+        p.wave.rng[slot] = rng;
+        octant = (d.x < 0.0f ? 1u : 0u) | (d.y < 0.0f ? 2u : 0u) | (d.z < 0.0f ? 4u : 0u);
+    }
+};
+
+// One path vertex of `slot`, hit by the ray of the path state ps at h (distance, triangle id).
+// kTimeSampling: compiled with the time-sampling branches (the flag is still read per slot).
+template <bool kGuided, bool kTimeSampling, class State>
+__device__ __forceinline__ void shade_vertex(const Params& p, int depth, uint32_t slot, const Batch& B,
+                                             const SceneDev& sc, const FilmDev& film, uint32_t max_bounces,
+                                             uint32_t flags, float2 h, State& ps, ShadeOut& o) {
+    o.shadow = o.next = o.guide = false;
+    const bool medium = sc.medium != 0;
+    const f3 sig_s = mk(sc.sig_s[0], sc.sig_s[1], sc.sig_s[2]);
+    const f3 sig_t = mk(sc.sig_t[0], sc.sig_t[1], sc.sig_t[2]);
+    const float lambda = sc.lambda;
+    const float g = sc.g;
+    const float total_time = (float)film.T * film.exposure + film.offset;
+    const float inv_inc = 1.0f / (float)B.ninc;
+    const uint32_t per_pix = B.ns * B.ninc;
+    const uint32_t lslot = slot - B.slot_begin;
+    const float4 ro = ps.ray_o();
+    const float4 rd = ps.ray_d();
+    const float4 th = ps.thr();
+    const uint32_t id = __float_as_uint(h.y);
+    const bool hit = id != kInvalid;
+    const float dsamp = ro.w;
+    const bool surface = hit && (!medium || h.x < dsamp);
+    if (depth == 0 && film.comps && lslot % B.ninc == 0) {
+        // film components: one camera-ray record per camera sample (Film.h:127-145)
+        const uint32_t pl = lslot / per_pix;
+        const uint32_t wpix = B.pix_begin + pl;
+        const size_t pixel = (size_t)(B.win_y0 + wpix / B.win_w) * film.W + (B.win_x0 + wpix % B.win_w);
+        f3 cp = mk(0.f, 0.f, 0.f), cn = cp;
+        if (hit) {
+            cp = mk(ro.x, ro.y, ro.z) + mk(rd.x, rd.y, rd.z) * h.x;
+            const float4 ng = __ldg(&sc.tri_ng[id]);
+            cn = mk(ng.x, ng.y, ng.z);
+        }
+        if (film.comps & 2u) atomicAdd(&film.cdepth[pixel], (double)(hit ? h.x : 3.40282347e+38f));
+        if (film.comps & 8u) {
+            atomicAdd(&film.cpos[pixel * 3], (double)cp.x);
+            atomicAdd(&film.cpos[pixel * 3 + 1], (double)cp.y);
+            atomicAdd(&film.cpos[pixel * 3 + 2], (double)cp.z);
+        }
+        if (film.comps & 16u) {
+            atomicAdd(&film.cnorm[pixel * 3], (double)cn.x);
+            atomicAdd(&film.cnorm[pixel * 3 + 1], (double)cn.y);
+            atomicAdd(&film.cnorm[pixel * 3 + 2], (double)cn.z);
+        }
+    }
+    if (medium || hit) {
+        // per-path RNG: state in memory, increment from the camera sample
+        const uint32_t pl = lslot / per_pix;
+        const uint32_t sl = (lslot - pl * per_pix) / B.ninc;
+        const uint32_t wpix = B.pix_begin + pl;
+        const uint32_t pixel = (B.win_y0 + wpix / B.win_w) * film.W + (B.win_x0 + wpix % B.win_w);
+        Pcg rng;
+        rng.state = ps.rng();
+        rng.inc = (cam_id(pixel, B.s0 + sl) << 1u) | 1ull;
+
+        float dist, pd;
+        if (surface) { dist = h.x; pd = medium ? tr_exp(-(dist * lambda)) : 1.0f; }
+        else { dist = dsamp; pd = tr_exp(-(dist * lambda)) * lambda; }
+        const float ptot = th.w * pd;
+        f3 f;
+        if (medium) {
+            f = mk((th.x * tr_exp(-(dist * sig_t.x))) / ptot, (th.y * tr_exp(-(dist * sig_t.y))) / ptot,
+                   (th.z * tr_exp(-(dist * sig_t.z))) / ptot);
+        } else {
+            f = mk(th.x / ptot, th.y / ptot, th.z / ptot);
+        }
+        const float time = rd.w + dist;
+        // camera unwarp: World::Li's record distance = closest surface along the camera
+        // ray, FLT_MAX when there is none (World.h:749-766, Ray.h:74-84)
+        float cam_d = 0.0f;
+        if (film.unwarp) {
+            if (depth == 0) {
+                cam_d = hit ? h.x : 3.40282347e+38f;
+                ps.set_cam_dist(cam_d);
+            } else {
+                cam_d = ps.cam_dist();
+            }
+        }
+        const f3 org = mk(ro.x, ro.y, ro.z), dir = mk(rd.x, rd.y, rd.z);
+        const f3 pos = org + dir * dist;
+        if (!(time > total_time)) {
+            f3 nrm = mk(0.f, 0.f, 0.f), kd = mk(0.f, 0.f, 0.f);
+            bool ggx = false;
+            float alpha = 0.0f;
+            if (surface) {
+                const float4 ng = __ldg(&sc.tri_ng[id]);
+                nrm = mk(ng.x, ng.y, ng.z);
+                const uint32_t mi = __float_as_uint(ng.w);
+                const float4 m = __ldg(&sc.mats[mi]);
+                kd = mk(m.x, m.y, m.z);
+                ggx = __float_as_uint(m.w) == 1u;
+                if (ggx) alpha = __ldg(&sc.mats2[mi]).x;
+            }
+            const f3 wo = mk(-dir.x, -dir.y, -dir.z);
+            // ---- next-event estimate ----
+            {
+                const float xl = pcg_float(rng);
+                uint32_t li = (uint32_t)(xl * (float)sc.num_lights);
+                if (li >= sc.num_lights) li = sc.num_lights - 1;
+                const float4* L = sc.lights + 5 * li;
+                const float4 L0 = __ldg(L), L1 = __ldg(L + 1);
+                const bool rect = __float_as_uint(L0.w) == 1u;
+                float pl_ = 1.0f / (float)sc.num_lights;
+                f3 lp = mk(L0.x, L0.y, L0.z);
+                if (rect) {
+                    const float xu = pcg_float(rng), xv = pcg_float(rng);
+                    const float4 L2 = __ldg(L + 2), L3 = __ldg(L + 3);
+                    lp = (lp + f3of(L2) * xu) + f3of(L3) * xv;
+                    pl_ = pl_ * (1.0f / L1.w);
+                }
+                f3 ld = pos - lp;
+                const float d2 = dot(ld, ld);
+                const float dl = sqrtf(d2);
+                ld = divs(ld, dl);
+                bool ok = true;
+                f3 irr;
+                if (rect) {
+                    const float4 L4 = __ldg(L + 4);
+                    const float dot_l = dot(ld, f3of(L4));
+                    if (!(dot_l > 0.0f)) ok = false;
+                    const float a = dot_l / (dl * dl);
+                    irr = mk(L1.x * a, L1.y * a, L1.z * a);
+                } else {
+                    irr = mk(L1.x / d2, L1.y / d2, L1.z / d2);
+                }
+                if (ok) {
+                    const f3 wl = mk(-ld.x, -ld.y, -ld.z);
+                    f3 fe;
+                    if (surface && ggx) {
+                        fe = ggx_eval_cos(kd, alpha, nrm, wo, wl);
+                    } else if (surface) {
+                        const float cs = dot(wl, nrm);
+                        const float cl = cs > 0.0f ? cs : 0.0f;
+                        fe = mk((kd.x * kInvPi) * cl, (kd.y * kInvPi) * cl, (kd.z * kInvPi) * cl);
+                    } else {
+                        const float ph = hg_eval(g, dot(dir, wl));
+                        fe = mk(ph * sig_s.x, ph * sig_s.y, ph * sig_s.z);
+                    }
+                    f3 att = mk(1.0f, 1.0f, 1.0f);
+                    if (medium)
+                        att = mk(tr_exp(-(sig_t.x * dl)), tr_exp(-(sig_t.y * dl)), tr_exp(-(sig_t.z * dl)));
+                    const float scale = inv_inc / pl_;
+                    const float Lr = (f.x * (fe.x * (irr.x * att.x))) * scale;
+                    const float Lg = (f.y * (fe.y * (irr.y * att.y))) * scale;
+                    const float Lb = (f.z * (fe.z * (irr.z * att.z))) * scale;
+                    const float tt = time + dl;
+                    const float tc = film.unwarp ? tt - cam_d : tt;      // StreakCameraFilm.h:167
+                    const float ps = (tc - film.offset) / film.exposure;
+                    const bool inside = ps < (float)film.T && ps >= 0.0f;
+                    const bool fin = finite3(Lr, Lg, Lb);
+                    // with bounce films every visible light connection is a sample (its
+                    // time and radiance aside; non-finite radiance becomes 0 as in
+                    // TransientRenderer.h:165-169); otherwise only useful ones are traced
+                    if ((inside && fin && (Lr != 0.0f || Lg != 0.0f || Lb != 0.0f)) || film.nbounce) {
+                        o.shadow = true;
+                        const uint32_t bin = inside ? (uint32_t)floorf(ps) : kBinOutside;
+                        o.sh_o = make_float4(lp.x, lp.y, lp.z, dl - kSigmaVis);
+                        o.sh_d = make_float4(ld.x, ld.y, ld.z, __uint_as_float(bin | ((uint32_t)depth << 24)));
+                        o.sh_L = fin ? make_float4(Lr, Lg, Lb, __uint_as_float(slot))
+                                   : make_float4(0.0f, 0.0f, 0.0f, __uint_as_float(slot));
+                    }
+                }
+            }
+            if constexpr (kTimeSampling) {
+                // ---- bidirectional connections: keep the eye vertex (value, pdf,
+                // delay) for the connection passes (connect_paths, BidirectionalPathTracing.h:
+                // 1018-1041); scenes without a medium, so every vertex is a surface ----
+                if ((flags & kFlagBidirectional) && surface && (uint32_t)depth + 2u <= max_bounces) {
+                    const size_t cap = p.wave.capacity;
+                    float4* v = p.bd.evert + (size_t)depth * 4 * cap + slot;
+                    v[0] = make_float4(pos.x, pos.y, pos.z, time);
+                    v[cap] = make_float4(nrm.x, nrm.y, nrm.z, ptot);
+                    v[2 * cap] = make_float4(kd.x, kd.y, kd.z, 0.0f);
+                    v[3 * cap] = make_float4(f.x, f.y, f.z, 0.0f);
+                    p.bd.ne[slot] = (uint8_t)(depth + 1);
+                }
+            }
+            if ((uint32_t)depth + 1u < max_bounces) {
+                // ---- Russian roulette (none in time-sampling mode: the walk ends when
+                // its time passes the film's, above) ----
+                const float albedo = surface ? avg3(kd)
+                    : avg3(mk(sig_s.x / sig_t.x, sig_s.y / sig_t.y, sig_s.z / sig_t.z));
+                const bool tsm = kTimeSampling && (flags & kFlagTimeSampling) != 0;
+                const bool survive = tsm || !(pcg_float(rng) > albedo);
+                const float prr = tsm ? 1.0f : albedo;
+                if (kGuided && surface && survive && !(ggx && alpha < p.guide.min_alpha)) {
+                    // ---- direction deferred to the learned proposal (k_guide) ----
+                    o.guide = true;
+                    o.gv[0] = make_uint4(__float_as_uint(pos.x), __float_as_uint(pos.y), __float_as_uint(pos.z),
+                                       __float_as_uint(time));
+                    o.gv[1] = make_uint4(__float_as_uint(dir.x), __float_as_uint(dir.y), __float_as_uint(dir.z),
+                                       __float_as_uint(prr));
+                    o.gv[2] = make_uint4(__float_as_uint(f.x), __float_as_uint(f.y), __float_as_uint(f.z),
+                                       __float_as_uint(__ldg(&sc.tri_ng[id]).w));
+                    o.gv[3] = make_uint4(__float_as_uint(nrm.x), __float_as_uint(nrm.y), __float_as_uint(nrm.z), slot);
+                } else if (survive) {
+                    // ---- outgoing direction ----
+                    f3 fa, nd;
+                    float pa;
+                    bool alive = true;
+                    bool angular = false;
+                    float nds_first = 0.0f;
+                    if (tsm && !surface) {
+                        // time sampling in the medium: the next free flight r first
+                        // (generate_path, BidirectionalPathTracing.h:530-545), then the
+                        // time-angular sampler towards the path's light point with
+                        // probability 1 when its bounds leave at least one exposure
+                        // (:365-405), else (or when its density is < 1e-5) the phase
+                        // function (:408-418)
+                        nds_first = -tr_log(pcg_float(rng)) / lambda;
+                        const float4 tg = ps.target();
+                        const f3 l = mk(tg.x, tg.y, tg.z) - pos;
+                        const float mod = sqrtf(dot(l, l));
+                        const float ta = mod + time;
+                        float t_a = ta, t_b = total_time;
+                        if (nds_first > mod) t_a = fmaxf(t_a, 2.0f * nds_first - mod);
+                        else t_a = fmaxf(t_a, mod);
+                        t_b = fminf(t_b, 2.0f * nds_first + mod);
+                        const bool use_ts = !((total_time - (ta + nds_first)) < film.exposure);
+                        (void)pcg_float(rng);                          // the choice xi < p_ts
+                        if (use_ts) {
+                            const float e = pcg_float(rng), e2 = pcg_float(rng);
+                            const TaSample ts = time_angular_sample(l, mod, nds_first, t_a, t_b, e, e2, dir, g);
+                            if (ts.pa >= 1e-5f) {
+                                angular = true;
+                                nd = ts.nd;
+                                fa = mk(ts.ph * sig_s.x, ts.ph * sig_s.y, ts.ph * sig_s.z);
+                                pa = ts.pa;
+                            }
+                        }
+                    }
+                    const float x1 = angular ? 0.0f : pcg_float(rng);
+                    const float x2 = angular ? 0.0f : pcg_float(rng);
+                    float sp, cp;
+                    tr_sincos2pi(x1, &sp, &cp);
+                    if (angular) {
+                    } else if (surface && ggx) {
+                        alive = ggx_sample(kd, alpha, nrm, wo, sp, cp, x2, nd, fa, pa);
+                    } else if (surface && (flags & kFlagOrthoFrame)) {
+                        // cosine sampling in an orthonormal frame (Duff et al. 2017)
+                        const float ct = sqrtf(x2);
+                        const float stt = sqrtf(1.0f - ct * ct);
+                        const Frame3 Fr = make_frame(nrm);
+                        nd = to_world(Fr, mk(cp * stt, sp * stt, ct));
+                        fa = mk((kd.x * kInvPi) * ct, (kd.y * kInvPi) * ct, (kd.z * kInvPi) * ct);
+                        pa = ct * kInvPi;
+                    } else if (surface) {
+                        const float ct = sqrtf(x2);
+                        const float stt = sqrtf(1.0f - ct * ct);
+                        const f3 aux = fabsf(nrm.x) > fabsf(nrm.z) ? mk(-nrm.y, nrm.x, nrm.z)
+                                                                   : mk(0.0f, -nrm.z, nrm.y);
+                        const f3 tv = normalize(aux);
+                        const f3 tu = cross(nrm, tv);
+                        const f3 w = ((tu * (cp * stt)) + (nrm * ct)) + (tv * (sp * stt));
+                        nd = normalize(w);
+                        const float ca = fabsf(dot(nrm, nd));
+                        fa = mk((kd.x * kInvPi) * ca, (kd.y * kInvPi) * ca, (kd.z * kInvPi) * ca);
+                        pa = ct * kInvPi;
+                    } else {
+                        float ct;
+                        if (fabsf(g) < 1e-4f) {
+                            ct = 1.0f - 2.0f * x2;
+                        } else {
+                            const float gg = g * g;
+                            const float a = (1.0f - gg) / ((1.0f - g) + (2.0f * g) * x2);
+                            ct = ((1.0f + gg) - a * a) / (2.0f * g);
+                            if (ct < -1.0f) ct = -1.0f;
+                            if (ct > 1.0f) ct = 1.0f;
+                        }
+                        const float stt = sqrtf(1.0f - ct * ct);
+                        // orthonormal frame around the propagation direction (Duff et al. 2017)
+                        const float sg = copysignf(1.0f, dir.z);
+                        const float aa = -1.0f / (sg + dir.z);
+                        const float bb = dir.x * dir.y * aa;
+                        const f3 t1 = mk(1.0f + sg * dir.x * dir.x * aa, sg * bb, -sg * dir.x);
+                        const f3 t2 = mk(bb, sg + dir.y * dir.y * aa, -dir.y);
+                        nd = ((t1 * (cp * stt)) + (t2 * (sp * stt))) + (dir * ct);
+                        const float ph = hg_eval(g, ct);
+                        fa = mk(ph * sig_s.x, ph * sig_s.y, ph * sig_s.z);
+                        pa = ph;
+                    }
+                    if (alive) {
+                        const f3 fn = mulv(f, fa);
+                        float nds = __int_as_float(0x7f800000);
+                        if (medium) nds = (tsm && !surface) ? nds_first : -tr_log(pcg_float(rng)) / lambda;
+                        ps.next(make_float4(pos.x, pos.y, pos.z, nds), make_float4(nd.x, nd.y, nd.z, time),
+                                make_float4(fn.x, fn.y, fn.z, prr * pa), rng.state);
+                        o.next = true;
+                    }
+                }
+            }
+        }
+        if (kGuided && o.guide)
+            o.gv[4] = make_uint4((uint32_t)rng.state, (uint32_t)(rng.state >> 32), (uint32_t)rng.inc,
+                               (uint32_t)(rng.inc >> 32));
+    }
+}
+
 // Register budgets (the kernel is latency-bound, so resident warps matter more than a few
-// spilled values, which stay in L1): the plain variant 64 registers (4 CTAs per SM); the guided
-// and time-sampling variants 80 (3 CTAs per SM; unbounded they took 146-172 registers and ran
-// one CTA of 8 warps per SM); the multi-scene variants 128 (2 CTAs, no spills).
+// spilled values, which stay in L1): the plain and guided variants 64 registers (4 CTAs per SM);
+// the time-sampling and multi-scene variants 80 (3 CTAs per SM; unbounded the former took 146-172
+// registers and ran one CTA of 8 warps per SM).
 template <bool kGuided, bool kMulti, bool kTimeSampling>
 __global__ void __launch_bounds__(256, kMulti ? 3 : (kTimeSampling ? 3 : 4))
     k_shade(const __grid_constant__ Params p, int depth) {
@@ -563,11 +901,9 @@ __global__ void __launch_bounds__(256, kMulti ? 3 : (kTimeSampling ? 3 : 4))
     for (uint32_t bbase = blockIdx.x * blockDim.x; bbase < n; bbase += gridDim.x * blockDim.x) {
         const uint32_t base = bbase + (threadIdx.x & ~31u);
         const uint32_t idx = base + lane;
-        uint32_t oct = 0, soct = 0;
-        bool want_shadow = false, want_next = false, want_guide = false;
-        uint4 gv[5];                     // guided-vertex record (kGuided only)
-        uint32_t slot = 0;
-        float4 sh_o = make_float4(0, 0, 0, 0), sh_d = make_float4(0, 0, 0, 0), sh_L = make_float4(0, 0, 0, 0);
+        uint32_t oct = 0, soct = 0, slot = 0;
+        ShadeOut o;
+        o.shadow = o.next = o.guide = false;
         if (idx < n) {
             slot = depth == 0 ? idx : qin[idx];
             // the slot's segment (pixels, samples) and scene: the launch's own in single-scene
@@ -578,307 +914,12 @@ __global__ void __launch_bounds__(256, kMulti ? 3 : (kTimeSampling ? 3 : 4))
                 Bp = &seg_of_slot(cur_batch(p), slot);
                 SS = p.multi.scenes + Bp->scene;
             }
-            const Batch& B = *Bp;
-            const SceneDev& sc = kMulti ? SS->scene : p.scene;
-            const FilmDev& film = kMulti ? SS->film : p.film;
-            const uint32_t max_bounces = kMulti ? SS->max_bounces : p.max_bounces;
-            const uint32_t flags = kMulti ? SS->flags : p.flags;
-            const bool medium = sc.medium != 0;
-            const f3 sig_s = mk(sc.sig_s[0], sc.sig_s[1], sc.sig_s[2]);
-            const f3 sig_t = mk(sc.sig_t[0], sc.sig_t[1], sc.sig_t[2]);
-            const float lambda = sc.lambda;
-            const float g = sc.g;
-            const float total_time = (float)film.T * film.exposure + film.offset;
-            const float inv_inc = 1.0f / (float)B.ninc;
-            const uint32_t per_pix = B.ns * B.ninc;
-            const uint32_t lslot = slot - B.slot_begin;
-            const float2 h = p.wave.hit[slot];
-            const float4 ro = p.wave.ray_o[slot];
-            const float4 rd = p.wave.ray_d[slot];
-            const float4 th = p.wave.thr[slot];
-            const uint32_t id = __float_as_uint(h.y);
-            const bool hit = id != kInvalid;
-            const float dsamp = ro.w;
-            const bool surface = hit && (!medium || h.x < dsamp);
-            if (depth == 0 && film.comps && lslot % B.ninc == 0) {
-                // film components: one camera-ray record per camera sample (Film.h:127-145)
-                const uint32_t pl = lslot / per_pix;
-                const uint32_t wpix = B.pix_begin + pl;
-                const size_t pixel = (size_t)(B.win_y0 + wpix / B.win_w) * film.W + (B.win_x0 + wpix % B.win_w);
-                f3 cp = mk(0.f, 0.f, 0.f), cn = cp;
-                if (hit) {
-                    cp = mk(ro.x, ro.y, ro.z) + mk(rd.x, rd.y, rd.z) * h.x;
-                    const float4 ng = __ldg(&sc.tri_ng[id]);
-                    cn = mk(ng.x, ng.y, ng.z);
-                }
-                if (film.comps & 2u) atomicAdd(&film.cdepth[pixel], (double)(hit ? h.x : 3.40282347e+38f));
-                if (film.comps & 8u) {
-                    atomicAdd(&film.cpos[pixel * 3], (double)cp.x);
-                    atomicAdd(&film.cpos[pixel * 3 + 1], (double)cp.y);
-                    atomicAdd(&film.cpos[pixel * 3 + 2], (double)cp.z);
-                }
-                if (film.comps & 16u) {
-                    atomicAdd(&film.cnorm[pixel * 3], (double)cn.x);
-                    atomicAdd(&film.cnorm[pixel * 3 + 1], (double)cn.y);
-                    atomicAdd(&film.cnorm[pixel * 3 + 2], (double)cn.z);
-                }
-            }
-            if (medium || hit) {
-                // per-path RNG: state in memory, increment from the camera sample
-                const uint32_t pl = lslot / per_pix;
-                const uint32_t sl = (lslot - pl * per_pix) / B.ninc;
-                const uint32_t wpix = B.pix_begin + pl;
-                const uint32_t pixel = (B.win_y0 + wpix / B.win_w) * film.W + (B.win_x0 + wpix % B.win_w);
-                Pcg rng;
-                rng.state = p.wave.rng[slot];
-                rng.inc = (cam_id(pixel, B.s0 + sl) << 1u) | 1ull;
-
-                float dist, pd;
-                if (surface) { dist = h.x; pd = medium ? tr_exp(-(dist * lambda)) : 1.0f; }
-                else { dist = dsamp; pd = tr_exp(-(dist * lambda)) * lambda; }
-                const float ptot = th.w * pd;
-                f3 f;
-                if (medium) {
-                    f = mk((th.x * tr_exp(-(dist * sig_t.x))) / ptot, (th.y * tr_exp(-(dist * sig_t.y))) / ptot,
-                           (th.z * tr_exp(-(dist * sig_t.z))) / ptot);
-                } else {
-                    f = mk(th.x / ptot, th.y / ptot, th.z / ptot);
-                }
-                const float time = rd.w + dist;
-                // camera unwarp: World::Li's record distance = closest surface along the camera
-                // ray, FLT_MAX when there is none (World.h:749-766, Ray.h:74-84)
-                float cam_d = 0.0f;
-                if (film.unwarp) {
-                    if (depth == 0) {
-                        cam_d = hit ? h.x : 3.40282347e+38f;
-                        p.wave.cam_dist[slot] = cam_d;
-                    } else {
-                        cam_d = p.wave.cam_dist[slot];
-                    }
-                }
-                const f3 org = mk(ro.x, ro.y, ro.z), dir = mk(rd.x, rd.y, rd.z);
-                const f3 pos = org + dir * dist;
-                if (!(time > total_time)) {
-                    f3 nrm = mk(0.f, 0.f, 0.f), kd = mk(0.f, 0.f, 0.f);
-                    bool ggx = false;
-                    float alpha = 0.0f;
-                    if (surface) {
-                        const float4 ng = __ldg(&sc.tri_ng[id]);
-                        nrm = mk(ng.x, ng.y, ng.z);
-                        const uint32_t mi = __float_as_uint(ng.w);
-                        const float4 m = __ldg(&sc.mats[mi]);
-                        kd = mk(m.x, m.y, m.z);
-                        ggx = __float_as_uint(m.w) == 1u;
-                        if (ggx) alpha = __ldg(&sc.mats2[mi]).x;
-                    }
-                    const f3 wo = mk(-dir.x, -dir.y, -dir.z);
-                    // ---- next-event estimate ----
-                    {
-                        const float xl = pcg_float(rng);
-                        uint32_t li = (uint32_t)(xl * (float)sc.num_lights);
-                        if (li >= sc.num_lights) li = sc.num_lights - 1;
-                        const float4* L = sc.lights + 5 * li;
-                        const float4 L0 = __ldg(L), L1 = __ldg(L + 1);
-                        const bool rect = __float_as_uint(L0.w) == 1u;
-                        float pl_ = 1.0f / (float)sc.num_lights;
-                        f3 lp = mk(L0.x, L0.y, L0.z);
-                        if (rect) {
-                            const float xu = pcg_float(rng), xv = pcg_float(rng);
-                            const float4 L2 = __ldg(L + 2), L3 = __ldg(L + 3);
-                            lp = (lp + f3of(L2) * xu) + f3of(L3) * xv;
-                            pl_ = pl_ * (1.0f / L1.w);
-                        }
-                        f3 ld = pos - lp;
-                        const float d2 = dot(ld, ld);
-                        const float dl = sqrtf(d2);
-                        ld = divs(ld, dl);
-                        bool ok = true;
-                        f3 irr;
-                        if (rect) {
-                            const float4 L4 = __ldg(L + 4);
-                            const float dot_l = dot(ld, f3of(L4));
-                            if (!(dot_l > 0.0f)) ok = false;
-                            const float a = dot_l / (dl * dl);
-                            irr = mk(L1.x * a, L1.y * a, L1.z * a);
-                        } else {
-                            irr = mk(L1.x / d2, L1.y / d2, L1.z / d2);
-                        }
-                        if (ok) {
-                            const f3 wl = mk(-ld.x, -ld.y, -ld.z);
-                            f3 fe;
-                            if (surface && ggx) {
-                                fe = ggx_eval_cos(kd, alpha, nrm, wo, wl);
-                            } else if (surface) {
-                                const float cs = dot(wl, nrm);
-                                const float cl = cs > 0.0f ? cs : 0.0f;
-                                fe = mk((kd.x * kInvPi) * cl, (kd.y * kInvPi) * cl, (kd.z * kInvPi) * cl);
-                            } else {
-                                const float ph = hg_eval(g, dot(dir, wl));
-                                fe = mk(ph * sig_s.x, ph * sig_s.y, ph * sig_s.z);
-                            }
-                            f3 att = mk(1.0f, 1.0f, 1.0f);
-                            if (medium)
-                                att = mk(tr_exp(-(sig_t.x * dl)), tr_exp(-(sig_t.y * dl)), tr_exp(-(sig_t.z * dl)));
-                            const float scale = inv_inc / pl_;
-                            const float Lr = (f.x * (fe.x * (irr.x * att.x))) * scale;
-                            const float Lg = (f.y * (fe.y * (irr.y * att.y))) * scale;
-                            const float Lb = (f.z * (fe.z * (irr.z * att.z))) * scale;
-                            const float tt = time + dl;
-                            const float tc = film.unwarp ? tt - cam_d : tt;      // StreakCameraFilm.h:167
-                            const float ps = (tc - film.offset) / film.exposure;
-                            const bool inside = ps < (float)film.T && ps >= 0.0f;
-                            const bool fin = finite3(Lr, Lg, Lb);
-                            // with bounce films every visible light connection is a sample (its
-                            // time and radiance aside; non-finite radiance becomes 0 as in
-                            // TransientRenderer.h:165-169); otherwise only useful ones are traced
-                            if ((inside && fin && (Lr != 0.0f || Lg != 0.0f || Lb != 0.0f)) || film.nbounce) {
-                                want_shadow = true;
-                                soct = (ld.x < 0.0f ? 1u : 0u) | (ld.y < 0.0f ? 2u : 0u) | (ld.z < 0.0f ? 4u : 0u);
-                                const uint32_t bin = inside ? (uint32_t)floorf(ps) : kBinOutside;
-                                sh_o = make_float4(lp.x, lp.y, lp.z, dl - kSigmaVis);
-                                sh_d = make_float4(ld.x, ld.y, ld.z, __uint_as_float(bin | ((uint32_t)depth << 24)));
-                                sh_L = fin ? make_float4(Lr, Lg, Lb, __uint_as_float(slot))
-                                           : make_float4(0.0f, 0.0f, 0.0f, __uint_as_float(slot));
-                            }
-                        }
-                    }
-                    if constexpr (kTimeSampling) {
-                        // ---- bidirectional connections: keep the eye vertex (value, pdf,
-                        // delay) for the connection passes (connect_paths, BidirectionalPathTracing.h:
-                        // 1018-1041); scenes without a medium, so every vertex is a surface ----
-                        if ((flags & kFlagBidirectional) && surface && (uint32_t)depth + 2u <= max_bounces) {
-                            const size_t cap = p.wave.capacity;
-                            float4* v = p.bd.evert + (size_t)depth * 4 * cap + slot;
-                            v[0] = make_float4(pos.x, pos.y, pos.z, time);
-                            v[cap] = make_float4(nrm.x, nrm.y, nrm.z, ptot);
-                            v[2 * cap] = make_float4(kd.x, kd.y, kd.z, 0.0f);
-                            v[3 * cap] = make_float4(f.x, f.y, f.z, 0.0f);
-                            p.bd.ne[slot] = (uint8_t)(depth + 1);
-                        }
-                    }
-                    if ((uint32_t)depth + 1u < max_bounces) {
-                        // ---- Russian roulette (none in time-sampling mode: the walk ends when
-                        // its time passes the film's, above) ----
-                        const float albedo = surface ? avg3(kd)
-                            : avg3(mk(sig_s.x / sig_t.x, sig_s.y / sig_t.y, sig_s.z / sig_t.z));
-                        const bool tsm = kTimeSampling && (flags & kFlagTimeSampling) != 0;
-                        const bool survive = tsm || !(pcg_float(rng) > albedo);
-                        const float prr = tsm ? 1.0f : albedo;
-                        if (kGuided && surface && survive && !(ggx && alpha < p.guide.min_alpha)) {
-                            // ---- direction deferred to the learned proposal (k_guide) ----
-                            want_guide = true;
-                            gv[0] = make_uint4(__float_as_uint(pos.x), __float_as_uint(pos.y), __float_as_uint(pos.z),
-                                               __float_as_uint(time));
-                            gv[1] = make_uint4(__float_as_uint(dir.x), __float_as_uint(dir.y), __float_as_uint(dir.z),
-                                               __float_as_uint(prr));
-                            gv[2] = make_uint4(__float_as_uint(f.x), __float_as_uint(f.y), __float_as_uint(f.z),
-                                               __float_as_uint(__ldg(&sc.tri_ng[id]).w));
-                            gv[3] = make_uint4(__float_as_uint(nrm.x), __float_as_uint(nrm.y), __float_as_uint(nrm.z), slot);
-                        } else if (survive) {
-                            // ---- outgoing direction ----
-                            f3 fa, nd;
-                            float pa;
-                            bool alive = true;
-                            bool angular = false;
-                            float nds_first = 0.0f;
-                            if (tsm && !surface) {
-                                // time sampling in the medium: the next free flight r first
-                                // (generate_path, BidirectionalPathTracing.h:530-545), then the
-                                // time-angular sampler towards the path's light point with
-                                // probability 1 when its bounds leave at least one exposure
-                                // (:365-405), else (or when its density is < 1e-5) the phase
-                                // function (:408-418)
-                                nds_first = -tr_log(pcg_float(rng)) / lambda;
-                                const float4 tg = p.wave.target[slot];
-                                const f3 l = mk(tg.x, tg.y, tg.z) - pos;
-                                const float mod = sqrtf(dot(l, l));
-                                const float ta = mod + time;
-                                float t_a = ta, t_b = total_time;
-                                if (nds_first > mod) t_a = fmaxf(t_a, 2.0f * nds_first - mod);
-                                else t_a = fmaxf(t_a, mod);
-                                t_b = fminf(t_b, 2.0f * nds_first + mod);
-                                const bool use_ts = !((total_time - (ta + nds_first)) < film.exposure);
-                                (void)pcg_float(rng);                          // the choice xi < p_ts
-                                if (use_ts) {
-                                    const float e = pcg_float(rng), e2 = pcg_float(rng);
-                                    const TaSample ts = time_angular_sample(l, mod, nds_first, t_a, t_b, e, e2, dir, g);
-                                    if (ts.pa >= 1e-5f) {
-                                        angular = true;
-                                        nd = ts.nd;
-                                        fa = mk(ts.ph * sig_s.x, ts.ph * sig_s.y, ts.ph * sig_s.z);
-                                        pa = ts.pa;
-                                    }
-                                }
-                            }
-                            const float x1 = angular ? 0.0f : pcg_float(rng);
-                            const float x2 = angular ? 0.0f : pcg_float(rng);
-                            float sp, cp;
-                            tr_sincos2pi(x1, &sp, &cp);
-                            if (angular) {
-                            } else if (surface && ggx) {
-                                alive = ggx_sample(kd, alpha, nrm, wo, sp, cp, x2, nd, fa, pa);
-                            } else if (surface && (flags & kFlagOrthoFrame)) {
-                                // cosine sampling in an orthonormal frame (Duff et al. 2017)
-                                const float ct = sqrtf(x2);
-                                const float stt = sqrtf(1.0f - ct * ct);
-                                const Frame3 Fr = make_frame(nrm);
-                                nd = to_world(Fr, mk(cp * stt, sp * stt, ct));
-                                fa = mk((kd.x * kInvPi) * ct, (kd.y * kInvPi) * ct, (kd.z * kInvPi) * ct);
-                                pa = ct * kInvPi;
-                            } else if (surface) {
-                                const float ct = sqrtf(x2);
-                                const float stt = sqrtf(1.0f - ct * ct);
-                                const f3 aux = fabsf(nrm.x) > fabsf(nrm.z) ? mk(-nrm.y, nrm.x, nrm.z)
-                                                                           : mk(0.0f, -nrm.z, nrm.y);
-                                const f3 tv = normalize(aux);
-                                const f3 tu = cross(nrm, tv);
-                                const f3 w = ((tu * (cp * stt)) + (nrm * ct)) + (tv * (sp * stt));
-                                nd = normalize(w);
-                                const float ca = fabsf(dot(nrm, nd));
-                                fa = mk((kd.x * kInvPi) * ca, (kd.y * kInvPi) * ca, (kd.z * kInvPi) * ca);
-                                pa = ct * kInvPi;
-                            } else {
-                                float ct;
-                                if (fabsf(g) < 1e-4f) {
-                                    ct = 1.0f - 2.0f * x2;
-                                } else {
-                                    const float gg = g * g;
-                                    const float a = (1.0f - gg) / ((1.0f - g) + (2.0f * g) * x2);
-                                    ct = ((1.0f + gg) - a * a) / (2.0f * g);
-                                    if (ct < -1.0f) ct = -1.0f;
-                                    if (ct > 1.0f) ct = 1.0f;
-                                }
-                                const float stt = sqrtf(1.0f - ct * ct);
-                                // orthonormal frame around the propagation direction (Duff et al. 2017)
-                                const float sg = copysignf(1.0f, dir.z);
-                                const float aa = -1.0f / (sg + dir.z);
-                                const float bb = dir.x * dir.y * aa;
-                                const f3 t1 = mk(1.0f + sg * dir.x * dir.x * aa, sg * bb, -sg * dir.x);
-                                const f3 t2 = mk(bb, sg + dir.y * dir.y * aa, -dir.y);
-                                nd = ((t1 * (cp * stt)) + (t2 * (sp * stt))) + (dir * ct);
-                                const float ph = hg_eval(g, ct);
-                                fa = mk(ph * sig_s.x, ph * sig_s.y, ph * sig_s.z);
-                                pa = ph;
-                            }
-                            if (alive) {
-                                const f3 fn = mulv(f, fa);
-                                float nds = __int_as_float(0x7f800000);
-                                if (medium) nds = (tsm && !surface) ? nds_first : -tr_log(pcg_float(rng)) / lambda;
-                                p.wave.ray_o[slot] = make_float4(pos.x, pos.y, pos.z, nds);
-                                p.wave.ray_d[slot] = make_float4(nd.x, nd.y, nd.z, time);
-                                p.wave.thr[slot] = make_float4(fn.x, fn.y, fn.z, prr * pa);
-                                want_next = true;
-                                oct = (nd.x < 0.0f ? 1u : 0u) | (nd.y < 0.0f ? 2u : 0u) | (nd.z < 0.0f ? 4u : 0u);
-                            }
-                        }
-                    }
-                }
-                if (kGuided && want_guide)
-                    gv[4] = make_uint4((uint32_t)rng.state, (uint32_t)(rng.state >> 32), (uint32_t)rng.inc,
-                                       (uint32_t)(rng.inc >> 32));
-                else
-                    p.wave.rng[slot] = rng.state;
-            }
+            WaveState ps{p, slot, 0u};
+            shade_vertex<kGuided, kTimeSampling>(p, depth, slot, *Bp, kMulti ? SS->scene : p.scene,
+                                                 kMulti ? SS->film : p.film, kMulti ? SS->max_bounces : p.max_bounces,
+                                                 kMulti ? SS->flags : p.flags, p.wave.hit[slot], ps, o);
+            oct = ps.octant;
+            soct = o.shadow ? (o.sh_d.x < 0.0f ? 1u : 0u) | (o.sh_d.y < 0.0f ? 2u : 0u) | (o.sh_d.z < 0.0f ? 4u : 0u) : 0u;
         }
         // ---- shadow queue: warp-aggregated appends (order preserved within the warp) ----
         const unsigned lt = lanemask_lt();
@@ -888,36 +929,136 @@ __global__ void __launch_bounds__(256, kMulti ? 3 : (kTimeSampling ? 3 : 4))
         if (threadIdx.x < 8) { oc[threadIdx.x] = 0; sc8[threadIdx.x] = 0; }
         __syncthreads();
         uint32_t rk = 0, rs = 0;
-        if (want_next) rk = atomicAdd(&oc[oct], 1u);
-        if (want_shadow) rs = atomicAdd(&sc8[soct], 1u);
+        if (o.next) rk = atomicAdd(&oc[oct], 1u);
+        if (o.shadow) rs = atomicAdd(&sc8[soct], 1u);
         __syncthreads();
         if (threadIdx.x == 0) {
             uint32_t tot = 0, tsh = 0;
-            for (int o = 0; o < 8; ++o) { ob[o] = tot; tot += oc[o]; sb8[o] = tsh; tsh += sc8[o]; }
+            for (int k = 0; k < 8; ++k) { ob[k] = tot; tot += oc[k]; sb8[k] = tsh; tsh += sc8[k]; }
             const uint32_t g0 = tot ? atomicAdd(&p.wave.counters[cnt_ext(depth + 1)], tot) : 0u;
             const uint32_t s0 = tsh ? atomicAdd(&p.wave.counters[cnt_sh(depth)], tsh) : 0u;
-            for (int o = 0; o < 8; ++o) { ob[o] += g0; sb8[o] += s0; }
+            for (int k = 0; k < 8; ++k) { ob[k] += g0; sb8[k] += s0; }
         }
         __syncthreads();
-        if (want_shadow) {
+        if (o.shadow) {
             const uint32_t k = sb8[soct] + rs;
-            p.wave.sh_o[k] = sh_o;
-            p.wave.sh_d[k] = sh_d;
-            p.wave.sh_L[k] = sh_L;
+            p.wave.sh_o[k] = o.sh_o;
+            p.wave.sh_d[k] = o.sh_d;
+            p.wave.sh_L[k] = o.sh_L;
         }
-        if (want_next) qout[ob[oct] + rk] = slot;
+        if (o.next) qout[ob[oct] + rk] = slot;
         if (kGuided) {
-            const unsigned mg = __ballot_sync(kFull, want_guide);
+            const unsigned mg = __ballot_sync(kFull, o.guide);
             uint32_t bg = 0;
             if (lane == 0 && mg) bg = atomicAdd(&p.wave.counters[cnt_guide(depth)], (uint32_t)__popc(mg));
             bg = __shfl_sync(kFull, bg, 0);
-            if (want_guide) {
+            if (o.guide) {
                 uint4* r = p.guide.vrec + (size_t)(bg + (uint32_t)__popc(mg & lt)) * 5;
 #pragma unroll
-                for (int q = 0; q < 5; ++q) r[q] = gv[q];
+                for (int q = 0; q < 5; ++q) r[q] = o.gv[q];
             }
         }
     }
+}
+
+// -----------------------------------------------------------------------------------------
+// Whole paths in one launch, for batches that do not fill the GPU (launch_paths).  Two neighbouring
+// lanes own a path: the even one walks it (camera ray, closest hits, vertices), the odd one casts the
+// shadow ray of the vertex before beside the walk's next closest-hit query and writes the splat
+// record.  The vertices, rays and records are those of the wavefront kernels.
+//
+// A wavefront launch over few rays lasts as long as its longest ray (50-60 us over 20 k triangles)
+// and a batch of depth D waits for 2 D of them; here a warp waits only for its own paths, and the
+// paths are spread over as many warps as are resident, so their rays share a warp with few others.
+// Bound by the dependent loads of the longest paths.  Measured (16 samples per pixel, depth 8):
+// 16 k / 65 k paths of the 34-triangle room 240 -> 115 / 252 -> 200 us, over 20 k triangles 455 -> 150
+// / 510 -> 280 us, over 328 k triangles 580 -> 190 / 770 -> 350 us.  Lanes whose path has ended stay
+// idle until their group of paths is done: refilling them (other depths, other directions) made
+// 131 k paths over 328 k triangles 448 -> 561 us.
+// -----------------------------------------------------------------------------------------
+constexpr int kPathMinBlocks = 5;    // 96 registers; 4 and 6 blocks per SM are within 5 %
+struct RegState {
+    float4 o, d, t, light;
+    unsigned long long rn;
+    float cam;
+    __device__ float4 ray_o() const { return o; }
+    __device__ float4 ray_d() const { return d; }
+    __device__ float4 thr() const { return t; }
+    __device__ unsigned long long rng() const { return rn; }
+    __device__ float4 target() const { return light; }
+    __device__ float cam_dist() const { return cam; }
+    __device__ void set_cam_dist(float v) { cam = v; }
+    __device__ void next(float4 no, float4 nd, float4 nt, unsigned long long r) { o = no; d = nd; t = nt; rn = r; }
+};
+__device__ __forceinline__ float4 shfl4(float4 v, int src) {
+    return make_float4(__shfl_sync(kFull, v.x, src), __shfl_sync(kFull, v.y, src), __shfl_sync(kFull, v.z, src),
+                       __shfl_sync(kFull, v.w, src));
+}
+template <bool kTimeSampling>
+__global__ void __launch_bounds__(kTraceBlock, kPathMinBlocks) k_path(const __grid_constant__ Params p, uint32_t per_warp) {
+    extern __shared__ int stack[];     // [stack entries][kTraceBlock]
+    __shared__ uint32_t totals[3];
+    if (threadIdx.x < 3) totals[threadIdx.x] = 0;
+    __syncthreads();
+    const int lane = (int)(threadIdx.x & 31u);
+    const bool shadow = (lane & 1) != 0;
+    const uint32_t w = blockIdx.x * (kTraceBlock / 32u) + (threadIdx.x >> 5), nw = gridDim.x * (kTraceBlock / 32u);
+    const uint32_t n = p.batch.n_slots;
+    const size_t rs = p.wave.capacity;          // record stride: records are [bounce][slot]
+    uint32_t rays = 0, splats = 0;
+    for (uint32_t group = w; (unsigned long long)group * per_warp < n; group += nw) {
+        const uint32_t slot = group * per_warp + (uint32_t)(lane >> 1);
+        const bool have = (uint32_t)(lane >> 1) < per_warp && slot < n;
+        // the ray to trace next: the walk's, or the shadow ray (its contribution in ps.t)
+        RegState ps;
+        bool busy = false;
+        uint32_t records = 0;
+        if (have && !shadow && p.max_bounces) {
+            const CameraPath cp = camera_path(slot, p.batch, p.film, p.cam, p.scene, p.seed, p.sqrt_spp, p.flags);
+            ps.o = cp.o; ps.d = cp.d; ps.rn = cp.rng; ps.light = cp.target;
+            ps.t = make_float4(1.0f, 1.0f, 1.0f, 1.0f);
+            busy = true;
+        }
+        for (int depth = 0; __any_sync(kFull, busy); ++depth) {
+            Trav st;
+            if (busy) {
+                WRay r;
+                wray_setup(r, mk(ps.o.x, ps.o.y, ps.o.z), mk(ps.d.x, ps.d.y, ps.d.z), kSigmaVis);
+                const SlabRay sr = slab_setup(p.scene, r.o, r.d, kSigmaVis);
+                trav_init(st, depth == 0 && (p.film.unwarp || p.film.comps) ? __int_as_float(0x7f800000) : ps.o.w);
+                trav_run<false>(p.scene, r, sr, st, stack + threadIdx.x, kTraceBlock, 0x7fffffff, nullptr, shadow);
+                ++rays;
+            }
+            __syncwarp();
+            ShadeOut o;
+            o.shadow = o.next = false;
+            if (busy) {
+                if (shadow) {
+                    if (st.bid == kInvalid) {
+                        p.wave.rec[(size_t)records * rs + slot] = make_float4(ps.t.x, ps.t.y, ps.t.z, ps.d.w);
+                        ++records;
+                    }
+                } else {
+                    shade_vertex<false, kTimeSampling>(p, depth, slot, p.batch, p.scene, p.film, p.max_bounces, p.flags,
+                                                       make_float2(st.best, __uint_as_float(st.bid)), ps, o);
+                }
+            }
+            __syncwarp();
+            const bool cast = __shfl_sync(kFull, (int)o.shadow, lane & ~1) != 0;
+            const float4 so = shfl4(o.sh_o, lane & ~1), sd = shfl4(o.sh_d, lane & ~1), sl = shfl4(o.sh_L, lane & ~1);
+            if (shadow) { ps.o = so; ps.d = sd; ps.t = sl; }
+            busy = shadow ? cast : o.next;
+        }
+        if (have && shadow) {
+            p.wave.rec_n[slot] = (uint8_t)records;
+            splats += records;
+        }
+    }
+    const uint32_t walks = __reduce_add_sync(kFull, shadow ? 0u : rays), casts = __reduce_add_sync(kFull, shadow ? rays : 0u);
+    splats = __reduce_add_sync(kFull, splats);
+    if (lane == 0) { atomicAdd(&totals[0], walks); atomicAdd(&totals[1], casts); atomicAdd(&totals[2], splats); }
+    __syncthreads();
+    if (threadIdx.x < 3 && totals[threadIdx.x]) atomicAdd(&p.wave.stats[threadIdx.x], (unsigned long long)totals[threadIdx.x]);
 }
 
 // -----------------------------------------------------------------------------------------
@@ -1594,6 +1735,28 @@ cudaError_t launch_shade(const Params& p, int depth, cudaStream_t s) {
             else k_shade<false, false, false><<<grid, block, 0, s>>>(p, depth);
         }
     }
+    return cudaGetLastError();
+}
+// The line lies where a batch's wavefront launches start to be bound by their rays rather than by
+// their longest one, which comes later the deeper the tree: 32 k paths per level of four-child
+// nodes.  Both sides there: 34 triangles (3 levels) 98 k paths 253 us each way (131 k: 269 wavefront,
+// 288 here); 20 k triangles (10 levels) 262 k: 690 / 660, 524 k: 845 / 1190; 328 k triangles (12
+// levels) 262 k: 1000 / 762, 524 k: 1165 / 1400.
+bool paths_fit(const Params& p) {
+    return p.batch.n_slots <= 32768u * (p.bvh_depth / 3u) && !p.multi.scenes && !p.guide.vrec && !p.bd.ne;
+}
+cudaError_t launch_paths(const Params& p, cudaStream_t s) {
+    if (reinterpret_cast<uintptr_t>(p.scene.nodes) & 31u) return cudaErrorMisalignedAddress;
+    int dev = 0, sms = 1;
+    cudaGetDevice(&dev);
+    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+    const uint32_t warps = (uint32_t)sms * kPathMinBlocks * (kTraceBlock / 32u);
+    const uint32_t n = p.batch.n_slots;
+    const uint32_t per_warp = std::min(16u, std::max(1u, (n + warps - 1) / warps));
+    const uint32_t per_block = per_warp * (kTraceBlock / 32u);
+    const uint32_t grid = std::max(1u, std::min((n + per_block - 1) / per_block, warps / (kTraceBlock / 32u)));
+    if (p.flags & kFlagTimeSampling) k_path<true><<<grid, kTraceBlock, trace_smem_bytes(p.bvh_depth), s>>>(p, per_warp);
+    else k_path<false><<<grid, kTraceBlock, trace_smem_bytes(p.bvh_depth), s>>>(p, per_warp);
     return cudaGetLastError();
 }
 cudaError_t launch_shadow(const Params& p, int depth, int grid, cudaStream_t s) {

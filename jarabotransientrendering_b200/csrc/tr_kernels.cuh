@@ -236,6 +236,9 @@ cudaError_t launch_raygen(const Params& p, cudaStream_t s);
 cudaError_t launch_extend(const Params& p, int depth, int grid, cudaStream_t s);
 cudaError_t launch_shade(const Params& p, int depth, cudaStream_t s);
 cudaError_t launch_shadow(const Params& p, int depth, int grid, cudaStream_t s);
+// whole paths (camera ray to last record) of a batch in one launch: for batches that paths_fit takes
+bool paths_fit(const Params& p);
+cudaError_t launch_paths(const Params& p, cudaStream_t s);
 // bsel < 0: the film itself; bsel = b: per-bounce film b (records of bounce min(depth, N-1) == b)
 // pixels per splat block: automatic (whole pixels filling one block) in single-scene mode,
 // each segment's splat_g in multi-scene mode
