@@ -148,6 +148,27 @@ size_t pool_idle_bytes(int device) {
     return reserved > used ? (size_t)(reserved - used) : 0;
 }
 
+size_t carve_wave(trk::Wave* w, void* block, uint32_t capacity, size_t R, bool time_sampling) {
+    size_t at = 0;
+    trk::Wave dummy{};
+    trk::Wave& v = w ? *w : dummy;
+    auto take = [&](auto*& p, size_t count) {
+        using T = std::remove_reference_t<decltype(*p)>;
+        p = reinterpret_cast<T*>(reinterpret_cast<uintptr_t>(block) + at);
+        at = (at + count * sizeof(T) + 255) & ~size_t(255);
+    };
+    const size_t n = capacity;
+    take(v.ray_o, n); take(v.ray_d, n); take(v.thr, n); take(v.rng, n); take(v.hit, n);
+    take(v.q[0], n); take(v.q[1], n);
+    take(v.sh_o, n); take(v.sh_d, n); take(v.sh_L, n);
+    take(v.rec, n * R); take(v.rec_n, n); take(v.cam_dist, n);
+    if (time_sampling) take(v.target, n);
+    else v.target = nullptr;
+    v.block = block;
+    v.capacity = capacity;
+    return at;
+}
+
 void ensure_wave(tr_ctx* x, uint32_t capacity) {
     if (x->wave.capacity >= capacity) return;
     // grow: drop the old buffers (they are only scratch between calls)
@@ -157,28 +178,15 @@ void ensure_wave(tr_ctx* x, uint32_t capacity) {
         x->allocs.erase(std::remove(x->allocs.begin(), x->allocs.end(), p), x->allocs.end());
     };
     trk::Wave& w = x->wave;
-    drop(w.ray_o); drop(w.ray_d); drop(w.thr); drop(w.rng); drop(w.hit); drop(w.q[0]); drop(w.q[1]);
-    drop(w.sh_o); drop(w.sh_d); drop(w.sh_L); drop(w.rec); drop(w.rec_n);
+    drop(w.block);
+    w.block = nullptr;
+    w.capacity = 0;
     size_t R = std::max<uint32_t>(1u, x->integ.max_bounces);
     // records per slot: one next-event estimate per bounce, plus with light subpaths one per
     // eye-light vertex pair with ie + il + 2 <= max_bounces
     if (x->integ.flags & TR_FLAG_BIDIRECTIONAL) R += R * (R - 1) / 2;
-    w.ray_o = x->alloc<float4>(capacity);
-    w.ray_d = x->alloc<float4>(capacity);
-    w.thr = x->alloc<float4>(capacity);
-    w.rng = x->alloc<unsigned long long>(capacity);
-    w.hit = x->alloc<float2>(capacity);
-    w.q[0] = x->alloc<uint32_t>(capacity);
-    w.q[1] = x->alloc<uint32_t>(capacity);
-    w.sh_o = x->alloc<float4>(capacity);
-    w.sh_d = x->alloc<float4>(capacity);
-    w.sh_L = x->alloc<float4>(capacity);
-    w.rec = x->alloc<float4>((size_t)capacity * R);
-    w.rec_n = x->alloc<uint8_t>(capacity);
-    drop(w.cam_dist);
-    w.cam_dist = x->alloc<float>(capacity);
-    drop(w.target);
-    w.target = (x->integ.flags & TR_FLAG_TIME_SAMPLING) ? x->alloc<float4>(capacity) : nullptr;
+    const bool tsm = (x->integ.flags & TR_FLAG_TIME_SAMPLING) != 0;
+    void* block = x->alloc<unsigned char>(carve_wave(nullptr, nullptr, capacity, R, tsm));
     if (x->integ.flags & TR_FLAG_BIDIRECTIONAL) {
         // light wave (own rays, queues, counters; shares target and ray counts) and the
         // subpath vertex arrays
@@ -216,7 +224,7 @@ void ensure_wave(tr_ctx* x, uint32_t capacity) {
         w.stats = x->alloc<unsigned long long>(8);
         TR_CUDA(cudaMemsetAsync(w.stats, 0, 8 * sizeof(unsigned long long), x->s()));
     }
-    w.capacity = capacity;
+    carve_wave(&w, block, capacity, R, tsm);
 }
 
 // Per-kind kernel times of the pending timed launches and the union of the traversal (extend,
@@ -269,26 +277,15 @@ void ensure_lane_wave(tr_ctx* x, int k) {
         cudaFree(p);
         x->allocs.erase(std::remove(x->allocs.begin(), x->allocs.end(), p), x->allocs.end());
     };
-    drop(w.ray_o); drop(w.ray_d); drop(w.thr); drop(w.rng); drop(w.hit); drop(w.q[0]); drop(w.q[1]);
-    drop(w.sh_o); drop(w.sh_d); drop(w.sh_L); drop(w.rec); drop(w.rec_n); drop(w.cam_dist); drop(w.target);
+    drop(w.block);
+    w.block = nullptr;
+    w.capacity = 0;
     const size_t R = std::max<uint32_t>(1u, x->integ.max_bounces);
-    w.ray_o = x->alloc<float4>(capacity);
-    w.ray_d = x->alloc<float4>(capacity);
-    w.thr = x->alloc<float4>(capacity);
-    w.rng = x->alloc<unsigned long long>(capacity);
-    w.hit = x->alloc<float2>(capacity);
-    w.q[0] = x->alloc<uint32_t>(capacity);
-    w.q[1] = x->alloc<uint32_t>(capacity);
-    w.sh_o = x->alloc<float4>(capacity);
-    w.sh_d = x->alloc<float4>(capacity);
-    w.sh_L = x->alloc<float4>(capacity);
-    w.rec = x->alloc<float4>((size_t)capacity * R);
-    w.rec_n = x->alloc<uint8_t>(capacity);
-    w.cam_dist = x->alloc<float>(capacity);
-    w.target = (x->integ.flags & TR_FLAG_TIME_SAMPLING) ? x->alloc<float4>(capacity) : nullptr;
+    const bool tsm = (x->integ.flags & TR_FLAG_TIME_SAMPLING) != 0;
+    void* block = x->alloc<unsigned char>(carve_wave(nullptr, nullptr, capacity, R, tsm));
     if (!w.counters) w.counters = x->alloc<uint32_t>(trk::kCounters);
     w.stats = x->wave.stats;
-    w.capacity = capacity;
+    carve_wave(&w, block, capacity, R, tsm);
 }
 
 // Lane k + 1's guided-vertex records (the training pool and its counters are shared: the
@@ -400,9 +397,11 @@ tr_status render_region(tr_ctx* x, uint32_t x0, uint32_t y0, uint32_t x1, uint32
     const uint32_t cap_max = (x->integ.flags & TR_FLAG_BIDIRECTIONAL) ? kDefaultCapacity / 2 : kDefaultCapacity;
     uint32_t cap = (uint32_t)std::min<uint64_t>(total_slots, cap_max);
     cap = std::max<uint32_t>(cap, ninc);
-    ensure_wave(x, cap);
     const bool guided = x->guide != nullptr;
     const bool bidir = (x->integ.flags & TR_FLAG_BIDIRECTIONAL) != 0;
+    // small renders: whole paths in one launch (per-kernel times need the kernels apart)
+    const bool whole = trk::paths_fit(total_slots, x->bvh_depth) && !guided && !bidir && !x->profiling;
+    ensure_wave(x, cap);
     if (guided) {
         ensure_guided(x, cap);
         // about 1.5 guided vertices per path; keep enough of them to fill the training pool
@@ -531,8 +530,6 @@ tr_status render_region(tr_ctx* x, uint32_t x0, uint32_t y0, uint32_t x1, uint32
             p.batch.pix_begin = (uint32_t)pb; p.batch.npix = npix;
             p.batch.s0 = s0 + sb; p.batch.ns = ns; p.batch.ninc = ninc;
             p.batch.n_slots = npix * per_pix;
-            // small batches: whole paths in one launch (per-kernel times need the kernels apart)
-            const bool whole = trk::paths_fit(p) && !x->profiling;
             if (whole) {
                 tl(1, [&] { return trk::launch_paths(p, ls); });
             } else {
@@ -686,11 +683,7 @@ tr_status render_region(tr_ctx* x, uint32_t x0, uint32_t y0, uint32_t x1, uint32
     x->stats.kernel_launches = launches;
     x->stats.extend_launches = ext_l;
     x->stats.shadow_launches = sh_l;
-    unsigned long long st[8];
-    TR_CUDA(cudaMemcpy(st, x->wave.stats, sizeof(st), cudaMemcpyDeviceToHost));
-    x->stats.closest_rays = st[0];
-    x->stats.shadow_rays = st[1];
-    x->stats.splats = st[2];
+    // the ray and splat counters stay on the device until tr_stats_get reads them
     x->stats.paths += total_slots;
     x->stats.camera_samples += win_pix * ns_total;
     x->stats.render_ms = ms;
@@ -1318,7 +1311,7 @@ extern "C" tr_status tr_render_region_noalloc(tr_ctx* x, uint32_t x0, uint32_t y
         p.batch.pix_begin = 0; p.batch.npix = (uint32_t)npix;
         p.batch.s0 = s0; p.batch.ns = ns; p.batch.ninc = x->integ.incoming_samples;
         p.batch.n_slots = (uint32_t)paths;
-        if (trk::paths_fit(p)) {
+        if (trk::paths_fit(paths, x->bvh_depth)) {
             TR_CUDA(trk::launch_paths(p, strm));
         } else {
             TR_CUDA(trk::launch_raygen(p, strm));

@@ -171,26 +171,13 @@ void ensure_batch_wave(tr_batch* b, uint32_t capacity) {
 
 // one lane's wave buffers; `stats` null: allocate the statistics counters, else share them
 void ensure_lane(tr_batch* b, trk::Wave& w, uint32_t capacity, unsigned long long* stats) {
-    b->drop(w.ray_o); b->drop(w.ray_d); b->drop(w.thr); b->drop(w.rng); b->drop(w.hit); b->drop(w.q[0]);
-    b->drop(w.q[1]); b->drop(w.sh_o); b->drop(w.sh_d); b->drop(w.sh_L); b->drop(w.rec); b->drop(w.rec_n);
-    w.ray_o = b->alloc<float4>(capacity);
-    w.ray_d = b->alloc<float4>(capacity);
-    w.thr = b->alloc<float4>(capacity);
-    w.rng = b->alloc<unsigned long long>(capacity);
-    w.hit = b->alloc<float2>(capacity);
-    w.q[0] = b->alloc<uint32_t>(capacity);
-    w.q[1] = b->alloc<uint32_t>(capacity);
-    w.sh_o = b->alloc<float4>(capacity);
-    w.sh_d = b->alloc<float4>(capacity);
-    w.sh_L = b->alloc<float4>(capacity);
-    w.rec = b->alloc<float4>((size_t)capacity * std::max<uint32_t>(1u, b->max_bounces));
-    w.rec_n = b->alloc<uint8_t>(capacity);
-    b->drop(w.cam_dist);
-    w.cam_dist = b->alloc<float>(capacity);
-    b->drop(w.target);
+    b->drop(w.block);
+    w.block = nullptr;
+    w.capacity = 0;
+    const size_t R = std::max<uint32_t>(1u, b->max_bounces);
     bool tsm = false;
     for (tr_ctx* x : b->ctx) tsm = tsm || (x->integ.flags & TR_FLAG_TIME_SAMPLING) != 0;
-    w.target = tsm ? b->alloc<float4>(capacity) : nullptr;
+    void* block = b->alloc<unsigned char>(carve_wave(nullptr, nullptr, capacity, R, tsm));
     if (!w.counters) w.counters = b->alloc<uint32_t>(trk::kCounters);
     if (stats) {
         w.stats = stats;
@@ -198,7 +185,7 @@ void ensure_lane(tr_batch* b, trk::Wave& w, uint32_t capacity, unsigned long lon
         w.stats = b->alloc<unsigned long long>(8);
         TR_CUDA(cudaMemsetAsync(w.stats, 0, 8 * sizeof(unsigned long long), b->stream));
     }
-    w.capacity = capacity;
+    carve_wave(&w, block, capacity, R, tsm);
 }
 
 void ensure_batch_guided(tr_batch* b, uint32_t capacity) {

@@ -244,6 +244,9 @@ struct tr_ctx {
 
 namespace tri {
 
+// Per-slot arrays of a wave of `capacity` slots with R records each, carved from one block (one
+// pool allocation instead of fourteen): with w null the bytes it takes, else w's pointers into it.
+size_t carve_wave(trk::Wave* w, void* block, uint32_t capacity, size_t R, bool time_sampling);
 void ensure_wave(tr_ctx* x, uint32_t capacity);
 void ensure_lane_wave(tr_ctx* x, int k);
 void ensure_lane_guided(tr_ctx* x, int k);

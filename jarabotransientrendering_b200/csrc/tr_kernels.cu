@@ -1742,9 +1742,7 @@ cudaError_t launch_shade(const Params& p, int depth, cudaStream_t s) {
 // nodes.  Both sides there: 34 triangles (3 levels) 98 k paths 253 us each way (131 k: 269 wavefront,
 // 288 here); 20 k triangles (10 levels) 262 k: 690 / 660, 524 k: 845 / 1190; 328 k triangles (12
 // levels) 262 k: 1000 / 762, 524 k: 1165 / 1400.
-bool paths_fit(const Params& p) {
-    return p.batch.n_slots <= 32768u * (p.bvh_depth / 3u) && !p.multi.scenes && !p.guide.vrec && !p.bd.ne;
-}
+bool paths_fit(unsigned long long paths, uint32_t bvh_depth) { return paths <= 32768ull * (bvh_depth / 3u); }
 cudaError_t launch_paths(const Params& p, cudaStream_t s) {
     if (reinterpret_cast<uintptr_t>(p.scene.nodes) & 31u) return cudaErrorMisalignedAddress;
     int dev = 0, sms = 1;

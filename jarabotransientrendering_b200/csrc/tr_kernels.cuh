@@ -117,6 +117,7 @@ struct BatchDesc {
     Batch seg[kMaxSegments];
 };
 struct Wave {
+    void* block;              // the one allocation the per-slot arrays below are carved from
     float4* ray_o;            // o.xyz, tfar (sampled free-flight distance or +inf)
     float4* ray_d;            // d.xyz, accumulated time
     float4* thr;              // throughput rgb, pending pdf factor (RR prob * direction pdf)
@@ -236,8 +237,9 @@ cudaError_t launch_raygen(const Params& p, cudaStream_t s);
 cudaError_t launch_extend(const Params& p, int depth, int grid, cudaStream_t s);
 cudaError_t launch_shade(const Params& p, int depth, cudaStream_t s);
 cudaError_t launch_shadow(const Params& p, int depth, int grid, cudaStream_t s);
-// whole paths (camera ray to last record) of a batch in one launch: for batches that paths_fit takes
-bool paths_fit(const Params& p);
+// whole paths (camera ray to last record) of a batch in one launch, for a plain render (no learned
+// proposal, no light subpaths) of few paths
+bool paths_fit(unsigned long long paths, uint32_t bvh_depth);
 cudaError_t launch_paths(const Params& p, cudaStream_t s);
 // bsel < 0: the film itself; bsel = b: per-bounce film b (records of bounce min(depth, N-1) == b)
 // pixels per splat block: automatic (whole pixels filling one block) in single-scene mode,
