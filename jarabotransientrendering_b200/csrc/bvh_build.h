@@ -27,11 +27,14 @@ struct alignas(16) GpuTri {
 static_assert(sizeof(GpuTri) == 48, "triangle must be 48 bytes");
 
 // Binary SAH tree node (output of the binned builders, input of the four-child collapse).
-struct BinNode {
-    float lo[3], hi[3];          // bounds of the node's triangles
-    int32_t left, right;         // children; left < 0: leaf
+struct alignas(16) BinNode {
+    float lo[3];                 // bounds of the node's triangles: lo, hi
+    int32_t left;                // children; left < 0: leaf
+    float hi[3];
+    int32_t right;
     uint32_t first, count;       // leaf: its triangles, [first, first + count) of the id order
     uint32_t n_tris;             // triangles in the subtree
+    uint32_t pad;
 };
 
 struct BvhBuildResult {

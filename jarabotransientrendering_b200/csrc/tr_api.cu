@@ -45,7 +45,9 @@ tr_status validate(const tr_scene* s, const tr_camera* c, const tr_film* f, cons
     if (s->num_lights == 0 || !s->lights)
         return fail(TR_ERR_INVALID_ARGUMENT, "scene has no light source (next-event estimation needs one)");
     if (s->num_lights > (uint32_t)trk::kMaxLights) return fail(TR_ERR_INVALID_ARGUMENT, "too many lights");
-    for (uint32_t i = 0; i < s->num_triangles; ++i)
+    uint32_t most = 0;                     // a plain maximum vectorises
+    for (uint32_t i = 0; i < s->num_triangles; ++i) most = std::max(most, s->triangle_material[i]);
+    for (uint32_t i = 0; most >= s->num_materials; ++i)
         if (s->triangle_material[i] >= s->num_materials)
             return fail(TR_ERR_INVALID_ARGUMENT, "triangle " + std::to_string(i) + " has material index out of range");
     for (uint32_t i = 0; i < s->num_materials; ++i) {
@@ -749,17 +751,24 @@ tr_status tr_create(const tr_scene* s, const tr_camera* c, const tr_film* f, con
         // the largest block is taken from the memory pool before any scratch (a film freed by an
         // earlier context is reused whole instead of mapped again)
         const size_t nstreak = (size_t)f->width * f->height * f->time_bins * 3u;
-        size_t free_b = 0, total_b = 0;
-        cudaMemGetInfo(&free_b, &total_b);
-        free_b += tri::pool_idle_bytes(device);      // kept by the pool for reuse
         const size_t nb = f->bounce_films;
-        if ((1 + nb) * nstreak * sizeof(double) + ((size_t)2 << 30) > free_b) {
+        const std::string too_big = "streak film of " + std::to_string(nstreak * 8 >> 20) +
+                                    " MiB does not fit in free device memory";
+        auto refuse_film = [&] {
+            cudaGetLastError();
+            cudaStreamSynchronize(x->stream);
             x->release();
             delete x;
-            return fail(TR_ERR_OUT_OF_MEMORY, "streak film of " + std::to_string(nstreak * 8 >> 20) +
-                                                  " MiB does not fit in free device memory");
+            cudaMemPoolTrimTo(tri::device_pool(device), 0);     // not kept for a film that was refused
+            return fail(TR_ERR_OUT_OF_MEMORY, too_big);
+        };
+        try {
+            x->d_streak = x->alloc<double>(nstreak);
+            if (nb) x->d_bstreak = x->alloc<double>(nb * nstreak);
+        } catch (const CudaError& e) {
+            if (e.code != cudaErrorMemoryAllocation) throw;
+            return refuse_film();
         }
-        x->d_streak = x->alloc<double>(nstreak);
         x->d_steady = x->alloc<double>((size_t)f->width * f->height * 3u);
         x->d_weight = x->alloc<double>((size_t)f->width * f->height);
         TR_CUDA(cudaMemsetAsync(x->d_streak, 0, nstreak * sizeof(double), x->stream));
@@ -767,7 +776,6 @@ tr_status tr_create(const tr_scene* s, const tr_camera* c, const tr_film* f, con
         TR_CUDA(cudaMemsetAsync(x->d_weight, 0, (size_t)f->width * f->height * sizeof(double), x->stream));
         if (nb) {
             const size_t npix = (size_t)f->width * f->height;
-            x->d_bstreak = x->alloc<double>(nb * nstreak);
             x->d_bsteady = x->alloc<double>(nb * npix * 3u);
             x->d_bweight = x->alloc<double>(nb * npix);
             TR_CUDA(cudaMemsetAsync(x->d_bstreak, 0, nb * nstreak * sizeof(double), x->stream));
@@ -800,6 +808,13 @@ tr_status tr_create(const tr_scene* s, const tr_camera* c, const tr_film* f, con
                                 cudaMemcpyHostToDevice, x->stream));
         TR_CUDA(cudaMemcpyAsync(d_t, s->triangles, sizeof(uint32_t) * 3 * ntri, cudaMemcpyHostToDevice, x->stream));
         TR_CUDA(cudaMemcpyAsync(d_m, s->triangle_material, sizeof(uint32_t) * ntri, cudaMemcpyHostToDevice, x->stream));
+
+        // 2 GiB have to be left for the path state (asked while the uploads are under way: the query
+        // takes 0.2 ms)
+        size_t free_b = 0, total_b = 0;
+        cudaMemGetInfo(&free_b, &total_b);
+        free_b += tri::pool_idle_bytes(device);      // kept by the pool for reuse
+        if (free_b < ((size_t)2 << 30)) return refuse_film();
 
         // BVH (replaces World::freeze -> rtcCommit): built on the device from the uploaded arrays,
         // nodes and leaf order left there; the host builder takes one-leaf scenes and names the
@@ -901,11 +916,15 @@ tr_status tr_create(const tr_scene* s, const tr_camera* c, const tr_film* f, con
         sc.bvh_depth = x->bvh_depth;
         {
             float lo[3] = {3.4e38f, 3.4e38f, 3.4e38f}, hi[3] = {-3.4e38f, -3.4e38f, -3.4e38f};
-            for (uint32_t i = 0; i < s->num_vertices; ++i)
-                for (int k = 0; k < 3; ++k) {
-                    lo[k] = std::min(lo[k], s->vertices[3 * (size_t)i + k]);
-                    hi[k] = std::max(hi[k], s->vertices[3 * (size_t)i + k]);
-                }
+            if (on_device) {
+                for (int k = 0; k < 3; ++k) { lo[k] = dbv.vlo[k]; hi[k] = dbv.vhi[k]; }
+            } else {
+                for (uint32_t i = 0; i < s->num_vertices; ++i)
+                    for (int k = 0; k < 3; ++k) {
+                        lo[k] = std::min(lo[k], s->vertices[3 * (size_t)i + k]);
+                        hi[k] = std::max(hi[k], s->vertices[3 * (size_t)i + k]);
+                    }
+            }
             sc.reach = 0.0f;
             for (int k = 0; k < 3; ++k) {
                 sc.reach = std::max(sc.reach, std::max(std::fabs(lo[k]), std::fabs(hi[k])));

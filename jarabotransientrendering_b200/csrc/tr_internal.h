@@ -282,6 +282,7 @@ struct DeviceBvh {
     uint32_t binary_depth = 0;
     uint32_t leaves = 0;
     double build_ms = 0.0;
+    float vlo[3], vhi[3];        // box of all vertices
 };
 // Binned-SAH build on the device (bvh_gpu.cu) from device-resident vertices [nv][3] and
 // triangles [nt][3], collapsed to four-child nodes as build_bvh does: the nodes go to
