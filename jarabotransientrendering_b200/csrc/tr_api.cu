@@ -268,11 +268,31 @@ void prof_publish(tr_ctx* x) {
     x->prof_dirty = false;
 }
 
-// Lane k + 1's buffers: the per-slot arrays of the first wave at its capacity, its own queue
-// counters, the first wave's statistics counters.
-void ensure_lane_wave(tr_ctx* x, int k) {
+// Gives the path state of all lanes back to the pool (its contents are only scratch between calls).
+void drop_waves(tr_ctx* x) {
+    auto drop = [&](void* p) {
+        if (!p) return;
+        cudaFree(p);
+        x->allocs.erase(std::remove(x->allocs.begin(), x->allocs.end(), p), x->allocs.end());
+    };
+    auto drop_wave = [&](trk::Wave& w) {
+        drop(w.block);
+        w.block = nullptr;
+        w.capacity = 0;
+    };
+    drop_wave(x->wave);
+    for (trk::Wave& w : x->lane_wave) drop_wave(w);
+    for (int k = 0; k + 1 < kWaveLanes; ++k) {
+        drop(x->lane_vrec[k]);
+        x->lane_vrec[k] = nullptr;
+        x->lane_vrec_cap[k] = 0;
+    }
+}
+
+// Lane k + 1's buffers: the per-slot arrays of `capacity` slots, its own queue counters, the first
+// wave's statistics counters.
+void ensure_lane_wave(tr_ctx* x, int k, uint32_t capacity) {
     trk::Wave& w = x->lane_wave[k];
-    const uint32_t capacity = x->wave.capacity;
     if (w.capacity >= capacity && w.counters) return;
     auto drop = [&](void* p) {
         if (!p) return;
@@ -292,12 +312,13 @@ void ensure_lane_wave(tr_ctx* x, int k) {
 
 // Lane k + 1's guided-vertex records (the training pool and its counters are shared: the
 // batches of all lanes fill it, each entry tagged with its batch).
-void ensure_lane_guided(tr_ctx* x, int k) {
-    const uint32_t capacity = x->wave.capacity;
+void ensure_lane_guided(tr_ctx* x, int k, uint32_t capacity) {
     if (x->lane_vrec_cap[k] >= capacity && x->lane_vrec[k]) return;
     if (x->lane_vrec[k]) {
         cudaFree(x->lane_vrec[k]);
         x->allocs.erase(std::remove(x->allocs.begin(), x->allocs.end(), (void*)x->lane_vrec[k]), x->allocs.end());
+        x->lane_vrec[k] = nullptr;
+        x->lane_vrec_cap[k] = 0;
     }
     x->lane_vrec[k] = x->alloc<uint4>((size_t)capacity * 5);
     x->lane_vrec_cap[k] = capacity;
@@ -314,6 +335,9 @@ void ensure_guided(tr_ctx* x, uint32_t capacity) {
     tr_ctx::PoolBuf& a = x->pool_alt;
     drop(g.vrec); drop(g.pool_feat); drop(g.pool_dir); drop(g.pool_w); drop(g.pool_meta);
     drop(a.feat); drop(a.dir); drop(a.w); drop(a.meta);
+    g.vrec = g.pool_feat = g.pool_meta = a.feat = a.meta = nullptr;
+    g.pool_dir = g.pool_w = a.dir = a.w = nullptr;
+    x->gw_capacity = 0;                  // until the new buffers are there
     g.vrec = x->alloc<uint4>((size_t)capacity * 5);
     const uint32_t pc = std::max<uint32_t>(1u, x->guide_pool);
     g.pool_feat = x->alloc<uint4>((size_t)pc * 8);
@@ -403,9 +427,60 @@ tr_status render_region(tr_ctx* x, uint32_t x0, uint32_t y0, uint32_t x1, uint32
     const bool bidir = (x->integ.flags & TR_FLAG_BIDIRECTIONAL) != 0;
     // small renders: whole paths in one launch (per-kernel times need the kernels apart)
     const bool whole = trk::paths_fit(total_slots, x->bvh_depth) && !guided && !bidir && !x->profiling;
-    ensure_wave(x, cap);
+    // samples per pixel per batch, pixels per batch and the lanes that take the batches in turn
+    const uint32_t ns_chunk = std::max<uint32_t>(1u, std::min<uint32_t>(ns_total, cap / ninc));
+    const uint32_t unit = std::max<uint32_t>(1u, cap / (ns_chunk * ninc));
+    int max_lanes = (!bidir && ns_chunk >= ns_total) ? kWaveLanes : 1;
+    // Large renders: fewer, larger batches.  Every traversal launch ends with its longest rays, so
+    // four times the rays per launch spend a smaller share in its tail: 67 M paths over 328 k
+    // triangles 49.0 ms in 2 M-slot batches on four lanes, 44.6 ms in 8 M-slot batches on two; 16.8
+    // M paths 12.9 -> 11.5 ms, guided 8.6 -> 8.0 ms; 5 M paths 4.3 -> 4.4 ms, so the line is at two
+    // batches of half that size.  RGBE delivery copies a batch's images when it is done and takes three lanes of 4 M (the
+    // last batches' copies are not hidden); sums, bound by the copy, keep the small batches.  A batch is a
+    // whole number of the small ones, whose splat blocks it keeps (the film's FP32 group sums do
+    // not depend on the batch size).
+    uint32_t large = 1;
+    if (max_lanes > 1 && total_slots >= kLargeCapacity && !(sink && sink->type != TR_FILM_RGBE)) {
+        const int lanes = sink ? 3 : 2;
+        const uint64_t slots = std::min<uint64_t>(sink ? kLargeCapacity / 2 : kLargeCapacity, total_slots / (uint64_t)lanes);
+        const size_t per_slot = (guided ? 80u : 0u) +
+            carve_wave(nullptr, nullptr, 1u << 16, std::max<uint32_t>(1u, x->integ.max_bounces), true) / (1u << 16);
+        const uint64_t room = kLargeWaveBytes / ((size_t)lanes * per_slot);
+        large = (uint32_t)std::max<uint64_t>(1u, std::min(slots, room) / ((uint64_t)unit * ns_chunk * ninc));
+        if (large > 1) max_lanes = lanes;
+    }
+    const uint32_t small_cap = cap;
+    auto buffers = [&](uint32_t n_lanes) {
+        ensure_wave(x, cap);
+        if (guided) ensure_guided(x, cap);
+        for (uint32_t k = 0; k + 1 < n_lanes; ++k) {
+            ensure_lane_wave(x, (int)k, cap);
+            if (guided) ensure_lane_guided(x, (int)k, cap);
+            if (!x->lane_stream[k]) TR_CUDA(cudaStreamCreateWithFlags(&x->lane_stream[k], cudaStreamNonBlocking));
+            if (!x->lane_shadow_stream[k])
+                TR_CUDA(cudaStreamCreateWithFlags(&x->lane_shadow_stream[k], cudaStreamNonBlocking));
+        }
+    };
+    auto lanes_of = [&]() {
+        const uint64_t ppb = (uint64_t)unit * large;
+        return (int)std::min<uint64_t>((uint64_t)max_lanes, (win_pix + ppb - 1) / ppb);
+    };
+    if (large > 1) {
+        cap = unit * large * ns_chunk * ninc;
+        try {
+            buffers((uint32_t)lanes_of());
+        } catch (const CudaError& e) {
+            if (e.code != cudaErrorMemoryAllocation) throw;
+            cudaGetLastError();                 // no room for them: give back what was taken, small batches
+            drop_waves(x);
+            large = 1;
+            cap = small_cap;
+            max_lanes = kWaveLanes;
+        }
+    }
+    const int lanes = lanes_of();
+    if (large == 1) buffers((uint32_t)lanes);
     if (guided) {
-        ensure_guided(x, cap);
         // about 1.5 guided vertices per path; keep enough of them to fill the training pool
         x->gw.keep_prob = x->guide_pool ? std::min(1.0f, (float)x->guide_pool / (1.5f * (float)total_slots)) : 0.0f;
         x->gw.mix_prob = x->guide_mix;
@@ -413,8 +488,6 @@ tr_status render_region(tr_ctx* x, uint32_t x0, uint32_t y0, uint32_t x1, uint32
         tr_status ts = guide_begin_render(x, x->s());
         if (ts != TR_OK) return ts;
     }
-    // samples per pixel per batch, and pixels per batch
-    uint32_t ns_chunk = std::max<uint32_t>(1u, std::min<uint32_t>(ns_total, cap / ninc));
     const bool film_was_clean = x->film_clean;
     x->film_clean = false;
     cudaStream_t strm = x->s();
@@ -491,29 +564,18 @@ tr_status render_region(tr_ctx* x, uint32_t x0, uint32_t y0, uint32_t x1, uint32
         }
     }
     // Wave lanes: with more than one pixel batch and each pixel in one batch only (a single
-    // sample chunk), consecutive batches alternate between kWaveLanes sets of wave buffers and
+    // sample chunk), consecutive batches alternate between several sets of wave buffers and
     // pairs of streams, so one batch's last, nearly empty depths run beside the next batch's
     // first ones.  The batches share no pixels; with the learned proposal they share the
     // training pool (entries tagged by batch).  Light subpaths (one light wave) keep a single
     // lane.
-    const uint64_t n_pix_batches = (win_pix + std::max<uint32_t>(1u, cap / (ns_chunk * ninc)) - 1) /
-                                   std::max<uint32_t>(1u, cap / (ns_chunk * ninc));
-    const int lanes = (!bidir && ns_chunk >= ns_total)
-                          ? (int)std::min<uint64_t>((uint64_t)kWaveLanes, n_pix_batches) : 1;
     uint32_t batch_no = 0;
-    for (int k = 0; k + 1 < lanes; ++k) {
-        ensure_lane_wave(x, k);
-        if (guided) ensure_lane_guided(x, k);
-        if (!x->lane_stream[k]) TR_CUDA(cudaStreamCreateWithFlags(&x->lane_stream[k], cudaStreamNonBlocking));
-        if (!x->lane_shadow_stream[k])
-            TR_CUDA(cudaStreamCreateWithFlags(&x->lane_shadow_stream[k], cudaStreamNonBlocking));
-    }
     TR_CUDA(cudaEventRecord(x->ev0, strm));
     for (int k = 0; k + 1 < lanes; ++k) TR_CUDA(order(strm, x->lane_stream[k]));
     for (uint64_t sb = 0; sb < ns_total; sb += ns_chunk) {
         const uint32_t ns = (uint32_t)std::min<uint64_t>(ns_chunk, ns_total - sb);
         const uint32_t per_pix = ns * ninc;
-        const uint32_t ppb = std::max<uint32_t>(1u, cap / per_pix);
+        const uint32_t ppb = large > 1 ? unit * large : std::max<uint32_t>(1u, cap / per_pix);
         for (uint64_t pb = 0; pb < win_pix; pb += ppb) {
             const uint32_t npix = (uint32_t)std::min<uint64_t>(ppb, win_pix - pb);
             trk::Params p = make_params(x);
@@ -530,6 +592,7 @@ tr_status render_region(tr_ctx* x, uint32_t x0, uint32_t y0, uint32_t x1, uint32
             auto tl = [&](int kind, auto&& launch) { timed_on(kind, ls, launch); };
             p.batch.win_x0 = x0; p.batch.win_y0 = y0; p.batch.win_w = win_w;
             p.batch.pix_begin = (uint32_t)pb; p.batch.npix = npix;
+            p.batch.splat_unit = large > 1 ? unit : npix;
             p.batch.s0 = s0 + sb; p.batch.ns = ns; p.batch.ninc = ninc;
             p.batch.n_slots = npix * per_pix;
             if (whole) {
@@ -1327,7 +1390,7 @@ extern "C" tr_status tr_render_region_noalloc(tr_ctx* x, uint32_t x0, uint32_t y
         // slot are reset by the ray generation kernel; the ray counters keep adding up)
         TR_CUDA(cudaMemsetAsync(w.counters, 0, sizeof(uint32_t) * trk::kCounters, strm));
         p.batch.win_x0 = x0; p.batch.win_y0 = y0; p.batch.win_w = x1 - x0;
-        p.batch.pix_begin = 0; p.batch.npix = (uint32_t)npix;
+        p.batch.pix_begin = 0; p.batch.npix = p.batch.splat_unit = (uint32_t)npix;
         p.batch.s0 = s0; p.batch.ns = ns; p.batch.ninc = x->integ.incoming_samples;
         p.batch.n_slots = (uint32_t)paths;
         if (trk::paths_fit(paths, x->bvh_depth)) {

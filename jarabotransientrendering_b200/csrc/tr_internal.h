@@ -54,6 +54,8 @@ T* dalloc(size_t count, size_t& total) {
 
 constexpr uint32_t kMaxBounces = 63;            // counters hold 64 depths
 constexpr uint32_t kDefaultCapacity = 1u << 21; // path slots per wavefront batch
+constexpr uint32_t kLargeCapacity = 1u << 23;   // of a large render's (render_region)
+constexpr size_t kLargeWaveBytes = (size_t)6 << 30;  // path state a large render's batches may take
 #ifndef TR_WAVE_LANES
 #define TR_WAVE_LANES 4
 #endif
@@ -248,8 +250,9 @@ namespace tri {
 // pool allocation instead of fourteen): with w null the bytes it takes, else w's pointers into it.
 size_t carve_wave(trk::Wave* w, void* block, uint32_t capacity, size_t R, bool time_sampling);
 void ensure_wave(tr_ctx* x, uint32_t capacity);
-void ensure_lane_wave(tr_ctx* x, int k);
-void ensure_lane_guided(tr_ctx* x, int k);
+void drop_waves(tr_ctx* x);
+void ensure_lane_wave(tr_ctx* x, int k, uint32_t capacity);
+void ensure_lane_guided(tr_ctx* x, int k, uint32_t capacity);
 void ensure_guided(tr_ctx* x, uint32_t capacity);
 trk::Params make_params(tr_ctx* x);
 trg::GuideDev guide_dev(tr_guide* g);

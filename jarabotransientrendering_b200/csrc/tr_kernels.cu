@@ -1136,10 +1136,15 @@ __global__ void __launch_bounds__(kSplatBlock) k_splat(const __grid_constant__ P
     const FilmDev& film = *Fp;
     const uint32_t T = film.T;
     const uint32_t TT = T * 3u;
-    const uint32_t pix0 = blk * G;
-    if (pix0 >= B.npix) return;
+    uint32_t pix0 = blk * G, pix_end = B.npix;
+    if constexpr (!kMulti) {
+        const uint32_t per_unit = (B.splat_unit + G - 1u) / G, unit = blk / per_unit;
+        pix0 = unit * B.splat_unit + (blk - unit * per_unit) * G;
+        pix_end = min(B.npix, (unit + 1u) * B.splat_unit);
+    }
+    if (pix0 >= pix_end) return;
     if (bsel >= (int)film.nbounce) return;                // this scene has no such bounce film
-    const uint32_t gp = min((uint32_t)G, B.npix - pix0);
+    const uint32_t gp = min((uint32_t)G, pix_end - pix0);
     // bsel < 0: the film; with bounce films its steady image is the base Film's (all samples).
     // bsel = b: bounce film b, fed by the records of bounce min(depth, N-1) == b.
     const size_t npix_film = (size_t)film.W * film.H;
@@ -1768,7 +1773,8 @@ cudaError_t launch_splat(const Params& p, cudaStream_t s, int bsel) {
         k_splat<true><<<p.multi.max_splat_blocks, kSplatBlock, 0, s>>>(p, 0, bsel);
     } else {
         const uint32_t G = splat_pixels_per_block(p.batch.ns * p.batch.ninc);
-        const uint32_t blocks = (p.batch.npix + G - 1) / G;
+        const uint32_t unit = p.batch.splat_unit, whole = p.batch.npix / unit;
+        const uint32_t blocks = whole * ((unit + G - 1) / G) + (p.batch.npix - whole * unit + G - 1) / G;
         // a fresh film's RGBE images: the cells each block adds to, one bit each (up to 32 KB;
         // beyond that every cell is read back)
         const size_t bits = (size_t)G * p.film.T;

@@ -106,6 +106,7 @@ struct Batch {
     uint32_t scene;                     // index into MultiDev::scenes (0 in single-scene mode)
     uint32_t blk_begin;                 // first splat block of this segment
     uint32_t splat_g;                   // pixels per splat block
+    uint32_t splat_unit;                // single scene: the splat blocks start anew every so many pixels
 };
 
 // Multi-scene rendering (tr_batch): per-scene data and the batch descriptors live in device
