@@ -1537,7 +1537,7 @@ extern "C" tr_status tr_guide_forward(tr_guide* g, const uint16_t* d_features, u
     try {
         TR_CUDA(cudaSetDevice(g->device));
         cudaStream_t s = stream ? static_cast<cudaStream_t>(stream) : g->stream;
-        TR_CUDA(trg::mlp_forward(g->dev(), reinterpret_cast<const uint4*>(d_features), n, d_out, nullptr, g->err, s));
+        TR_CUDA(trg::mlp_forward(g->dev(), reinterpret_cast<const uint4*>(d_features), n, d_out, g->err, s));
         return guide_check_err(g, s);
     } catch (const CudaError& e) {
         return fail(TR_ERR_CUDA, e.what());
@@ -1545,30 +1545,22 @@ extern "C" tr_status tr_guide_forward(tr_guide* g, const uint16_t* d_features, u
 }
 
 namespace tri {
-// Enqueues one training step (forward, loss gradient, backward, weight gradients, Adam, weight
-// repacking) on stream s without waiting for it; the loss lands in g->scalars[1].
+// Enqueues one training step on stream s without waiting for it; the loss lands in g->scalars[1].
 void train_enqueue(tr_guide* g, const uint4* x, const float* d_dirs, const float* d_weights, uint32_t n, float lr,
                    cudaStream_t s) {
     g->ensure(n);
-    TR_CUDA(trg::mlp_forward(g->dev(), x, n, g->out, g->act, g->err, s));
-    TR_CUDA(cudaMemsetAsync(g->scalars, 0, 4 * sizeof(float), s));
-    TR_CUDA(trg::mix_grad(g->out, d_dirs, d_weights, n, g->scalars, g->dy_bf, g->scalars + 1, s));
-    TR_CUDA(trg::mlp_backward(g->dev(), g->dy_bf, g->act, n, g->dh, g->err, s));
-    TR_CUDA(cudaMemsetAsync(g->grads, 0, sizeof(float) * TR_GUIDE_PARAMS, s));
-    float* gb = g->grads + 4 * 4096;
-    const size_t mrow = (size_t)n * 8;
-    trg::DwLayers dw{};
-    dw.prev[0] = x;                  dw.grad_bf[0] = g->dh;
-    dw.prev[1] = g->act;             dw.grad_bf[1] = g->dh + mrow;
-    dw.prev[2] = g->act + mrow;      dw.grad_bf[2] = g->dh + 2 * mrow;
-    dw.prev[3] = g->act + 2 * mrow;  dw.grad_bf[3] = g->dy_bf;                // output layer
-    for (int l = 0; l < 4; ++l) { dw.gw[l] = g->grads + 4096 * l; dw.gb[l] = gb + 64 * l; }
-    TR_CUDA(trg::weight_grad(dw, n, g->spin, g->err, s));
-    if (lr > 0.0f) {
-        g->step += 1;
-        TR_CUDA(trg::adam(g->params, g->grads, g->m1, g->m2, TR_GUIDE_PARAMS, lr, g->step, s));
-        TR_CUDA(trg::pack_weights(g->params, g->w_fwd, g->w_bwd, s));
-    }
+    if (lr > 0.0f) g->step += 1;
+    trg::TrainArgs a{};
+    a.net = g->dev();
+    a.x = x; a.dirs = d_dirs; a.w = d_weights;
+    a.act = g->act; a.dy = g->dy_bf; a.dh = g->dh;
+    a.scratch = g->scratch; a.loss = g->scalars + 1;
+    a.params = g->params; a.grads = g->grads; a.m1 = g->m1; a.m2 = g->m2;
+    a.w_fwd = g->w_fwd; a.w_bwd = g->w_bwd;
+    a.err = g->err;
+    a.lr = lr;
+    a.step = g->step;
+    TR_CUDA(trg::train_step(a, n, s));
 }
 }  // namespace tri
 

@@ -33,28 +33,41 @@ struct GuideDev {
     uint32_t spin;         // polls of an mbarrier before a tensor-core wait counts as timed out
 };
 
-// m_dev (optional): the row count in device memory, at most m (rows beyond it are skipped)
-cudaError_t mlp_forward(const GuideDev& g, const uint4* x, uint32_t m, float* out, uint4* act, int* err,
-                        cudaStream_t s, const uint32_t* m_dev = nullptr);
-cudaError_t mlp_backward(const GuideDev& g, const uint4* dy, const uint4* act, uint32_t m, uint4* dh, int* err,
-                         cudaStream_t s);
+cudaError_t mlp_forward(const GuideDev& g, const uint4* x, uint32_t m, float* out, int* err, cudaStream_t s);
 int mlp_grid(int device);
 // CTAs of `kernel` that fit on the device at once (SMs x CTAs per SM, from the kernel's
 // registers, shared memory and `tmem_cols` tensor-memory columns per CTA), for persistent loops
 int resident_grid(int device, const void* kernel, int threads, size_t dyn_smem, int tmem_cols = 64);
 cudaError_t pack_weights(const float* params, uint8_t* w_fwd, uint8_t* w_bwd, cudaStream_t s);
-cudaError_t mix_grad(const float* out, const float* dirs, const float* w, uint32_t m, float* wsum, uint4* dy_bf,
-                     float* loss, cudaStream_t s);
-// weight-gradient operands of the four layers: gw[l] += prev[l]^T grad[l], gb[l] += column sums
+// weight-gradient operands of the four layers
 struct DwLayers {
     const uint4* prev[4];      // [m][64] bf16 layer inputs (features, H1, H2, H3)
     const uint4* grad_bf[4];   // [m][64] bf16 gradients w.r.t. the layer outputs
-    float* gw[4];
-    float* gb[4];
+    float* part;               // [layer][CTA][65][64] sums over each CTA's rows: weights, bias
 };
-// tensor-core weight gradients; `spin` bounds each mbarrier wait (timeout: *err = 1)
-cudaError_t weight_grad(const DwLayers& L, uint32_t m, uint32_t spin, int* err, cudaStream_t s);
-cudaError_t adam(float* params, const float* grads, float* m1, float* m2, uint32_t n, float lr, uint32_t step,
-                 cudaStream_t s);
+struct UpdateArgs {
+    const float *part, *loss_part;
+    uint32_t nparts, ntiles;
+    const int* err;
+    float *loss, *params, *grads, *m1, *m2;
+    uint8_t *w_fwd, *w_bwd;
+    float lr, c1, c2;
+};
+// One training step (weight sum, forward + loss gradient + backward, weight gradients, update):
+// gradients to grads, the batch loss to *loss, with lr > 0 Adam step `step` and repacked weights.  The
+// same bits on every run.  scratch: train_scratch_floats(m); act, dh [3][m][64], dy [m][64] bf16.
+struct TrainArgs {
+    GuideDev net;
+    const uint4* x;
+    const float *dirs, *w;
+    uint4 *act, *dy, *dh;
+    float *scratch, *loss, *params, *grads, *m1, *m2;
+    uint8_t *w_fwd, *w_bwd;
+    int* err;
+    float lr;
+    uint32_t step;
+};
+size_t train_scratch_floats(uint32_t m);
+cudaError_t train_step(const TrainArgs& a, uint32_t m, cudaStream_t s);
 
 }  // namespace trg

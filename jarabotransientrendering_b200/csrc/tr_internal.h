@@ -82,7 +82,7 @@ struct tr_guide {
     float* scalars = nullptr;  // [0] weight sum, [1] loss
     uint32_t cap = 0;
     uint4* act = nullptr;
-    float* out = nullptr;
+    float* scratch = nullptr;          // partial sums of a training step
     uint4* dy_bf = nullptr;
     uint4* dh = nullptr;       // BF16 hidden-layer gradients [3][n][64]
     uint32_t step = 0;
@@ -104,9 +104,12 @@ struct tr_guide {
     }
     void ensure(uint32_t n) {
         if (cap >= n) return;
-        drop(act); drop(out); drop(dy_bf); drop(dh);
+        drop(act); drop(scratch); drop(dy_bf); drop(dh);
+        act = dy_bf = dh = nullptr;
+        scratch = nullptr;
+        cap = 0;
         act = alloc<uint4>((size_t)3 * n * 8);
-        out = alloc<float>((size_t)n * trg::kOut);
+        scratch = alloc<float>(trg::train_scratch_floats(n));
         dy_bf = alloc<uint4>((size_t)n * 8);
         dh = alloc<uint4>((size_t)3 * n * 8);
         cap = n;
