@@ -213,11 +213,25 @@ void ensure_wave(tr_ctx* x, uint32_t capacity) {
         bd.nl = x->alloc<uint8_t>(capacity);
         bd.ne = x->alloc<uint8_t>(capacity);
         bd.L0 = x->alloc<float4>(capacity);
-        // connection queue of one eye depth (up to nvert rays per slot) and the record flags
+        // connection queues of one eye depth (up to nvert rays per slot) and the record flags.  With
+        // two queues the next depth's rays are set up while this one's are traced.
         drop(bd.co_o); drop(bd.co_d); drop(bd.co_L); drop(bd.valid);
-        bd.co_o = x->alloc<float4>(nv * capacity);
-        bd.co_d = x->alloc<float4>(nv * capacity);
-        bd.co_L = x->alloc<float4>(nv * capacity);
+        bd.co_o = bd.co_d = bd.co_L = nullptr;
+        bd.valid = nullptr;
+        for (x->bd_queues = 2;; x->bd_queues = 1) {
+            try {
+                const size_t q = nv * x->bd_queues * capacity;
+                bd.co_o = x->alloc<float4>(q);
+                bd.co_d = x->alloc<float4>(q);
+                bd.co_L = x->alloc<float4>(q);
+                break;
+            } catch (const CudaError& e) {
+                if (e.code != cudaErrorMemoryAllocation || x->bd_queues == 1) throw;
+                cudaGetLastError();
+                drop(bd.co_o); drop(bd.co_d);
+                bd.co_o = bd.co_d = nullptr;
+            }
+        }
         bd.ncand = x->integ.max_bounces * (std::max<uint32_t>(1u, x->integ.max_bounces) - 1u) / 2u;
         bd.valid = x->alloc<uint8_t>(R * capacity);
     }
@@ -623,6 +637,39 @@ tr_status render_region(tr_ctx* x, uint32_t x0, uint32_t y0, uint32_t x1, uint32
                 launches += 1 + 2ull * x->bd.nvert;
                 ext_l += x->bd.nvert;
             }
+            // Eye-light vertex connections, one eye depth at a time: rays with their samples into a
+            // connection queue, traced by k_shadow (records on blocked pairs), compacted after the
+            // next-event records.  A depth's pairs need its eye vertices and all light vertices, so they
+            // run on two more streams beside the rest of the eye walk.
+            cudaStream_t s_gen = nullptr, s_conn = nullptr;
+            trk::Params pc = p;
+            if (bidir && x->bd.nvert) {
+                if (!x->lane_stream[0]) TR_CUDA(cudaStreamCreateWithFlags(&x->lane_stream[0], cudaStreamNonBlocking));
+                if (!x->lane_shadow_stream[0])
+                    TR_CUDA(cudaStreamCreateWithFlags(&x->lane_shadow_stream[0], cudaStreamNonBlocking));
+                for (cudaEvent_t& e : x->bd_free)
+                    if (!e) TR_CUDA(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
+                s_gen = x->lane_stream[0];
+                s_conn = x->lane_shadow_stream[0];
+                const size_t R = (size_t)x->integ.max_bounces + x->bd.ncand;
+                TR_CUDA(cudaMemsetAsync(x->bd.valid, 0, R * x->wave.capacity, ls));
+                TR_CUDA(order(x->light_stream, s_gen));
+            }
+            auto connect = [&](uint32_t ie) {
+                const uint32_t k = ie % x->bd_queues;
+                const size_t at = (size_t)k * std::max<uint32_t>(1u, x->bd.nvert) * x->wave.capacity;
+                if (ie >= x->bd_queues) TR_CUDA(cudaStreamWaitEvent(s_gen, x->bd_free[k], 0));
+                TR_CUDA(order(ls, s_gen));
+                pc.bd.co_o = x->bd.co_o + at; pc.bd.co_d = x->bd.co_d + at; pc.bd.co_L = x->bd.co_L + at;
+                pc.wave.sh_o = pc.bd.co_o; pc.wave.sh_d = pc.bd.co_d; pc.wave.sh_L = pc.bd.co_L;
+                timed_on(3, s_gen, [&] { return trk::launch_connect_gen(pc, (int)ie, s_gen); });
+                TR_CUDA(order(s_gen, s_conn));
+                const int dq = (int)(x->integ.max_bounces + ie);
+                timed_on(3, s_conn, [&] { return trk::launch_shadow(pc, dq, x->trace_grid, s_conn); });
+                TR_CUDA(cudaEventRecord(x->bd_free[k], s_conn));
+                launches += 2;
+                sh_l += 1;
+            };
             for (uint32_t d = 0; d < (whole ? 0u : x->integ.max_bounces); ++d) {
                 tl(1, [&] { return trk::launch_extend(p, (int)d, x->trace_grid, ls); });
                 if (d > 0) TR_CUDA(order(lsh, ls));
@@ -640,6 +687,7 @@ tr_status render_region(tr_ctx* x, uint32_t x0, uint32_t y0, uint32_t x1, uint32
                 }
                 TR_CUDA(order(ls, lsh));
                 timed_on(3, lsh, [&] { return trk::launch_shadow(p, (int)d, x->trace_grid, lsh); });
+                if (s_gen && d < x->bd.nvert) connect(d);
             }
             if (!whole && x->integ.max_bounces) TR_CUDA(order(lsh, ls));
             if (guided && x->guide_pool) {
@@ -647,24 +695,10 @@ tr_status render_region(tr_ctx* x, uint32_t x0, uint32_t y0, uint32_t x1, uint32
                 launches += 2;
             }
             if (bidir) TR_CUDA(order(x->light_stream, ls));
-            if (bidir && x->bd.nvert) {
-                // eye-light vertex connections, one eye depth at a time: rays with their samples
-                // into the connection queue, traced by k_shadow (records on blocked pairs),
-                // then compacted after the next-event records
-                const size_t R = (size_t)x->integ.max_bounces + x->bd.ncand;
-                TR_CUDA(cudaMemsetAsync(x->bd.valid, 0, R * x->wave.capacity, ls));
-                trk::Params pc = p;
-                pc.wave.sh_o = x->bd.co_o;
-                pc.wave.sh_d = x->bd.co_d;
-                pc.wave.sh_L = x->bd.co_L;
-                for (uint32_t ie = 0; ie < x->bd.nvert; ++ie) {
-                    tl(3, [&] { return trk::launch_connect_gen(p, (int)ie, ls); });
-                    const int dq = (int)(x->integ.max_bounces + ie);
-                    tl(3, [&] { return trk::launch_shadow(pc, dq, x->trace_grid, ls); });
-                }
+            if (s_gen) {
+                TR_CUDA(order(s_conn, ls));
                 tl(3, [&] { return trk::launch_connect_compact(p, ls); });
-                launches += 1 + 2ull * x->bd.nvert;
-                sh_l += x->bd.nvert;
+                launches += 1;
             }
             if (rgbe && sb + ns >= ns_total) {
                 // final pixels: the splat blocks encode their images as they finish them

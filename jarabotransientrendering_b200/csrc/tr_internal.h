@@ -158,6 +158,8 @@ struct tr_ctx {
     trk::Wave lwave{};                      // light subpaths (TR_FLAG_BIDIRECTIONAL)
     trk::BidirWave bd{};
     uint32_t* d_lcounters = nullptr;
+    uint32_t bd_queues = 1;                 // connection queues (two when memory allows)
+    cudaEvent_t bd_free[2]{};               // a queue's rays have been traced
     // film streaming (tr_render_film)
     cudaStream_t copy_stream = nullptr;
     // shadow rays of one depth beside the closest-hit rays of the next (tr_render_region)
@@ -223,6 +225,10 @@ struct tr_ctx {
     void release() {
         if (ev_snap) { cudaEventDestroy(ev_snap); ev_snap = nullptr; }
         if (ev_train) { cudaEventDestroy(ev_train); ev_train = nullptr; }
+        for (cudaEvent_t& e : bd_free) {
+            if (e) cudaEventDestroy(e);
+            e = nullptr;
+        }
         for (cudaEvent_t e : prof_events) cudaEventDestroy(e);
         prof_events.clear();
         for (cudaEvent_t e : dep_events) cudaEventDestroy(e);

@@ -1551,8 +1551,9 @@ __device__ float mis_quantity(const Params& p, uint32_t slot, uint32_t t, uint32
 // slot, the pairs (ie, il) with ie + il + 2 <= max_bounces whose delays fit the film each get a
 // connection ray from the light vertex to the eye vertex in the connection queue, with the
 // sample the pair contributes -- value fe * (fv * (f_l * L0)) / w, time = distance + both
-// delays, bounce ie + il + 1 -- and its fixed record index (after the slot's next-event
-// records, in (ie, il) order).  k_shadow then records the pairs whose segment is blocked (the
+// delays, bounce ie + il + 1 -- and its fixed record index (after the max_bounces next-event records a
+// slot can have, in (ie, il) order, so the pairs of an eye depth can be queued while the eye walk goes
+// on).  k_shadow then records the pairs whose segment is blocked (the
 // reference connects when World::intersects returns true, World.h:617-639 / 693-697).
 // One slot per thread; the warp appends its rays with one atomic.
 __global__ void __launch_bounds__(256) k_connect_gen(const __grid_constant__ Params p, int ie) {
@@ -1605,7 +1606,6 @@ __global__ void __launch_bounds__(256) k_connect_gen(const __grid_constant__ Par
         wbase = __shfl_sync(kFull, wbase, 0);
         if (!have || cnt == 0) continue;
         uint32_t q = wbase + incl - cnt;
-        const uint32_t n0 = p.wave.rec_n[slot];
         const float4 L0 = p.bd.L0[slot];
         const float cam_d = film.unwarp ? p.wave.cam_dist[slot] : 0.0f;
         const float4 e_npdf = make_float4(E.n.x, E.n.y, E.n.z, E.pdf);
@@ -1636,7 +1636,7 @@ __global__ void __launch_bounds__(256) k_connect_gen(const __grid_constant__ Par
             const uint32_t bounce = uie + il + 1u;
             uint32_t bw = bin | (bounce << 24) | kConnRay;
             if (!(inside || film.nbounce)) bw |= kConnNoRecord;
-            const uint32_t k = n0 + off + il;
+            const uint32_t k = maxb + off + il;
             p.bd.co_o[q] = make_float4(Lv.pos.x, Lv.pos.y, Lv.pos.z, dd - kSigmaVis);
             p.bd.co_d[q] = make_float4(l2e.x, l2e.y, l2e.z, __uint_as_float(bw));
             p.bd.co_L[q] = fin ? make_float4(Lr, Lg, Lb, __uint_as_float(slot | (k << 24)))
@@ -1656,9 +1656,9 @@ __global__ void __launch_bounds__(256) k_connect_compact(const __grid_constant__
         const uint32_t n0 = p.wave.rec_n[slot];
         uint32_t j = n0;
         for (uint32_t c = 0; c < p.bd.ncand; ++c) {
-            const size_t k = (size_t)(n0 + c) * cap + slot;
+            const size_t k = (size_t)(p.max_bounces + c) * cap + slot;
             if (!p.bd.valid[k]) continue;
-            if (j != n0 + c) p.wave.rec[(size_t)j * cap + slot] = p.wave.rec[k];
+            if (j != p.max_bounces + c) p.wave.rec[(size_t)j * cap + slot] = p.wave.rec[k];
             ++j;
         }
         splats += j - n0;
