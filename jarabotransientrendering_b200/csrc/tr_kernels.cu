@@ -76,8 +76,8 @@ __device__ __forceinline__ void slab_axis(float o, float d, float reach, f2& m, 
     m = pack2(neg ? mf : mn, neg ? mn : mf);
     a = pack2(neg ? af : an, neg ? an : af);
 }
-__device__ __forceinline__ SlabRay slab_setup(const SceneDev& sc, f3 o, f3 d, float tnear) {
-    const float reach = tnear < 0.0f ? sc.reach : 0.0f;
+__device__ __forceinline__ SlabRay slab_setup(float scene_reach, f3 o, f3 d, float tnear) {
+    const float reach = tnear < 0.0f ? scene_reach : 0.0f;
     SlabRay s;
     slab_axis(o.x, d.x, reach, s.mx, s.ax);
     slab_axis(o.y, d.y, reach, s.my, s.ay);
@@ -116,6 +116,10 @@ struct Trav {
     uint32_t bid;
 };
 struct Bary { float u, v; };
+// What the traversal reads of a scene, by value: a multi-scene launch keeps it in registers (read
+// through the scene table it cost a dependent load per visit).
+struct Geo { const float4 *nodes, *tris; };
+__device__ __forceinline__ Geo geo_of(const SceneDev& sc) { return Geo{sc.nodes, sc.tris}; }
 __device__ __forceinline__ void trav_init(Trav& st, float tfar) {
     st.node = 0; st.sp = 0; st.best = tfar; st.bid = kInvalid;
 }
@@ -132,7 +136,7 @@ __device__ __forceinline__ void trav_init(Trav& st, float tfar) {
 // six blocks per SM without spills beat seven or eight with them: the 4.9 M-path pass over that
 // mesh takes 4.33 ms (8 blocks 4.52, 5 blocks 4.60; subtract-and-multiply test, 8 blocks: 4.60).
 template <bool kAnyHit>
-__device__ __forceinline__ bool trav_run(const SceneDev& sc, const WRay& r, const SlabRay& s, Trav& st,
+__device__ __forceinline__ bool trav_run(const Geo& sc, const WRay& r, const SlabRay& s, Trav& st,
                                          int* __restrict__ stack, int stride, int budget, Bary* uv = nullptr,
                                          bool any = kAnyHit) {
     const float kInf = __int_as_float(0x7f800000);
@@ -373,7 +377,7 @@ __global__ void __launch_bounds__(kTraceBlock, kTraceMinBlocks) k_extend(const _
     bool busy = false;
     Feed feed = feed_init(n);
     uint32_t slot = 0;
-    const SceneDev* sc = &p.scene;
+    Geo geo = geo_of(p.scene);
     WRay r;
     SlabRay sr;
     Trav st;
@@ -385,13 +389,13 @@ __global__ void __launch_bounds__(kTraceBlock, kTraceMinBlocks) k_extend(const _
                 const FilmDev* film = &p.film;
                 if constexpr (kMulti) {
                     const SceneSlot& S = p.multi.scenes[seg_of_slot(cur_batch(p), slot).scene];
-                    sc = &S.scene;
+                    geo = geo_of(S.scene);
                     film = &S.film;
                 }
                 const float4 o = p.wave.ray_o[slot];
                 const float4 d = p.wave.ray_d[slot];
                 wray_setup(r, mk(o.x, o.y, o.z), mk(d.x, d.y, d.z), kSigmaVis);
-                sr = slab_setup(*sc, r.o, r.d, kSigmaVis);
+                sr = slab_setup(0.0f, r.o, r.d, kSigmaVis);
                 // camera unwarp and the film components need the camera ray's closest surface
                 // at any distance (World::Li's record, World.h:749-766); shade still decides
                 // surface vs medium event by comparing with the sampled distance (o.w)
@@ -400,7 +404,7 @@ __global__ void __launch_bounds__(kTraceBlock, kTraceMinBlocks) k_extend(const _
             }
         }
         if (!__any_sync(kFull, busy)) break;
-        if (busy && trav_run<false>(*sc, r, sr, st, stack + threadIdx.x, kTraceBlock, kTravBudget)) {
+        if (busy && trav_run<false>(geo, r, sr, st, stack + threadIdx.x, kTraceBlock, kTravBudget)) {
             p.wave.hit[slot] = make_float2(st.best, __uint_as_float(st.bid));
             busy = false;
         }
@@ -423,7 +427,7 @@ __global__ void __launch_bounds__(kTraceBlock, kTraceMinBlocks) k_shadow(const _
     bool busy = false;
     Feed feed = feed_init(n);
     uint32_t idx = 0;
-    const SceneDev* sc = &p.scene;
+    Geo geo = geo_of(p.scene);
     WRay r;
     SlabRay sr;
     Trav st;
@@ -435,15 +439,15 @@ __global__ void __launch_bounds__(kTraceBlock, kTraceMinBlocks) k_shadow(const _
                 const float4 o = p.wave.sh_o[idx];
                 const float4 d = p.wave.sh_d[idx];
                 if constexpr (kMulti)
-                    sc = &p.multi.scenes[seg_of_slot(cur_batch(p), __float_as_uint(p.wave.sh_L[idx].w)).scene].scene;
+                    geo = geo_of(p.multi.scenes[seg_of_slot(cur_batch(p), __float_as_uint(p.wave.sh_L[idx].w)).scene].scene);
                 wray_setup(r, mk(o.x, o.y, o.z), mk(d.x, d.y, d.z), kSigmaVis);
-                sr = slab_setup(*sc, r.o, r.d, kSigmaVis);
+                sr = slab_setup(0.0f, r.o, r.d, kSigmaVis);
                 trav_init(st, o.w);
                 busy = true;
             }
         }
         if (!__any_sync(kFull, busy)) break;
-        if (busy && trav_run<true>(*sc, r, sr, st, stack + threadIdx.x, kTraceBlock, kTravBudget)) {
+        if (busy && trav_run<true>(geo, r, sr, st, stack + threadIdx.x, kTraceBlock, kTravBudget)) {
             const float4 d = p.wave.sh_d[idx];
             const uint32_t dw = __float_as_uint(d.w);
             if (dw & kConnRay) {
@@ -1024,9 +1028,9 @@ __global__ void __launch_bounds__(kTraceBlock, kPathMinBlocks) k_path(const __gr
             if (busy) {
                 WRay r;
                 wray_setup(r, mk(ps.o.x, ps.o.y, ps.o.z), mk(ps.d.x, ps.d.y, ps.d.z), kSigmaVis);
-                const SlabRay sr = slab_setup(p.scene, r.o, r.d, kSigmaVis);
+                const SlabRay sr = slab_setup(0.0f, r.o, r.d, kSigmaVis);
                 trav_init(st, depth == 0 && (p.film.unwarp || p.film.comps) ? __int_as_float(0x7f800000) : ps.o.w);
-                trav_run<false>(p.scene, r, sr, st, stack + threadIdx.x, kTraceBlock, 0x7fffffff, nullptr, shadow);
+                trav_run<false>(geo_of(p.scene), r, sr, st, stack + threadIdx.x, kTraceBlock, 0x7fffffff, nullptr, shadow);
                 ++rays;
             }
             __syncwarp();
@@ -1298,14 +1302,14 @@ __global__ void __launch_bounds__(kTraceBlock, kTraceMinBlocks) k_trace_user(con
                 i = k;
                 const float4 a = rays[2 * (size_t)i], b = rays[2 * (size_t)i + 1];
                 wray_setup(r, mk(a.x, a.y, a.z), mk(b.x, b.y, b.z), a.w);
-                sr = slab_setup(sc, r.o, r.d, a.w);
+                sr = slab_setup(sc.reach, r.o, r.d, a.w);
                 trav_init(st, b.w);
                 uv = Bary{0.f, 0.f};
                 busy = true;
             }
         }
         if (!__any_sync(kFull, busy)) break;
-        if (busy && trav_run<kAnyHit>(sc, r, sr, st, stack + threadIdx.x, kTraceBlock, kTravBudget, &uv)) {
+        if (busy && trav_run<kAnyHit>(geo_of(sc), r, sr, st, stack + threadIdx.x, kTraceBlock, kTravBudget, &uv)) {
             out[i] = HitOut{st.best, st.bid, uv.u, uv.v};
             busy = false;
         }
