@@ -647,17 +647,27 @@ __device__ __forceinline__ void shade_vertex(const Params& p, int depth, uint32_
         rng.state = ps.rng();
         rng.inc = (cam_id(pixel, B.s0 + sl) << 1u) | 1ull;
 
-        float dist, pd;
-        if (surface) { dist = h.x; pd = medium ? tr_exp(-(dist * lambda)) : 1.0f; }
-        else { dist = dsamp; pd = tr_exp(-(dist * lambda)) * lambda; }
-        const float ptot = th.w * pd;
+        // transmittances exp(-sigma d), evaluated once where coefficients are equal (a gray medium, and
+        // the free-flight rate of one: two of the vertex's seven exponentials)
+        auto transmit = [&](float d, float known_rate, float known) {
+            const float x = sig_t.x == known_rate ? known : tr_exp(-(d * sig_t.x));
+            const float y = sig_t.y == sig_t.x ? x : tr_exp(-(d * sig_t.y));
+            return mk(x, y, sig_t.z == sig_t.x ? x : tr_exp(-(d * sig_t.z)));
+        };
+        const float dist = surface ? h.x : dsamp;
+        float pd = 1.0f;
         f3 f;
         if (medium) {
-            f = mk((th.x * tr_exp(-(dist * sig_t.x))) / ptot, (th.y * tr_exp(-(dist * sig_t.y))) / ptot,
-                   (th.z * tr_exp(-(dist * sig_t.z))) / ptot);
+            const float e = tr_exp(-(dist * lambda));
+            pd = surface ? e : e * lambda;
+            const f3 tr = transmit(dist, lambda, e);
+            const float ptot = th.w * pd;
+            f = mk((th.x * tr.x) / ptot, (th.y * tr.y) / ptot, (th.z * tr.z) / ptot);
         } else {
+            const float ptot = th.w * pd;
             f = mk(th.x / ptot, th.y / ptot, th.z / ptot);
         }
+        const float ptot = th.w * pd;
         const float time = rd.w + dist;
         // camera unwarp: World::Li's record distance = closest surface along the camera
         // ray, FLT_MAX when there is none (World.h:749-766, Ray.h:74-84)
@@ -731,8 +741,7 @@ __device__ __forceinline__ void shade_vertex(const Params& p, int depth, uint32_
                         fe = mk(ph * sig_s.x, ph * sig_s.y, ph * sig_s.z);
                     }
                     f3 att = mk(1.0f, 1.0f, 1.0f);
-                    if (medium)
-                        att = mk(tr_exp(-(sig_t.x * dl)), tr_exp(-(sig_t.y * dl)), tr_exp(-(sig_t.z * dl)));
+                    if (medium) att = transmit(dl, -1.0f, 0.0f);
                     const float scale = inv_inc / pl_;
                     const float Lr = (f.x * (fe.x * (irr.x * att.x))) * scale;
                     const float Lg = (f.y * (fe.y * (irr.y * att.y))) * scale;
