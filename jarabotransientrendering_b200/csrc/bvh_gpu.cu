@@ -5,9 +5,9 @@
 //
 // Three phases, with the counts they hand on kept on the device (the host waits once per few
 // levels, once after the subtrees and once after the collapse):
-//  * levels over the nodes of more than kMid triangles: bounds, bins, split, partition, one launch
-//    each.  A warp takes a run of positions; in the bins its lane b keeps bin b of the three axes in
-//    registers and looks at every triangle of the run, so there are no atomics per triangle;
+//  * levels over the nodes of more than kMid triangles: bins, split, partition (with the children's
+//    boxes), one launch each; a warp takes a run of positions and collects in shared memory and
+//    registers, with one set of global atomics per node it meets;
 //  * the subtrees of at most kMid triangles, one block each, level by level in shared memory, one
 //    warp per node;
 //  * the four-child collapse, one launch per level, nodes in breadth-first order.
@@ -175,78 +175,39 @@ __global__ void k_start(Dev d, uint32_t na, uint32_t nt) {
     if (i0 == 0) (nt > kMid ? d.act[0] : d.mid)[0] = make_uint4(0, nt, 0, 0);
 }
 
-// Box and centroid box of every active node of level parity cur (the root's come from k_prims).
-__global__ void __launch_bounds__(256) k_bounds(Dev d, int cur, uint32_t nt) {
-    if (d.counters[kActive + cur] == 0u) return;
-    const uint32_t lane = threadIdx.x & 31u;
-    const uint32_t p0 = ((blockIdx.x * blockDim.x + threadIdx.x) >> 5) * kWarpRun, p1 = min(nt, p0 + kWarpRun);
-    // a block whose positions all belong to one node collects in shared memory first
-    __shared__ uint32_t keys[12];
-    const uint32_t b0 = blockIdx.x * 8u * kWarpRun, b1 = min(nt, b0 + 8u * kWarpRun);
-    const int32_t one = d.pn[cur][b0] == d.pn[cur][b1 - 1u] ? d.pn[cur][b0] : -1;
-    if (threadIdx.x < 12) keys[threadIdx.x] = empty_key((int)(threadIdx.x % 6u));
-    __syncthreads();
-    Box nb, cb;
-    clear(nb); clear(cb);
-    int32_t node = -1;                                // the node the boxes are of (warp uniform)
-    auto flush = [&]() {
-        warp_union(nb); warp_union(cb);
-        if (lane == 0) {
-            uint32_t* to = one >= 0 ? keys : d.nc[cur] + 12 * node;
+// A warp's bins in shared memory, [axis][box keys, count][bin], and one lane's view of them: bin
+// `lane` of the three axes.
+constexpr uint32_t kBinWords = 21u * kBins;
+struct LaneBins { Box box[3]; uint32_t count[3]; };
+__device__ __forceinline__ void clear_bins(uint32_t* bins, uint32_t lane) {
+#pragma unroll
+    for (uint32_t k = 0; k < 21u; ++k) bins[k * kBins + lane] = k % 7u < 3u ? 0xffffffffu : 0u;
+}
+// one triangle per calling lane into bin b of axis a
+__device__ __forceinline__ void add(uint32_t* bins, uint32_t a, uint32_t b, const uint32_t* lo, const uint32_t* hi) {
+    uint32_t* at = bins + 7u * a * kBins + b;
+#pragma unroll
+    for (int k = 0; k < 3; ++k) {
+        atomicMin(at + k * kBins, lo[k]);
+        atomicMax(at + (3 + k) * kBins, hi[k]);
+    }
+    atomicAdd(at + 6 * kBins, 1u);
+}
+__device__ __forceinline__ LaneBins lane_bins(const uint32_t* bins, uint32_t lane) {
+    LaneBins B;
+#pragma unroll
+    for (int a = 0; a < 3; ++a) {
+        clear(B.box[a]);
+        B.count[a] = bins[(7 * a + 6) * kBins + lane];
+        if (B.count[a]) {
 #pragma unroll
             for (int k = 0; k < 3; ++k) {
-                atomicMin(to + k, key_of(nb.lo[k])); atomicMax(to + 3 + k, key_of(nb.hi[k]));
-                atomicMin(to + 6 + k, key_of(cb.lo[k])); atomicMax(to + 9 + k, key_of(cb.hi[k]));
+                B.box[a].lo[k] = of_key(bins[(7 * a + k) * kBins + lane]);
+                B.box[a].hi[k] = of_key(bins[(7 * a + 3 + k) * kBins + lane]);
             }
         }
-        clear(nb); clear(cb);
-    };
-    for (uint32_t b = p0; b < p1; b += 32u) {
-        const uint32_t i = b + lane;
-        const int32_t n = i < p1 ? d.pn[cur][i] : -1;
-        float4 lo, hi;
-        if (n >= 0) {
-            const uint32_t id = d.ids[cur][i];
-            lo = d.plo[id];
-            hi = d.phi[id];
-        }
-        // the nodes of these 32 positions, one after the other (more than kMid positions each)
-        unsigned left = __ballot_sync(kAll, n >= 0);
-        while (left) {
-            const int32_t m = __shfl_sync(kAll, n, __ffs(left) - 1);
-            if (m != node && node >= 0) flush();
-            node = m;
-            if (n == m) {
-                grow(nb, lo, hi);
-                const float4 c = make_float4(centre(lo.x, hi.x), centre(lo.y, hi.y), centre(lo.z, hi.z), 0.f);
-                grow(cb, c, c);
-            }
-            left &= ~__ballot_sync(kAll, n == m);
-        }
     }
-    if (node >= 0) flush();
-    if (one < 0) return;
-    __syncthreads();
-    if (threadIdx.x < 12) {
-        if (threadIdx.x % 6u < 3) atomicMin(&d.nc[cur][12 * one + threadIdx.x], keys[threadIdx.x]);
-        else atomicMax(&d.nc[cur][12 * one + threadIdx.x], keys[threadIdx.x]);
-    }
-}
-
-// Registers of one lane: bin `lane` of the three axes (box and count).
-struct LaneBins { Box box[3]; uint32_t count[3]; };
-__device__ __forceinline__ void clear(LaneBins& B) {
-#pragma unroll
-    for (int a = 0; a < 3; ++a) { clear(B.box[a]); B.count[a] = 0; }
-}
-// triangle (lo, hi) with its packed bins (five bits per axis)
-__device__ __forceinline__ void add(LaneBins& B, float4 lo, float4 hi, uint32_t bins, uint32_t lane) {
-#pragma unroll
-    for (int a = 0; a < 3; ++a)
-        if (((bins >> (5 * a)) & 31u) == lane) {
-            grow(B.box[a], lo, hi);
-            ++B.count[a];
-        }
+    return B;
 }
 
 // The SAH sweep over a warp's bins: the cheapest split in (axis, bin) order, as the host's strict
@@ -314,76 +275,69 @@ __device__ __forceinline__ Split sweep(const LaneBins& B, uint32_t usable, int l
     return s;
 }
 
-// Bins of every active node.  A warp stages 32 triangles (boxes and packed bins) in shared memory
-// at a time; its lanes then look at each of them, broadcast, and keep their own bin in registers
-// until the node changes: 33 us per level of 328 k triangles where atomics per triangle and axis
-// took 58 us (runs of 512 positions, a quarter of the warps: 62 us).
+// Bins of every active node.  A warp adds its run's triangles to bins of its own in shared memory (a
+// lane per triangle, integer min / max: lanes meet only in the same bin) and those to the node's when
+// the node changes: 18 us per level of 328 k triangles (with each lane scanning the run for its own bin in
+// registers 33 us, with bins shared by a block and float atomics 58 us).
 __global__ void __launch_bounds__(256) k_bin(Dev d, int cur, uint32_t nt) {
     if (blockIdx.x == 0 && threadIdx.x == 0) d.counters[kActive + (cur ^ 1)] = 0u;   // counted by this level's k_split
     if (d.counters[kActive + cur] == 0u) return;
-    __shared__ float4 slo[8][32], shi[8][32];
-    const uint32_t lane = threadIdx.x & 31u, w = threadIdx.x >> 5;
+    __shared__ uint32_t all_bins[8][kBinWords];
+    const uint32_t lane = threadIdx.x & 31u;
+    uint32_t* bins = all_bins[threadIdx.x >> 5];
     const uint32_t p0 = ((blockIdx.x * blockDim.x + threadIdx.x) >> 5) * kWarpRun, p1 = min(nt, p0 + kWarpRun);
-    LaneBins B;
-    clear(B);
+    clear_bins(bins, lane);
+    __syncwarp();
     int32_t node = -1;
     auto flush = [&]() {
-        uint32_t* bb = d.bb + (size_t)node * 21u * kBins + lane;
+        __syncwarp();
+        uint32_t* bb = d.bb + (size_t)node * kBinWords + lane;
 #pragma unroll
         for (int a = 0; a < 3; ++a) {
-            if (B.count[a]) {
+            const uint32_t c = bins[(7 * a + 6) * kBins + lane];
+            if (c) {
 #pragma unroll
                 for (int k = 0; k < 3; ++k) {
-                    atomicMin(bb + (7 * a + k) * kBins, key_of(B.box[a].lo[k]));
-                    atomicMax(bb + (7 * a + 3 + k) * kBins, key_of(B.box[a].hi[k]));
+                    atomicMin(bb + (7 * a + k) * kBins, bins[(7 * a + k) * kBins + lane]);
+                    atomicMax(bb + (7 * a + 3 + k) * kBins, bins[(7 * a + 3 + k) * kBins + lane]);
                 }
-                atomicAdd(bb + (7 * a + 6) * kBins, B.count[a]);
+                atomicAdd(bb + (7 * a + 6) * kBins, c);
             }
         }
-        clear(B);
+        __syncwarp();
+        clear_bins(bins, lane);
+        __syncwarp();
     };
     for (uint32_t b = p0; b < p1; b += 32u) {
         const uint32_t i = b + lane;
         const int32_t n = i < p1 ? d.pn[cur][i] : -1;
-        if (!__any_sync(kAll, n >= 0)) continue;
+        uint32_t lo[3], hi[3], at[3];
+        bool use[3] = {false, false, false};
         if (n >= 0) {
             const uint32_t id = d.ids[cur][i];
-            float4 lo = d.plo[id];
-            const float4 hi = d.phi[id];
-            const float c[3] = {centre(lo.x, hi.x), centre(lo.y, hi.y), centre(lo.z, hi.z)};
-            uint32_t bins = 0;
+            const float4 l = d.plo[id], h = d.phi[id];
+            const float c[3] = {centre(l.x, h.x), centre(l.y, h.y), centre(l.z, h.z)};
+            lo[0] = key_of(l.x); lo[1] = key_of(l.y); lo[2] = key_of(l.z);
+            hi[0] = key_of(h.x); hi[1] = key_of(h.y); hi[2] = key_of(h.z);
 #pragma unroll
             for (int a = 0; a < 3; ++a) {
                 const float clo = of_key(d.nc[cur][12 * n + 6 + a]), ext = of_key(d.nc[cur][12 * n + 9 + a]) - clo;
-                if (ext > 0.f) bins |= (uint32_t)bin_of(c[a], clo, (float)kBins / ext) << (5 * a);
+                use[a] = ext > 0.f;
+                at[a] = use[a] ? (uint32_t)bin_of(c[a], clo, (float)kBins / ext) : 0u;
             }
-            lo.w = __uint_as_float(bins);
-            slo[w][lane] = lo;
-            shi[w][lane] = hi;
         }
-        __syncwarp();
         unsigned left = __ballot_sync(kAll, n >= 0);
         while (left) {
             const int32_t m = __shfl_sync(kAll, n, __ffs(left) - 1);
             if (m != node && node >= 0) flush();
             node = m;
-            const unsigned mine = __ballot_sync(kAll, n == m);
-            if (mine == kAll) {
-#pragma unroll 4
-                for (int j = 0; j < 32; ++j) {
-                    const float4 lo = slo[w][j], hi = shi[w][j];
-                    add(B, lo, hi, __float_as_uint(lo.w), lane);
-                }
-            } else {
-                for (unsigned r = mine; r; r &= r - 1u) {
-                    const int j = __ffs(r) - 1;
-                    const float4 lo = slo[w][j], hi = shi[w][j];
-                    add(B, lo, hi, __float_as_uint(lo.w), lane);
-                }
+            if (n == m) {
+#pragma unroll
+                for (uint32_t a = 0; a < 3; ++a)
+                    if (use[a]) add(bins, a, at[a], lo, hi);
             }
-            left &= ~mine;
+            left &= ~__ballot_sync(kAll, n == m);
         }
-        __syncwarp();
     }
     if (node >= 0) flush();
 }
@@ -409,24 +363,13 @@ __global__ void __launch_bounds__(128) k_split(Dev d, int cur) {
     const uint4 A = d.act[cur][n];
     const uint32_t first = A.x, count = A.y;
     const uint32_t* nc = d.nc[cur] + 12 * n;
-    uint32_t* bb = d.bb + (size_t)n * 21u * kBins + lane;
-    LaneBins B;
+    uint32_t* bb = d.bb + (size_t)n * kBinWords;
     uint32_t usable = 0;
 #pragma unroll
-    for (int a = 0; a < 3; ++a) {
+    for (int a = 0; a < 3; ++a)
         if (of_key(nc[9 + a]) - of_key(nc[6 + a]) > 0.f) usable |= 1u << a;
-        B.count[a] = bb[(7 * a + 6) * kBins];
-        clear(B.box[a]);
-        if (B.count[a]) {
-#pragma unroll
-            for (int k = 0; k < 3; ++k) {
-                B.box[a].lo[k] = of_key(bb[(7 * a + k) * kBins]);
-                B.box[a].hi[k] = of_key(bb[(7 * a + 3 + k) * kBins]);
-            }
-        }
-#pragma unroll
-        for (int k = 0; k < 7; ++k) bb[(7 * a + k) * kBins] = k < 3 ? 0xffffffffu : 0u;
-    }
+    const LaneBins B = lane_bins(bb, (uint32_t)lane);
+    clear_bins(bb, (uint32_t)lane);
     if (lane < 24) d.nc[cur ^ 1][24 * n + lane] = empty_key(lane);
     const Split s = sweep(B, usable, lane);
     if (lane != 0) return;
@@ -453,8 +396,9 @@ __global__ void __launch_bounds__(128) k_split(Dev d, int cur) {
 }
 
 // Triangles into their child's range (order within a child is arbitrary: min/max and counts do not
-// depend on it); finished positions are carried over unchanged.  A warp whose run lies in one node
-// takes its slots of each child with one atomic, else the lanes going to the same child do so per 32
+// depend on it), and the boxes and centroid boxes of the children that go on to the next level;
+// finished positions are carried over unchanged.  A warp whose run lies in one node reduces the boxes and
+// takes its slots of each child with one set of atomics, else the lanes do so one by one and per 32
 // positions.
 __global__ void __launch_bounds__(256) k_partition(Dev d, int cur, uint32_t nt) {
     constexpr int kIt = (int)(kWarpRun / 32u);
@@ -465,6 +409,8 @@ __global__ void __launch_bounds__(256) k_partition(Dev d, int cur, uint32_t nt) 
     int32_t node[kIt];
     uint32_t id[kIt];
     unsigned right = 0, move = 0;                     // bit k: position p0 + 32 k + lane goes right / is moved
+    Box nb[2], cb[2];                                 // of the lane's triangles, by side
+    clear(nb[0]); clear(nb[1]); clear(cb[0]); clear(cb[1]);
     bool same = true;
     int32_t first_node = 0;
 #pragma unroll
@@ -475,18 +421,50 @@ __global__ void __launch_bounds__(256) k_partition(Dev d, int cur, uint32_t nt) 
         if (k == 0) first_node = __shfl_sync(kAll, node[0], 0);
         same = same && node[k] == first_node;
     }
+    const bool one = __all_sync(kAll, same && first_node >= 0);      // the whole run in one node
+    auto add_box = [&](int32_t child, const Box& n, const Box& c) {
+        uint32_t* to = d.nc[cur ^ 1] + 12 * child;
+#pragma unroll
+        for (int e = 0; e < 3; ++e) {
+            atomicMin(to + e, key_of(n.lo[e])); atomicMax(to + 3 + e, key_of(n.hi[e]));
+            atomicMin(to + 6 + e, key_of(c.lo[e])); atomicMax(to + 9 + e, key_of(c.hi[e]));
+        }
+    };
 #pragma unroll
     for (int k = 0; k < kIt; ++k) {
         const int32_t n = node[k];
         if (n < 0) continue;
         const int32_t ax = d.d_ax[n];
+        const float4 lo = d.plo[id[k]], hi = d.phi[id[k]];
+        const float4 c = make_float4(centre(lo.x, hi.x), centre(lo.y, hi.y), centre(lo.z, hi.z), 0.f);
+        bool r;
         if (ax < 0) {
-            if (p0 + 32u * k + lane - d.act[cur][n].x >= d.d_nl[n]) right |= 1u << k;
+            r = p0 + 32u * k + lane - d.act[cur][n].x >= d.d_nl[n];
         } else {
             const float2 sc = d.d_scale[n];
-            const float c = centre(reinterpret_cast<const float*>(d.plo + id[k])[ax], reinterpret_cast<const float*>(d.phi + id[k])[ax]);
-            if (bin_of(c, sc.x, sc.y) > d.d_split[n]) right |= 1u << k;
+            r = bin_of(ax == 0 ? c.x : ax == 1 ? c.y : c.z, sc.x, sc.y) > d.d_split[n];
             move |= 1u << k;
+        }
+        if (r) right |= 1u << k;
+        if (one) {
+            if (r) { grow(nb[1], lo, hi); grow(cb[1], c, c); }
+            else { grow(nb[0], lo, hi); grow(cb[0], c, c); }
+        } else if (d.d_child[2 * n + (r ? 1 : 0)] >= 0) {
+            Box b1, b2;
+            clear(b1); clear(b2);
+            grow(b1, lo, hi);
+            grow(b2, c, c);
+            add_box(d.d_child[2 * n + (r ? 1 : 0)], b1, b2);
+        }
+    }
+    if (one) {
+#pragma unroll
+        for (int side = 0; side < 2; ++side) {
+            const int32_t child = d.d_child[2 * first_node + side];
+            if (child < 0) continue;                  // warp uniform
+            warp_union(nb[side]);
+            warp_union(cb[side]);
+            if (lane == 0) add_box(child, nb[side], cb[side]);
         }
     }
     const bool run = __all_sync(kAll, same && move == (1u << kIt) - 1u);
@@ -529,8 +507,9 @@ __global__ void __launch_bounds__(256) k_partition(Dev d, int cur, uint32_t nt) 
 
 // One block per subtree of at most kMid triangles, down to the leaves (written where the subtree's
 // triangle positions are): its nodes level by level, 8 or 16 lanes per node of at most as many
-// triangles, one warp per larger node.  Bound by min / max issue: 328 k triangles take 363 us (420 us
-// with a warp sweep per node of 9 to 16, 507 us with a warp per node and leaf).
+// triangles, one warp per larger node.  Bound by min / max issue and the latency of a node's steps: 328 k
+// triangles take 251 us (363 us with the bins scanned by their lanes, 420 us with a warp sweep per
+// node of 9 to 16 too, 507 us with a warp per node and leaf).
 struct MidItem { uint16_t first, count; uint32_t out; };
 // Nodes of at most G triangles, one per G lanes of the warp (lane t of a group: its node's triangle t);
 // `on`: the lane's group has a node.  Every triangle's bin is a split candidate on each axis; the lanes
@@ -634,6 +613,7 @@ __global__ void __launch_bounds__(kMidThreads) k_mid(Dev d, int cur, uint32_t* _
     __shared__ uint16_t perm[kMid], tmp[kMid];
     __shared__ MidItem q[2][kMid];
     __shared__ uint32_t qn[2], next_node, max_depth;
+    __shared__ uint32_t all_bins[kMidThreads / 32][kBinWords];
     if (blockIdx.x >= d.counters[kNumMid]) return;
     const uint4 S = d.mid[blockIdx.x];
     const uint32_t n = S.y;
@@ -731,26 +711,27 @@ __global__ void __launch_bounds__(kMidThreads) k_mid(Dev d, int cur, uint32_t* _
                     scale[a] = ext > 0.f ? (float)kBins / ext : 0.f;
                     usable |= ext > 0.f ? 1u << a : 0u;
                 }
-                // packed bins of the node's triangles (beside their boxes)
+                // the triangles' packed bins (beside their boxes) and the warp's bins of them
+                uint32_t* wb = all_bins[warp];
+                clear_bins(wb, (uint32_t)lane);
+                __syncwarp();
                 for (uint32_t i = f + lane; i < f + cnt; i += 32u) {
                     const uint32_t j = perm[i];
                     const float4 lo = slo[j], hi = shi[j];
                     const float ce[3] = {centre(lo.x, hi.x), centre(lo.y, hi.y), centre(lo.z, hi.z)};
+                    const uint32_t kl[3] = {key_of(lo.x), key_of(lo.y), key_of(lo.z)}, kh[3] = {key_of(hi.x), key_of(hi.y), key_of(hi.z)};
                     uint32_t bins = 0;
 #pragma unroll
-                    for (int a = 0; a < 3; ++a)
-                        if ((usable >> a) & 1u) bins |= (uint32_t)bin_of(ce[a], cb.lo[a], scale[a]) << (5 * a);
+                    for (uint32_t a = 0; a < 3; ++a)
+                        if ((usable >> a) & 1u) {
+                            const uint32_t bin = (uint32_t)bin_of(ce[a], cb.lo[a], scale[a]);
+                            bins |= bin << (5 * a);
+                            add(wb, a, bin, kl, kh);
+                        }
                     slo[j].w = __uint_as_float(bins);
                 }
                 __syncwarp();
-                LaneBins B;
-                clear(B);
-#pragma unroll 4
-                for (uint32_t i = f; i < f + cnt; ++i) {
-                    const uint32_t j = perm[i];
-                    const float4 lo = slo[j], hi = shi[j];
-                    add(B, lo, hi, __float_as_uint(lo.w), (uint32_t)lane);
-                }
+                const LaneBins B = lane_bins(wb, (uint32_t)lane);
                 const Split s = sweep(B, usable, lane);
                 uint32_t nl = cnt / 2;                   // median split by position without a SAH split
                 if (s.axis >= 0) {
@@ -940,7 +921,6 @@ bool build_bvh_device(const float* d_v, uint32_t nv, const uint32_t* d_t, uint32
     for (bool more = nt > kMid; more;) {
         for (uint32_t k = 0; k < ahead; ++k, ++level) {
             const uint32_t na = level < 28 ? std::min(amax, 1u << level) : amax;
-            if (level) k_bounds<<<run_blocks, 256, 0, s>>>(d, cur, nt);      // the root's come from k_prims
             k_bin<<<run_blocks, 256, 0, s>>>(d, cur, nt);
             k_split<<<(na + 3) / 4, 128, 0, s>>>(d, cur);                    // one warp per active node
             k_partition<<<run_blocks, 256, 0, s>>>(d, cur, nt);
