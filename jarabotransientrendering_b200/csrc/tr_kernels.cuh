@@ -264,6 +264,9 @@ cudaError_t launch_build_tris(const float* vertices, const uint32_t* triangles, 
 // FP64 film sums -> FP32 (film streaming)
 cudaError_t launch_to_f32(const double* src, float* dst, size_t n, cudaStream_t s);
 
+// arrays of n[k] doubles to dst[k] (null: skipped) on the same device, in one launch
+cudaError_t launch_copy3(const double* const* src, double* const* dst, const size_t* n, cudaStream_t s);
+
 cudaError_t launch_advance(uint32_t* cur, uint32_t step, cudaStream_t s);
 cudaError_t launch_trace_user(const SceneDev& sc, const float* rays, uint32_t n, int any_hit,
                               void* out_hits, uint32_t* cursor, int grid, cudaStream_t s);
