@@ -609,6 +609,10 @@ tr_status render_region(tr_ctx* x, uint32_t x0, uint32_t y0, uint32_t x1, uint32
             p.batch.splat_unit = large > 1 ? unit : npix;
             p.batch.s0 = s0 + sb; p.batch.ns = ns; p.batch.ninc = ninc;
             p.batch.n_slots = npix * per_pix;
+            // one batch in flight: its last depths in one launch (per-kernel timing keeps them apart)
+            if (!whole && lanes == 1 && !guided && !bidir && !x->profiling && !(x->integ.flags & TR_FLAG_TIME_SAMPLING) &&
+                x->integ.max_bounces >= trk::kTailMinBounces)
+                p.tail_paths = trk::kTailPaths;
             if (whole) {
                 tl(1, [&] { return trk::launch_paths(p, ls); });
             } else {
@@ -690,6 +694,10 @@ tr_status render_region(tr_ctx* x, uint32_t x0, uint32_t y0, uint32_t x1, uint32
                 if (s_gen && d < x->bd.nvert) connect(d);
             }
             if (!whole && x->integ.max_bounces) TR_CUDA(order(lsh, ls));
+            if (p.tail_paths) {
+                tl(1, [&] { return trk::launch_tail(p, ls); });
+                launches += 1;
+            }
             if (guided && x->guide_pool) {
                 TR_CUDA(trk::launch_train_gather(p, x->pool_state, ls));
                 launches += 2;

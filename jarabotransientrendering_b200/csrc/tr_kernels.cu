@@ -365,6 +365,11 @@ __device__ __forceinline__ bool refill(Feed& f, bool busy, uint32_t* cursor, uin
     return got && !busy;
 }
 
+// depths that may be left to launch_tail
+__device__ __forceinline__ bool in_tail(const Params& p, int depth) {
+    return depth > 0 && (uint32_t)depth + kTailDepths <= p.max_bounces;
+}
+
 // Closest hit of each queued ray.  Persistent warps; a lane whose ray is done takes the next
 // queued ray at the warp's next refill point, so the lanes stay busy while rays of very
 // different traversal lengths share a warp.
@@ -374,6 +379,7 @@ __global__ void __launch_bounds__(kTraceBlock, kTraceMinBlocks) k_extend(const _
     uint32_t n0 = p.batch.n_slots;
     if constexpr (kMulti) n0 = cur_batch(p).n_slots;
     const uint32_t n = depth == 0 ? n0 : p.wave.counters[cnt_ext(depth)];
+    if (!kMulti && n <= p.tail_paths && in_tail(p, depth)) return;      // left to launch_tail
     const uint32_t* q = p.wave.q[depth & 1];
     uint32_t* cursor = &p.wave.counters[cur_ext(depth)];
     if (blockIdx.x == 0 && threadIdx.x == 0) atomicAdd(&p.wave.stats[0], (unsigned long long)n);
@@ -909,6 +915,7 @@ __global__ void __launch_bounds__(256, kMulti ? 3 : (kTimeSampling ? 3 : 4))
     uint32_t n0 = p.batch.n_slots;
     if constexpr (kMulti) n0 = cur_batch(p).n_slots;
     const uint32_t n = depth == 0 ? n0 : p.wave.counters[cnt_ext(depth)];
+    if (!kMulti && n <= p.tail_paths && in_tail(p, depth)) return;      // left to launch_tail
     const uint32_t* qin = p.wave.q[depth & 1];
     uint32_t* qout = p.wave.q[(depth + 1) & 1];
     const unsigned lane = threadIdx.x & 31u;
@@ -991,6 +998,7 @@ __global__ void __launch_bounds__(256, kMulti ? 3 : (kTimeSampling ? 3 : 4))
 // / 510 -> 280 us, over 328 k triangles 580 -> 190 / 770 -> 350 us.  Lanes whose path has ended stay
 // idle until their group of paths is done: refilling them (other depths, other directions) made
 // 131 k paths over 328 k triangles 448 -> 561 us.
+// kTail: the paths that a wavefront batch has left at its first depth with few of them (launch_tail).
 // -----------------------------------------------------------------------------------------
 constexpr int kPathMinBlocks = 5;    // 96 registers; 4 and 6 blocks per SM are within 5 %
 struct RegState {
@@ -1010,7 +1018,7 @@ __device__ __forceinline__ float4 shfl4(float4 v, int src) {
     return make_float4(__shfl_sync(kFull, v.x, src), __shfl_sync(kFull, v.y, src), __shfl_sync(kFull, v.z, src),
                        __shfl_sync(kFull, v.w, src));
 }
-template <bool kTimeSampling>
+template <bool kTimeSampling, bool kTail>
 __global__ void __launch_bounds__(kTraceBlock, kPathMinBlocks) k_path(const __grid_constant__ Params p, uint32_t per_warp) {
     extern __shared__ int stack[];     // [stack entries][kTraceBlock]
     __shared__ uint32_t totals[3];
@@ -1019,23 +1027,40 @@ __global__ void __launch_bounds__(kTraceBlock, kPathMinBlocks) k_path(const __gr
     const int lane = (int)(threadIdx.x & 31u);
     const bool shadow = (lane & 1) != 0;
     const uint32_t w = blockIdx.x * (kTraceBlock / 32u) + (threadIdx.x >> 5), nw = gridDim.x * (kTraceBlock / 32u);
-    const uint32_t n = p.batch.n_slots;
+    uint32_t n = p.batch.n_slots;
+    int first = 0;
+    if constexpr (kTail) {
+        // the first depth whose queue the wavefront kernels left
+        n = kInvalid;
+        for (first = 1; in_tail(p, first) && (n = p.wave.counters[cnt_ext(first)]) > p.tail_paths;) ++first;
+        if (n > p.tail_paths) n = 0;
+        per_warp = min(16u, max(1u, (n + nw - 1u) / nw));
+    }
     const size_t rs = p.wave.capacity;          // record stride: records are [bounce][slot]
     uint32_t rays = 0, splats = 0;
     for (uint32_t group = w; (unsigned long long)group * per_warp < n; group += nw) {
-        const uint32_t slot = group * per_warp + (uint32_t)(lane >> 1);
+        uint32_t slot = group * per_warp + (uint32_t)(lane >> 1);
         const bool have = (uint32_t)(lane >> 1) < per_warp && slot < n;
+        if (kTail && have) slot = p.wave.q[first & 1][slot];
         // the ray to trace next: the walk's, or the shadow ray (its contribution in ps.t)
         RegState ps;
         bool busy = false;
         uint32_t records = 0;
-        if (have && !shadow && p.max_bounces) {
+        if constexpr (kTail) {
+            if (have && shadow) records = p.wave.rec_n[slot];
+            if (have && !shadow) {
+                ps.o = p.wave.ray_o[slot]; ps.d = p.wave.ray_d[slot]; ps.t = p.wave.thr[slot];
+                ps.rn = p.wave.rng[slot]; ps.cam = p.wave.cam_dist[slot];
+                busy = true;
+            }
+        } else if (have && !shadow && p.max_bounces) {
             const CameraPath cp = camera_path(slot, p.batch, p.film, p.cam, p.scene, p.seed, p.sqrt_spp, p.flags);
             ps.o = cp.o; ps.d = cp.d; ps.rn = cp.rng; ps.light = cp.target;
             ps.t = make_float4(1.0f, 1.0f, 1.0f, 1.0f);
             busy = true;
         }
-        for (int depth = 0; __any_sync(kFull, busy); ++depth) {
+        const uint32_t recorded = records;
+        for (int depth = first; __any_sync(kFull, busy); ++depth) {
             Trav st;
             if (busy) {
                 WRay r;
@@ -1067,7 +1092,7 @@ __global__ void __launch_bounds__(kTraceBlock, kPathMinBlocks) k_path(const __gr
         }
         if (have && shadow) {
             p.wave.rec_n[slot] = (uint8_t)records;
-            splats += records;
+            splats += records - recorded;
         }
     }
     const uint32_t walks = __reduce_add_sync(kFull, shadow ? 0u : rays), casts = __reduce_add_sync(kFull, shadow ? rays : 0u);
@@ -1786,8 +1811,24 @@ cudaError_t launch_paths(const Params& p, cudaStream_t s) {
     const uint32_t per_warp = std::min(16u, std::max(1u, (n + warps - 1) / warps));
     const uint32_t per_block = per_warp * (kTraceBlock / 32u);
     const uint32_t grid = std::max(1u, std::min((n + per_block - 1) / per_block, warps / (kTraceBlock / 32u)));
-    if (p.flags & kFlagTimeSampling) k_path<true><<<grid, kTraceBlock, trace_smem_bytes(p.bvh_depth), s>>>(p, per_warp);
-    else k_path<false><<<grid, kTraceBlock, trace_smem_bytes(p.bvh_depth), s>>>(p, per_warp);
+    if (p.flags & kFlagTimeSampling) k_path<true, false><<<grid, kTraceBlock, trace_smem_bytes(p.bvh_depth), s>>>(p, per_warp);
+    else k_path<false, false><<<grid, kTraceBlock, trace_smem_bytes(p.bvh_depth), s>>>(p, per_warp);
+    return cudaGetLastError();
+}
+// The deepest depths of a batch that has the GPU to itself: few paths, and three launches per depth
+// that last as long as their longest ray.  From the first depth with at most tail_paths paths (what the
+// resident warps take at sixteen each) k_path walks them to their end; the wavefront launches behind
+// it find empty queues.  Where the line lies: three depths or more have to be left (room, depth 6, two
+// left: 774 -> 794 us), and a render of less than kTailMinBounces only pays for the empty launch (775 ->
+// 781 us).  Depth 8: 131 k room paths 344 -> 331 us, 524 k over 20 k triangles 1001 -> 942, 1 M over 328 k
+// triangles 1946 -> 1854; depth 12: 1 M room paths 1075 -> 1044.  A quarter or three times the paths gain
+// less (1 M room paths 1048 / 1085 us).  Batches on several lanes fill each other's tails (equal).
+cudaError_t launch_tail(const Params& p, cudaStream_t s) {
+    if (reinterpret_cast<uintptr_t>(p.scene.nodes) & 31u) return cudaErrorMisalignedAddress;
+    int dev = 0, sms = 1;
+    cudaGetDevice(&dev);
+    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+    k_path<false, true><<<sms * kPathMinBlocks, kTraceBlock, trace_smem_bytes(p.bvh_depth), s>>>(p, 1u);
     return cudaGetLastError();
 }
 cudaError_t launch_shadow(const Params& p, int depth, int grid, cudaStream_t s) {

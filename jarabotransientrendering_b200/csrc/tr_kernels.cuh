@@ -197,6 +197,7 @@ struct Params {
     GuideWave guide;
     MultiDev multi;              // used by the kMulti kernel variants only
     BidirWave bd;                // light subpaths and vertex connections
+    uint32_t tail_paths;         // from the first depth with at most so many paths on, they are launch_tail's
 };
 
 // ---- per-slot view (device) ------------------------------------------------------------
@@ -242,6 +243,10 @@ cudaError_t launch_shadow(const Params& p, int depth, int grid, cudaStream_t s);
 // proposal, no light subpaths) of few paths
 bool paths_fit(unsigned long long paths, uint32_t bvh_depth);
 cudaError_t launch_paths(const Params& p, cudaStream_t s);
+cudaError_t launch_tail(const Params& p, cudaStream_t s);      // after a batch's last depth, with tail_paths
+constexpr uint32_t kTailPaths = 148u * 5u * 4u * 16u;
+constexpr uint32_t kTailDepths = 3;         // at least so many depths are left to launch_tail
+constexpr uint32_t kTailMinBounces = 7;
 // bsel < 0: the film itself; bsel = b: per-bounce film b (records of bounce min(depth, N-1) == b)
 // pixels per splat block: automatic (whole pixels filling one block) in single-scene mode,
 // each segment's splat_g in multi-scene mode
