@@ -1,5 +1,5 @@
-// bvh_build.cpp - binned-SAH BVH builder (host) producing the 64-byte two-child node layout
-// the GPU traversal reads.  Replaces Embree's BVH build inside World::freeze / rtcCommit
+// bvh_build.cpp - binned-SAH BVH builder (host): a two-child tree, collapsed to four-child nodes.
+// Replaces Embree's BVH build inside World::freeze / rtcCommit
 // (src/RayTracing/World.h:543-550) for the GPU path.
 #include "bvh_build.h"
 

@@ -6,9 +6,8 @@
 
 namespace trh {
 
-// 128-byte four-child node, read by the kernels as eight 16-byte vector loads:
-//   q0..q5 = child bounds lo.x[4], hi.x[4], lo.y[4], hi.y[4], lo.z[4], hi.z[4]
-//   q6 = child refs[4], q7 = padding
+// 128-byte four-child node of the host build; the upload lays it out as DevNode, which the kernels
+// read (tr_internal.h).
 // ref >= 0: interior node index; ref < 0: leaf, ~ref = (first_triangle << 3) | count
 // (count 0: empty slot, never entered).
 struct alignas(16) GpuNode {

@@ -10,6 +10,8 @@
 //   splat   (per group of whole pixels: records read bounce-major; lanes with equal
 //            (pixel, bin) keys found with __match_any_sync, summed in FP32 by a shuffle tree,
 //            one native FP64 atomicAdd per group into the film in HBM)
+// A small batch runs path (all of the above but splat, in one launch, two lanes per path) and splat;
+// a larger one on its own leaves its last depths to path.
 // Reference path: src/Integrator/BidirectionalPathTracing.h:485-692,975-1140 and
 // src/Film/StreakCameraFilm.h:139-192 (details at each kernel).
 #include "tr_bsdf.cuh"
