@@ -19,9 +19,13 @@ namespace tri {
 // records msg as the thread's last error (tr_last_error) and returns s
 tr_status fail(tr_status s, const std::string& msg);
 
+// A failed CUDA call.  The runtime's own record of the error is taken back with it: the launchers report
+// cudaGetLastError(), so one left behind (an allocation that did not fit) would fail the thread's next launch.
 struct CudaError : std::runtime_error {
     cudaError_t code;
-    CudaError(cudaError_t c, const char* what) : std::runtime_error(std::string(what) + ": " + cudaGetErrorString(c)), code(c) {}
+    CudaError(cudaError_t c, const char* what) : std::runtime_error(std::string(what) + ": " + cudaGetErrorString(c)), code(c) {
+        cudaGetLastError();
+    }
 };
 
 #define TR_CUDA(call)                                           \
