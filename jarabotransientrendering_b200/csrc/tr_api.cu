@@ -171,76 +171,77 @@ size_t carve_wave(trk::Wave* w, void* block, uint32_t capacity, size_t R, bool t
     return at;
 }
 
+// Gives the first wave's path state back to the pool, the light subpaths' and connections' with it.
+static void drop_first_wave(tr_ctx* x) {
+    trk::Wave& lw = x->lwave;
+    trk::BidirWave& bd = x->bd;
+    x->drop(x->wave.block);
+    x->wave.capacity = 0;
+    x->drop(lw.ray_o); x->drop(lw.ray_d); x->drop(lw.thr); x->drop(lw.rng); x->drop(lw.hit); x->drop(lw.q[0]); x->drop(lw.q[1]);
+    x->drop(bd.lvert); x->drop(bd.evert); x->drop(bd.nl); x->drop(bd.ne); x->drop(bd.L0);
+    x->drop(bd.co_o); x->drop(bd.co_d); x->drop(bd.co_L); x->drop(bd.valid);
+}
+
 void ensure_wave(tr_ctx* x, uint32_t capacity) {
     if (x->wave.capacity >= capacity) return;
     // grow: drop the old buffers (they are only scratch between calls)
-    auto drop = [&](void* p) {
-        if (!p) return;
-        cudaFree(p);
-        x->allocs.erase(std::remove(x->allocs.begin(), x->allocs.end(), p), x->allocs.end());
-    };
+    drop_first_wave(x);
     trk::Wave& w = x->wave;
-    drop(w.block);
-    w.block = nullptr;
-    w.capacity = 0;
     size_t R = std::max<uint32_t>(1u, x->integ.max_bounces);
     // records per slot: one next-event estimate per bounce, plus with light subpaths one per
     // eye-light vertex pair with ie + il + 2 <= max_bounces
     if (x->integ.flags & TR_FLAG_BIDIRECTIONAL) R += R * (R - 1) / 2;
     const bool tsm = (x->integ.flags & TR_FLAG_TIME_SAMPLING) != 0;
-    void* block = x->alloc<unsigned char>(carve_wave(nullptr, nullptr, capacity, R, tsm));
-    if (x->integ.flags & TR_FLAG_BIDIRECTIONAL) {
-        // light wave (own rays, queues, counters; shares target and ray counts) and the
-        // subpath vertex arrays
-        trk::Wave& lw = x->lwave;
-        trk::BidirWave& bd = x->bd;
-        drop(lw.ray_o); drop(lw.ray_d); drop(lw.thr); drop(lw.rng); drop(lw.hit); drop(lw.q[0]); drop(lw.q[1]);
-        drop(bd.lvert); drop(bd.evert); drop(bd.nl); drop(bd.ne); drop(bd.L0);
-        lw = trk::Wave{};
-        lw.ray_o = x->alloc<float4>(capacity);
-        lw.ray_d = x->alloc<float4>(capacity);
-        lw.thr = x->alloc<float4>(capacity);
-        lw.rng = x->alloc<unsigned long long>(capacity);
-        lw.hit = x->alloc<float2>(capacity);
-        lw.q[0] = x->alloc<uint32_t>(capacity);
-        lw.q[1] = x->alloc<uint32_t>(capacity);
-        if (!x->d_lcounters) x->d_lcounters = x->alloc<uint32_t>(trk::kCounters);
-        lw.counters = x->d_lcounters;
-        bd.nvert = std::max<uint32_t>(1u, x->integ.max_bounces) - 1u;
-        const size_t nv = std::max<uint32_t>(1u, bd.nvert);
-        bd.lvert = x->alloc<float4>(nv * 4 * capacity);
-        bd.evert = x->alloc<float4>(nv * 4 * capacity);
-        bd.nl = x->alloc<uint8_t>(capacity);
-        bd.ne = x->alloc<uint8_t>(capacity);
-        bd.L0 = x->alloc<float4>(capacity);
-        // connection queues of one eye depth (up to nvert rays per slot) and the record flags.  With
-        // two queues the next depth's rays are set up while this one's are traced.
-        drop(bd.co_o); drop(bd.co_d); drop(bd.co_L); drop(bd.valid);
-        bd.co_o = bd.co_d = bd.co_L = nullptr;
-        bd.valid = nullptr;
-        for (x->bd_queues = 2;; x->bd_queues = 1) {
-            try {
-                const size_t q = nv * x->bd_queues * capacity;
-                bd.co_o = x->alloc<float4>(q);
-                bd.co_d = x->alloc<float4>(q);
-                bd.co_L = x->alloc<float4>(q);
-                break;
-            } catch (const CudaError& e) {
-                if (e.code != cudaErrorMemoryAllocation || x->bd_queues == 1) throw;
-                cudaGetLastError();
-                drop(bd.co_o); drop(bd.co_d);
-                bd.co_o = bd.co_d = nullptr;
+    try {
+        w.block = x->alloc<unsigned char>(carve_wave(nullptr, nullptr, capacity, R, tsm));
+        if (x->integ.flags & TR_FLAG_BIDIRECTIONAL) {
+            // light wave (own rays, queues, counters; shares target and ray counts) and the
+            // subpath vertex arrays
+            trk::Wave& lw = x->lwave;
+            trk::BidirWave& bd = x->bd;
+            lw.ray_o = x->alloc<float4>(capacity);
+            lw.ray_d = x->alloc<float4>(capacity);
+            lw.thr = x->alloc<float4>(capacity);
+            lw.rng = x->alloc<unsigned long long>(capacity);
+            lw.hit = x->alloc<float2>(capacity);
+            lw.q[0] = x->alloc<uint32_t>(capacity);
+            lw.q[1] = x->alloc<uint32_t>(capacity);
+            if (!x->d_lcounters) x->d_lcounters = x->alloc<uint32_t>(trk::kCounters);
+            lw.counters = x->d_lcounters;
+            bd.nvert = std::max<uint32_t>(1u, x->integ.max_bounces) - 1u;
+            bd.ncand = x->integ.max_bounces * bd.nvert / 2u;
+            const size_t nv = std::max<uint32_t>(1u, bd.nvert);
+            bd.lvert = x->alloc<float4>(nv * 4 * capacity);
+            bd.evert = x->alloc<float4>(nv * 4 * capacity);
+            bd.nl = x->alloc<uint8_t>(capacity);
+            bd.ne = x->alloc<uint8_t>(capacity);
+            bd.L0 = x->alloc<float4>(capacity);
+            // connection queues of one eye depth (up to nvert rays per slot) and the record flags.  With
+            // two queues the next depth's rays are set up while this one's are traced.
+            for (x->bd_queues = 2;; x->bd_queues = 1) {
+                try {
+                    const size_t q = nv * x->bd_queues * capacity;
+                    bd.co_o = x->alloc<float4>(q);
+                    bd.co_d = x->alloc<float4>(q);
+                    bd.co_L = x->alloc<float4>(q);
+                    bd.valid = x->alloc<uint8_t>(R * capacity);
+                    break;
+                } catch (const CudaError& e) {
+                    if (e.code != cudaErrorMemoryAllocation || x->bd_queues == 1) throw;
+                    x->drop(bd.co_o); x->drop(bd.co_d); x->drop(bd.co_L);
+                }
             }
         }
-        bd.ncand = x->integ.max_bounces * (std::max<uint32_t>(1u, x->integ.max_bounces) - 1u) / 2u;
-        bd.valid = x->alloc<uint8_t>(R * capacity);
+        if (!w.counters) w.counters = x->alloc<uint32_t>(trk::kCounters);
+        if (!w.stats) {
+            w.stats = x->alloc<unsigned long long>(8);
+            TR_CUDA(cudaMemsetAsync(w.stats, 0, 8 * sizeof(unsigned long long), x->s()));
+        }
+    } catch (const CudaError&) {
+        drop_first_wave(x);
+        throw;
     }
-    if (!w.counters) w.counters = x->alloc<uint32_t>(trk::kCounters);
-    if (!w.stats) {
-        w.stats = x->alloc<unsigned long long>(8);
-        TR_CUDA(cudaMemsetAsync(w.stats, 0, 8 * sizeof(unsigned long long), x->s()));
-    }
-    carve_wave(&w, block, capacity, R, tsm);
+    carve_wave(&w, w.block, capacity, R, tsm);
 }
 
 // Per-kind kernel times of the pending timed launches and the union of the traversal (extend,
@@ -284,21 +285,11 @@ void prof_publish(tr_ctx* x) {
 
 // Gives the path state of all lanes back to the pool (its contents are only scratch between calls).
 void drop_waves(tr_ctx* x) {
-    auto drop = [&](void* p) {
-        if (!p) return;
-        cudaFree(p);
-        x->allocs.erase(std::remove(x->allocs.begin(), x->allocs.end(), p), x->allocs.end());
-    };
-    auto drop_wave = [&](trk::Wave& w) {
-        drop(w.block);
-        w.block = nullptr;
-        w.capacity = 0;
-    };
-    drop_wave(x->wave);
-    for (trk::Wave& w : x->lane_wave) drop_wave(w);
+    drop_first_wave(x);
     for (int k = 0; k + 1 < kWaveLanes; ++k) {
-        drop(x->lane_vrec[k]);
-        x->lane_vrec[k] = nullptr;
+        x->drop(x->lane_wave[k].block);
+        x->lane_wave[k].capacity = 0;
+        x->drop(x->lane_vrec[k]);
         x->lane_vrec_cap[k] = 0;
     }
 }
@@ -308,49 +299,32 @@ void drop_waves(tr_ctx* x) {
 void ensure_lane_wave(tr_ctx* x, int k, uint32_t capacity) {
     trk::Wave& w = x->lane_wave[k];
     if (w.capacity >= capacity && w.counters) return;
-    auto drop = [&](void* p) {
-        if (!p) return;
-        cudaFree(p);
-        x->allocs.erase(std::remove(x->allocs.begin(), x->allocs.end(), p), x->allocs.end());
-    };
-    drop(w.block);
-    w.block = nullptr;
+    x->drop(w.block);
     w.capacity = 0;
     const size_t R = std::max<uint32_t>(1u, x->integ.max_bounces);
     const bool tsm = (x->integ.flags & TR_FLAG_TIME_SAMPLING) != 0;
-    void* block = x->alloc<unsigned char>(carve_wave(nullptr, nullptr, capacity, R, tsm));
+    w.block = x->alloc<unsigned char>(carve_wave(nullptr, nullptr, capacity, R, tsm));
     if (!w.counters) w.counters = x->alloc<uint32_t>(trk::kCounters);
     w.stats = x->wave.stats;
-    carve_wave(&w, block, capacity, R, tsm);
+    carve_wave(&w, w.block, capacity, R, tsm);
 }
 
 // Lane k + 1's guided-vertex records (the training pool and its counters are shared: the
 // batches of all lanes fill it, each entry tagged with its batch).
 void ensure_lane_guided(tr_ctx* x, int k, uint32_t capacity) {
     if (x->lane_vrec_cap[k] >= capacity && x->lane_vrec[k]) return;
-    if (x->lane_vrec[k]) {
-        cudaFree(x->lane_vrec[k]);
-        x->allocs.erase(std::remove(x->allocs.begin(), x->allocs.end(), (void*)x->lane_vrec[k]), x->allocs.end());
-        x->lane_vrec[k] = nullptr;
-        x->lane_vrec_cap[k] = 0;
-    }
+    x->drop(x->lane_vrec[k]);
+    x->lane_vrec_cap[k] = 0;
     x->lane_vrec[k] = x->alloc<uint4>((size_t)capacity * 5);
     x->lane_vrec_cap[k] = capacity;
 }
 
 void ensure_guided(tr_ctx* x, uint32_t capacity) {
     if (x->gw_capacity >= capacity && x->gw.pool_cap == x->guide_pool && x->pool_state && x->pool_alt.state) return;
-    auto drop = [&](void* p) {
-        if (!p) return;
-        cudaFree(p);
-        x->allocs.erase(std::remove(x->allocs.begin(), x->allocs.end(), p), x->allocs.end());
-    };
     trk::GuideWave& g = x->gw;
     tr_ctx::PoolBuf& a = x->pool_alt;
-    drop(g.vrec); drop(g.pool_feat); drop(g.pool_dir); drop(g.pool_w); drop(g.pool_meta);
-    drop(a.feat); drop(a.dir); drop(a.w); drop(a.meta);
-    g.vrec = g.pool_feat = g.pool_meta = a.feat = a.meta = nullptr;
-    g.pool_dir = g.pool_w = a.dir = a.w = nullptr;
+    x->drop(g.vrec); x->drop(g.pool_feat); x->drop(g.pool_dir); x->drop(g.pool_w); x->drop(g.pool_meta);
+    x->drop(a.feat); x->drop(a.dir); x->drop(a.w); x->drop(a.meta);
     x->gw_capacity = 0;                  // until the new buffers are there
     g.vrec = x->alloc<uint4>((size_t)capacity * 5);
     const uint32_t pc = std::max<uint32_t>(1u, x->guide_pool);
@@ -485,8 +459,7 @@ tr_status render_region(tr_ctx* x, uint32_t x0, uint32_t y0, uint32_t x1, uint32
             buffers((uint32_t)lanes_of());
         } catch (const CudaError& e) {
             if (e.code != cudaErrorMemoryAllocation) throw;
-            cudaGetLastError();                 // no room for them: give back what was taken, small batches
-            drop_waves(x);
+            drop_waves(x);                      // no room for them: give back what was taken, small batches
             large = 1;
             cap = small_cap;
             max_lanes = kWaveLanes;
@@ -860,7 +833,6 @@ tr_status tr_create(const tr_scene* s, const tr_camera* c, const tr_film* f, con
         const std::string too_big = "streak film of " + std::to_string(nstreak * 8 >> 20) +
                                     " MiB does not fit in free device memory";
         auto refuse_film = [&] {
-            cudaGetLastError();
             cudaStreamSynchronize(x->stream);
             x->release();
             delete x;
@@ -1307,12 +1279,8 @@ tr_status tr_trace_rays(tr_ctx* x, const float* rays, uint32_t n, int any_hit, t
     try {
         TR_CUDA(cudaSetDevice(x->device));
         if (x->ray_cap < n) {
-            auto drop = [&](void* p) {
-                if (!p) return;
-                cudaFree(p);
-                x->allocs.erase(std::remove(x->allocs.begin(), x->allocs.end(), p), x->allocs.end());
-            };
-            drop(x->d_rays); drop(x->d_hits);
+            x->ray_cap = 0;
+            x->drop(x->d_rays); x->drop(x->d_hits);
             x->d_rays = x->alloc<float>((size_t)n * 8);
             x->d_hits = x->alloc<tr_hit>(n);
             x->ray_cap = n;

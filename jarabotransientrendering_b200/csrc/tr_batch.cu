@@ -73,10 +73,13 @@ struct tr_batch {
         allocs.push_back(p);
         return p;
     }
-    void drop(void* p) {
+    // gives p's memory back and forgets the address
+    template <class T>
+    void drop(T*& p) {
         if (!p) return;
         cudaFree(p);
-        allocs.erase(std::remove(allocs.begin(), allocs.end(), p), allocs.end());
+        allocs.erase(std::remove(allocs.begin(), allocs.end(), (void*)p), allocs.end());
+        p = nullptr;
     }
     void drop_graph() {
         if (exec) cudaGraphExecDestroy(exec);
@@ -178,12 +181,11 @@ void ensure_batch_wave(tr_batch* b, uint32_t capacity) {
 // one lane's wave buffers; `stats` null: allocate the statistics counters, else share them
 void ensure_lane(tr_batch* b, trk::Wave& w, uint32_t capacity, unsigned long long* stats) {
     b->drop(w.block);
-    w.block = nullptr;
     w.capacity = 0;
     const size_t R = std::max<uint32_t>(1u, b->max_bounces);
     bool tsm = false;
     for (tr_ctx* x : b->ctx) tsm = tsm || (x->integ.flags & TR_FLAG_TIME_SAMPLING) != 0;
-    void* block = b->alloc<unsigned char>(carve_wave(nullptr, nullptr, capacity, R, tsm));
+    w.block = b->alloc<unsigned char>(carve_wave(nullptr, nullptr, capacity, R, tsm));
     if (!w.counters) w.counters = b->alloc<uint32_t>(trk::kCounters);
     if (stats) {
         w.stats = stats;
@@ -191,13 +193,14 @@ void ensure_lane(tr_batch* b, trk::Wave& w, uint32_t capacity, unsigned long lon
         w.stats = b->alloc<unsigned long long>(8);
         TR_CUDA(cudaMemsetAsync(w.stats, 0, 8 * sizeof(unsigned long long), b->stream));
     }
-    carve_wave(&w, block, capacity, R, tsm);
+    carve_wave(&w, w.block, capacity, R, tsm);
 }
 
 void ensure_batch_guided(tr_batch* b, uint32_t capacity) {
     if (b->gw_capacity == capacity && b->gw.pool_cap == b->pool && b->pool_state) return;
     b->drop_graph();
     trk::GuideWave& g = b->gw;
+    b->gw_capacity = 0;                  // until the new buffers are there
     b->drop(g.vrec); b->drop(g.pool_feat); b->drop(g.pool_dir); b->drop(g.pool_w); b->drop(g.pool_meta);
     g.vrec = b->alloc<uint4>((size_t)capacity * 5);
     for (uint4*& v : b->lane_vrec) {
@@ -302,8 +305,9 @@ tr_status batch_render(tr_batch* b, const uint64_t* s_begin, const uint32_t* s_c
     if (pl.batches.size() > b->batches_cap) {
         b->drop_graph();
         b->drop(b->d_batches);
+        b->batches_cap = 0;
+        b->d_batches = b->alloc<trk::BatchDesc>(pl.batches.size() * 2);
         b->batches_cap = (uint32_t)pl.batches.size() * 2;
-        b->d_batches = b->alloc<trk::BatchDesc>(b->batches_cap);
     }
     TR_CUDA(cudaMemcpyAsync(b->d_batches, pl.batches.data(), pl.batches.size() * sizeof(trk::BatchDesc),
                             cudaMemcpyHostToDevice, s));

@@ -124,8 +124,9 @@ struct tr_ctx {
     int device = 0;
     cudaStream_t stream = nullptr;
     cudaEvent_t ev0 = nullptr, ev1 = nullptr;
-    size_t bytes = 0;
-    std::vector<void*> allocs;
+    size_t bytes = 0;                       // device memory held
+    struct Alloc { void* p; size_t bytes; };
+    std::vector<Alloc> allocs;
 
     // scene
     float4* d_nodes = nullptr;
@@ -222,9 +223,22 @@ struct tr_ctx {
 
     template <class T>
     T* alloc(size_t n) {
+        const size_t before = bytes;
         T* p = tri::dalloc<T>(n, bytes);
-        allocs.push_back(p);
+        allocs.push_back({p, bytes - before});
         return p;
+    }
+    // gives p's memory back and forgets the address, so that it is never freed or used again
+    template <class T>
+    void drop(T*& p) {
+        if (!p) return;
+        const auto it = std::find_if(allocs.begin(), allocs.end(), [&](const Alloc& a) { return a.p == p; });
+        if (it != allocs.end()) {
+            cudaFree(p);
+            bytes -= it->bytes;
+            allocs.erase(it);
+        }
+        p = nullptr;
     }
     void release() {
         if (ev_snap) { cudaEventDestroy(ev_snap); ev_snap = nullptr; }
@@ -245,7 +259,7 @@ struct tr_ctx {
         }
         if (light_stream) cudaStreamDestroy(light_stream);
         shadow_stream = light_stream = nullptr;
-        for (void* p : allocs) cudaFree(p);
+        for (const Alloc& a : allocs) cudaFree(a.p);
         allocs.clear();
         if (ev0) cudaEventDestroy(ev0);
         if (ev1) cudaEventDestroy(ev1);

@@ -2,6 +2,7 @@
 fit or are no longer needed."""
 import contextlib
 
+import numpy as np
 import pytest
 
 from jarabotransientrendering_b200 import _abi, scenes as S
@@ -43,3 +44,51 @@ def test_render_after_a_failed_one(gpu):
                 ctx.render(1, 15)
         ctx.render(1, 15)
         assert (ctx.film()["weight"] == 16).all()
+
+
+def _bidirectional():
+    sc = S.cornell(width=256, height=256, time_bins=16, exposure=0.4, max_bounces=16, sqrt_spp=4)     # 1 M paths
+    sc.flags |= S.FLAG_TIME_SAMPLING | S.FLAG_BIDIRECTIONAL
+    return sc
+
+
+def _connections(gpu, spare):
+    """The film and counters of ``_bidirectional``, rendered with ``spare`` bytes of device memory to take (0: all)."""
+    with gpu.Context(_bidirectional()) as ctx:
+        with _only(spare) if spare else contextlib.nullcontext():
+            ctx.render(0, 16)
+        return ctx.film(), ctx.stats()
+
+
+def test_connections_with_room_for_one_queue(gpu):
+    """Light subpaths set up the next depth's connections while this one's are traced where two queues fit, one
+    after the other where one fits, also when it is the record flags that do not: the same film and rays."""
+    full, cf = _connections(gpu, 0)
+    with gpu.Context(_bidirectional()) as ctx:
+        base = ctx.stats()["device_bytes"]
+    queue = 15 * 3 * 16 << 20                                # 15 rays of 48 bytes in each of 1 M slots
+    flags = (16 + 120) << 20                                 # one per record
+    for spare in (cf["device_bytes"] - base - queue // 2, cf["device_bytes"] - base - flags // 2):
+        one, co = _connections(gpu, spare)
+        assert co["device_bytes"] == cf["device_bytes"] - queue
+        for k in ("paths", "closest_rays", "shadow_rays", "splats"):
+            assert co[k] == cf[k]
+        for k in full:
+            assert np.allclose(one[k], full[k], rtol=1e-12, atol=0.0), k
+
+
+def test_context_renders_after_running_out_of_memory(gpu):
+    """A render that found no memory leaves its context as it was: nothing of it stays held, and with memory
+    there again the same context renders the same film."""
+    full, cf = _connections(gpu, 0)
+    with gpu.Context(_bidirectional()) as ctx:
+        for share in (0.2, 0.5, 0.8):                        # of what the render takes with one queue
+            with _only(share * (cf["device_bytes"] - (720 << 20))):
+                with pytest.raises(gpu.TransientError, match="memory"):
+                    ctx.render(0, 16)
+                assert ctx.stats()["device_bytes"] < 256 * MB
+        ctx.render(0, 16)
+        f, c = ctx.film(), ctx.stats()
+    assert c["device_bytes"] == cf["device_bytes"] and c["shadow_rays"] == cf["shadow_rays"]
+    for k in full:
+        assert np.allclose(f[k], full[k], rtol=1e-12, atol=0.0), k
