@@ -319,31 +319,40 @@ void ensure_lane_guided(tr_ctx* x, int k, uint32_t capacity) {
     x->lane_vrec_cap[k] = capacity;
 }
 
-void ensure_guided(tr_ctx* x, uint32_t capacity) {
-    if (x->gw_capacity >= capacity && x->gw.pool_cap == x->guide_pool && x->pool_state && x->pool_alt.state) return;
+// The training pools and the network's snapshot.  Their size is the caller's, whatever a render's batches
+// are, so the samples a render leaves for the next one's training stay when that one's batches are larger.
+void ensure_guide_pools(tr_ctx* x) {
     trk::GuideWave& g = x->gw;
     tr_ctx::PoolBuf& a = x->pool_alt;
-    x->drop(g.vrec); x->drop(g.pool_feat); x->drop(g.pool_dir); x->drop(g.pool_w); x->drop(g.pool_meta);
-    x->drop(a.feat); x->drop(a.dir); x->drop(a.w); x->drop(a.meta);
-    x->gw_capacity = 0;                  // until the new buffers are there
-    g.vrec = x->alloc<uint4>((size_t)capacity * 5);
-    const uint32_t pc = std::max<uint32_t>(1u, x->guide_pool);
-    g.pool_feat = x->alloc<uint4>((size_t)pc * 8);
-    g.pool_dir = x->alloc<float>((size_t)pc * 3);
-    g.pool_w = x->alloc<float>(pc);
-    g.pool_meta = x->alloc<uint4>(pc);
-    a.feat = x->alloc<uint4>((size_t)pc * 8);
-    a.dir = x->alloc<float>((size_t)pc * 3);
-    a.w = x->alloc<float>(pc);
-    a.meta = x->alloc<uint4>(pc);
-    g.pool_cap = x->guide_pool;
+    if (g.pool_cap != x->guide_pool || !a.meta) {
+        x->pool_pending = 0;             // a reallocated pool holds nothing to train on
+        x->drop(g.pool_feat); x->drop(g.pool_dir); x->drop(g.pool_w); x->drop(g.pool_meta);
+        x->drop(a.feat); x->drop(a.dir); x->drop(a.w); x->drop(a.meta);
+        const uint32_t pc = std::max<uint32_t>(1u, x->guide_pool);
+        g.pool_feat = x->alloc<uint4>((size_t)pc * 8);
+        g.pool_dir = x->alloc<float>((size_t)pc * 3);
+        g.pool_w = x->alloc<float>(pc);
+        g.pool_meta = x->alloc<uint4>(pc);
+        a.feat = x->alloc<uint4>((size_t)pc * 8);
+        a.dir = x->alloc<float>((size_t)pc * 3);
+        a.w = x->alloc<float>(pc);
+        a.meta = x->alloc<uint4>(pc);
+        g.pool_cap = x->guide_pool;
+    }
     if (!x->pool_state) x->pool_state = x->alloc<uint32_t>(2);
     if (!a.state) a.state = x->alloc<uint32_t>(2);
     if (!x->w_snap) x->w_snap = x->alloc<uint4>(4 * 8192 / 16);
     if (!x->bias_snap) x->bias_snap = x->alloc<float>(4 * 64);
     if (!x->ev_snap) TR_CUDA(cudaEventCreateWithFlags(&x->ev_snap, cudaEventDisableTiming));
     if (!x->ev_train) TR_CUDA(cudaEventCreateWithFlags(&x->ev_train, cudaEventDisableTiming));
-    x->pool_pending = 0;                 // a reallocated pool holds nothing to train on
+}
+
+// The first lane's guided-vertex records.
+void ensure_guided(tr_ctx* x, uint32_t capacity) {
+    if (x->gw_capacity >= capacity) return;
+    x->drop(x->gw.vrec);
+    x->gw_capacity = 0;
+    x->gw.vrec = x->alloc<uint4>((size_t)capacity * 5);
     x->gw_capacity = capacity;
 }
 
@@ -440,7 +449,10 @@ tr_status render_region(tr_ctx* x, uint32_t x0, uint32_t y0, uint32_t x1, uint32
     const uint32_t small_cap = cap;
     auto buffers = [&](uint32_t n_lanes) {
         ensure_wave(x, cap);
-        if (guided) ensure_guided(x, cap);
+        if (guided) {
+            ensure_guide_pools(x);
+            ensure_guided(x, cap);
+        }
         for (uint32_t k = 0; k + 1 < n_lanes; ++k) {
             ensure_lane_wave(x, (int)k, cap);
             if (guided) ensure_lane_guided(x, (int)k, cap);
@@ -1737,7 +1749,7 @@ extern "C" tr_status tr_set_guide(tr_ctx* x, tr_guide* g, float mix_prob, float 
     x->guide = g;
     x->guide_mix = mix_prob;
     x->guide_lr = lr;
-    x->guide_pool = train_pool;     // ensure_guided reallocates the pool when its size changes
+    x->guide_pool = train_pool;     // ensure_guide_pools reallocates the pools when their size changes
     x->pool_pending = 0;            // samples collected for another guide are not trained on
     return TR_OK;
 }

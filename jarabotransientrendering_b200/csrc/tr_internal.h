@@ -280,6 +280,7 @@ void ensure_wave(tr_ctx* x, uint32_t capacity);
 void drop_waves(tr_ctx* x);
 void ensure_lane_wave(tr_ctx* x, int k, uint32_t capacity);
 void ensure_lane_guided(tr_ctx* x, int k, uint32_t capacity);
+void ensure_guide_pools(tr_ctx* x);
 void ensure_guided(tr_ctx* x, uint32_t capacity);
 trk::Params make_params(tr_ctx* x);
 trg::GuideDev guide_dev(tr_guide* g);

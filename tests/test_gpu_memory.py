@@ -5,7 +5,7 @@ import contextlib
 import numpy as np
 import pytest
 
-from jarabotransientrendering_b200 import _abi, scenes as S
+from jarabotransientrendering_b200 import _abi, renderer as R, scenes as S
 
 pytestmark = pytest.mark.gpu
 
@@ -92,3 +92,22 @@ def test_context_renders_after_running_out_of_memory(gpu):
     assert c["device_bytes"] == cf["device_bytes"] and c["shadow_rays"] == cf["shadow_rays"]
     for k in full:
         assert np.allclose(f[k], full[k], rtol=1e-12, atol=0.0), k
+
+
+# from one batch of half a million slots to one of two million; to the large batches of at least 8.4 M paths
+@pytest.mark.parametrize("first,second", [(2, 8), (8, 32)])
+def test_pending_training_samples_survive_larger_batches(gpu, first, second):
+    """The samples a guided pass collected train the proposal during the next pass, of whatever size."""
+    sc = S.guided(width=512, height=512, time_bins=8, exposure=0.64, sqrt_spp=8, max_bounces=3)
+    sc.flags = S.FLAG_ORTHONORMAL_FRAME
+    g = R.Guide(device=0, seed=1)
+    try:
+        with gpu.Context(sc) as ctx:
+            ctx.set_guide(g, mix_prob=0.5, learning_rate=1e-3, train_pool=16384)
+            ctx.render(0, first)
+            before = g.params()
+            ctx.render(first, second)
+            assert ctx.stats()["train_steps"] == 1
+            assert (g.params() != before).any()
+    finally:
+        g.close()
