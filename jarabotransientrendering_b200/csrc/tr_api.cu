@@ -422,6 +422,21 @@ tr_status render_region(tr_ctx* x, uint32_t x0, uint32_t y0, uint32_t x1, uint32
     cap = std::max<uint32_t>(cap, ninc);
     const bool guided = x->guide != nullptr;
     const bool bidir = (x->integ.flags & TR_FLAG_BIDIRECTIONAL) != 0;
+    const uint32_t T = x->film.time_bins;
+    const bool f32 = sink && sink->type == TR_FILM_F32;
+    const bool rgbe = sink && sink->type == TR_FILM_RGBE;
+    // what the render needs beside its batches comes first, so that batches larger than they have to be
+    // never take its memory.  RGBE: the images of the whole film in device memory (a third of the FP32
+    // bytes), so each batch is encoded on its own lane right after its splat and the copy stream only copies
+    const size_t cells = (size_t)x->film.width * x->film.height * ((size_t)T + 1u);
+    if (rgbe && x->rgbe_cells < cells) {
+        x->d_rgbe = x->alloc<uchar4>(cells);
+        x->rgbe_cells = cells;
+    }
+    if (guided) {
+        ensure_guide_pools(x);
+        if (x->guide_lr > 0.0f && x->pool_pending >= kTrainLeast) x->guide->ensure(std::min(x->pool_pending, kTrainBatch));
+    }
     // small renders: whole paths in one launch (per-kernel times need the kernels apart)
     const bool whole = trk::paths_fit(total_slots, x->bvh_depth) && !guided && !bidir && !x->profiling;
     // samples per pixel per batch, pixels per batch and the lanes that take the batches in turn
@@ -449,10 +464,7 @@ tr_status render_region(tr_ctx* x, uint32_t x0, uint32_t y0, uint32_t x1, uint32
     const uint32_t small_cap = cap;
     auto buffers = [&](uint32_t n_lanes) {
         ensure_wave(x, cap);
-        if (guided) {
-            ensure_guide_pools(x);
-            ensure_guided(x, cap);
-        }
+        if (guided) ensure_guided(x, cap);
         for (uint32_t k = 0; k + 1 < n_lanes; ++k) {
             ensure_lane_wave(x, (int)k, cap);
             if (guided) ensure_lane_guided(x, (int)k, cap);
@@ -534,9 +546,6 @@ tr_status render_region(tr_ctx* x, uint32_t x0, uint32_t y0, uint32_t x1, uint32
     // film streaming: once a pixel batch of the last sample chunk is splatted its film rows are
     // final; the copy stream waits for that point and copies them (FP32: converted on the
     // device first, into a staging buffer the copy stream reuses in order)
-    const uint32_t T = x->film.time_bins;
-    const bool f32 = sink && sink->type == TR_FILM_F32;
-    const bool rgbe = sink && sink->type == TR_FILM_RGBE;
     if (sink) {
         if (!x->copy_stream) {
             // highest priority: its FP32 conversions get SMs as soon as a traversal launch's
@@ -553,13 +562,6 @@ tr_status render_region(tr_ctx* x, uint32_t x0, uint32_t y0, uint32_t x1, uint32
         if (f32 && x->stage_floats < stage) {
             x->d_stage = x->alloc<float>(stage);
             x->stage_floats = stage;
-        }
-        // RGBE: the images of the whole film in device memory (a third of the FP32 bytes), so each
-        // batch is encoded on its own lane right after its splat and the copy stream only copies
-        const size_t cells = (size_t)x->film.width * x->film.height * ((size_t)T + 1u);
-        if (rgbe && x->rgbe_cells < cells) {
-            x->d_rgbe = x->alloc<uchar4>(cells);
-            x->rgbe_cells = cells;
         }
     }
     // Wave lanes: with more than one pixel batch and each pixel in one batch only (a single
@@ -1661,10 +1663,9 @@ tr_status train_on_pool(tr_guide* g, const trk::GuideWave& gw, const uint32_t* p
     if (e) return guide_check_err(g, s);
     // ... the training steps are enqueued back to back, and one more for their status and loss
     const uint32_t n = std::min(fill, pool);
-    const uint32_t batch = 65536;
     try {
-        for (uint32_t off = 0; off + 1024 <= n; off += batch) {
-            const uint32_t m = std::min(batch, n - off);
+        for (uint32_t off = 0; off + kTrainLeast <= n; off += kTrainBatch) {
+            const uint32_t m = std::min(kTrainBatch, n - off);
             train_enqueue(g, gw.pool_feat + (size_t)off * 8, gw.pool_dir + (size_t)off * 3, gw.pool_w + off, m, lr, s);
             stats.train_steps += 1;
         }
@@ -1693,10 +1694,10 @@ tr_status guide_begin_render(tr_ctx* x, cudaStream_t s) {
         // training on the previous render's pool runs on the guide's stream, after the snapshot
         TR_CUDA(cudaEventRecord(x->ev_snap, s));
         TR_CUDA(cudaStreamWaitEvent(g->stream, x->ev_snap, 0));
-        const uint32_t n = x->pool_pending, batch = 65536;
+        const uint32_t n = x->pool_pending;
         const tr_ctx::PoolBuf& a = x->pool_alt;
-        for (uint32_t off = 0; off + 1024 <= n; off += batch) {
-            const uint32_t m = std::min(batch, n - off);
+        for (uint32_t off = 0; off + kTrainLeast <= n; off += kTrainBatch) {
+            const uint32_t m = std::min(kTrainBatch, n - off);
             train_enqueue(g, a.feat + (size_t)off * 8, a.dir + (size_t)off * 3, a.w + off, m, x->guide_lr, g->stream);
             x->stats.train_steps += 1;
         }

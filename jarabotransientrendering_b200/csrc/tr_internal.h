@@ -66,6 +66,7 @@ constexpr size_t kLargeWaveBytes = (size_t)6 << 30;  // path state a large rende
 constexpr int kWaveLanes = TR_WAVE_LANES;        // wave buffer sets batches alternate between
 // default roughness below which GGX vertices sample their BSDF instead of the learned proposal
 constexpr float kGuideMinAlpha = 0.5f;
+constexpr uint32_t kTrainBatch = 65536, kTrainLeast = 1024;     // samples of a training step: at most, at least
 
 }  // namespace tri
 

@@ -111,3 +111,16 @@ def test_pending_training_samples_survive_larger_batches(gpu, first, second):
             assert (g.params() != before).any()
     finally:
         g.close()
+
+
+def test_rgbe_images_do_not_cost_a_large_render_its_fallback(gpu):
+    """A frame whose large batches fit but not beside its RGBE images takes the small ones."""
+    sc = S.cornell(width=512, height=512, time_bins=1023, exposure=0.005, max_bounces=3, sqrt_spp=8)
+    steady = np.zeros((512, 512, 4), np.uint8)
+    with gpu.Context(sc) as ctx:
+        ctx.render(0, 1)
+        # three batches of 4 M slots take 2.2 GB, the images 1.1 GB, four batches of 2 M slots 1.5 GB
+        with _only(2850 * MB):
+            ctx.render_film(1, 63, steady=steady)
+        f = ctx.film(streak=False)
+    assert (f["weight"] == 64).all() and steady.any()
