@@ -150,6 +150,13 @@ size_t pool_idle_bytes(int device) {
     return reserved > used ? (size_t)(reserved - used) : 0;
 }
 
+void dfree(const std::vector<void*>& blocks) {
+    cudaDeviceSynchronize();
+    for (void* p : blocks)
+        if (p) cudaFreeAsync(p, 0);
+    cudaStreamSynchronize(0);                    // back in the pool, for every stream
+}
+
 size_t carve_wave(trk::Wave* w, void* block, uint32_t capacity, size_t R, bool time_sampling) {
     size_t at = 0;
     trk::Wave dummy{};
@@ -1536,7 +1543,7 @@ extern "C" tr_status tr_guide_create(int device, uint64_t seed, tr_guide** out) 
         TR_CUDA(trg::pack_weights(g->params, g->w_fwd, g->w_bwd, g->stream));
         TR_CUDA(cudaStreamSynchronize(g->stream));
     } catch (const CudaError& e) {
-        for (void* q : g->allocs) cudaFree(q);
+        dfree(g->allocs);
         delete g;
         return fail(TR_ERR_CUDA, e.what());
     }
@@ -1640,7 +1647,7 @@ extern "C" tr_status tr_guide_destroy(tr_guide* g) {
     if (!g) return TR_OK;
     cudaSetDevice(g->device);
     if (g->stream) cudaStreamSynchronize(g->stream);
-    for (void* q : g->allocs) cudaFree(q);
+    dfree(g->allocs);
     if (g->stream) cudaStreamDestroy(g->stream);
     delete g;
     return TR_OK;

@@ -37,8 +37,7 @@ struct CudaError : std::runtime_error {
 // Device memory of contexts, guides and batches comes from one stream-ordered pool per device
 // that keeps freed memory for the next allocations (release threshold unlimited), so creating
 // and destroying contexts does not map and unmap gigabytes each time; memory goes back to the
-// driver only through tr_release_cached_memory or at exit.  Frees stay cudaFree (which waits
-// for the device and returns the block to its pool).
+// driver only through tr_release_cached_memory or at exit.
 cudaMemPool_t device_pool(int device);
 // pool memory of `device` reserved but not in use (free for the next allocations)
 size_t pool_idle_bytes(int device);
@@ -55,6 +54,12 @@ T* dalloc(size_t count, size_t& total) {
     total += count * sizeof(T);
     return static_cast<T*>(p);
 }
+
+// Gives memory of the current device back to its pool once the device is idle (any stream may have used it).
+// In stream order, not by cudaFree: what that returns the pool can hand out again but goes on counting as used,
+// and pool_idle_bytes would miss it.
+void dfree(const std::vector<void*>& blocks);
+inline void dfree(void* p) { dfree(std::vector<void*>{p}); }
 
 constexpr uint32_t kMaxBounces = 63;            // counters hold 64 depths
 constexpr uint32_t kDefaultCapacity = 1u << 21; // path slots per wavefront batch
@@ -100,7 +105,7 @@ struct tr_guide {
     }
     void drop(void* p) {
         if (!p) return;
-        cudaFree(p);
+        tri::dfree(p);
         allocs.erase(std::remove(allocs.begin(), allocs.end(), p), allocs.end());
     }
     trg::GuideDev dev() const {
@@ -235,7 +240,7 @@ struct tr_ctx {
         if (!p) return;
         const auto it = std::find_if(allocs.begin(), allocs.end(), [&](const Alloc& a) { return a.p == p; });
         if (it != allocs.end()) {
-            cudaFree(p);
+            tri::dfree(p);
             bytes -= it->bytes;
             allocs.erase(it);
         }
@@ -260,7 +265,9 @@ struct tr_ctx {
         }
         if (light_stream) cudaStreamDestroy(light_stream);
         shadow_stream = light_stream = nullptr;
-        for (const Alloc& a : allocs) cudaFree(a.p);
+        std::vector<void*> blocks;
+        for (const Alloc& a : allocs) blocks.push_back(a.p);
+        tri::dfree(blocks);
         allocs.clear();
         if (ev0) cudaEventDestroy(ev0);
         if (ev1) cudaEventDestroy(ev1);

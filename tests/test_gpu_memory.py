@@ -124,3 +124,16 @@ def test_rgbe_images_do_not_cost_a_large_render_its_fallback(gpu):
             ctx.render_film(1, 63, steady=steady)
         f = ctx.film(streak=False)
     assert (f["weight"] == 64).all() and steady.any()
+
+
+def test_freed_memory_counts_as_free(gpu):
+    """What destroyed contexts left in the library's pool counts as free memory for the next one."""
+    def scene(bins):
+        return S.cornell(width=256, height=256, time_bins=bins, exposure=0.01, sqrt_spp=1, max_bounces=2)
+    _abi.check(_abi.lib().tr_release_cached_memory(0))
+    gpu.Context(scene(2040)).close()                         # 3.2 GB
+    with _only(1000 * MB, release=False):
+        before = _free()
+        for _ in range(3):                                   # 1.1 GB of the 3.2, of which 2.1 and 1.0 beside are left
+            gpu.Context(scene(680)).close()
+        assert abs(_free() - before) < 64 * MB
