@@ -179,14 +179,14 @@ size_t carve_wave(trk::Wave* w, void* block, uint32_t capacity, size_t R, bool t
 }
 
 // Gives the first wave's path state back to the pool, the light subpaths' and connections' with it.
-static void drop_first_wave(tr_ctx* x) {
+static void drop_first_wave(tr_ctx* x, cudaStream_t after = nullptr) {
+    auto drop = [&](auto*&... p) { (x->drop(p, after), ...); };
     trk::Wave& lw = x->lwave;
     trk::BidirWave& bd = x->bd;
-    x->drop(x->wave.block);
-    x->wave.capacity = 0;
-    x->drop(lw.ray_o); x->drop(lw.ray_d); x->drop(lw.thr); x->drop(lw.rng); x->drop(lw.hit); x->drop(lw.q[0]); x->drop(lw.q[1]);
-    x->drop(bd.lvert); x->drop(bd.evert); x->drop(bd.nl); x->drop(bd.ne); x->drop(bd.L0);
-    x->drop(bd.co_o); x->drop(bd.co_d); x->drop(bd.co_L); x->drop(bd.valid);
+    drop(x->wave.block, x->gw.vrec);
+    x->wave.capacity = x->gw_capacity = 0;
+    drop(lw.ray_o, lw.ray_d, lw.thr, lw.rng, lw.hit, lw.q[0], lw.q[1]);
+    drop(bd.lvert, bd.evert, bd.nl, bd.ne, bd.L0, bd.co_o, bd.co_d, bd.co_L, bd.valid);
 }
 
 void ensure_wave(tr_ctx* x, uint32_t capacity) {
@@ -291,12 +291,12 @@ void prof_publish(tr_ctx* x) {
 }
 
 // Gives the path state of all lanes back to the pool (its contents are only scratch between calls).
-void drop_waves(tr_ctx* x) {
-    drop_first_wave(x);
+void drop_waves(tr_ctx* x, cudaStream_t after) {
+    drop_first_wave(x, after);
     for (int k = 0; k + 1 < kWaveLanes; ++k) {
-        x->drop(x->lane_wave[k].block);
+        x->drop(x->lane_wave[k].block, after);
         x->lane_wave[k].capacity = 0;
-        x->drop(x->lane_vrec[k]);
+        x->drop(x->lane_vrec[k], after);
         x->lane_vrec_cap[k] = 0;
     }
 }
@@ -485,16 +485,31 @@ tr_status render_region(tr_ctx* x, uint32_t x0, uint32_t y0, uint32_t x1, uint32
         return (int)std::min<uint64_t>((uint64_t)max_lanes, (win_pix + ppb - 1) / ppb);
     };
     if (large > 1) {
+        // they may take what the pool holds, and of the rest what leaves a new context its share (the query
+        // takes 0.2 ms: asked only where the pool is short of them)
         cap = unit * large * ns_chunk * ninc;
+        const size_t need = (size_t)lanes_of() *
+            (carve_wave(nullptr, nullptr, cap, std::max<uint32_t>(1u, x->integ.max_bounces),
+                        (x->integ.flags & TR_FLAG_TIME_SAMPLING) != 0) + (guided ? (size_t)cap * 5 * sizeof(uint4) : 0));
+        size_t room = pool_idle_bytes(x->device), free_b = 0, total_b = 0;
+        if (room < need) {
+            TR_CUDA(cudaMemGetInfo(&free_b, &total_b));
+            room += free_b;
+            if (room < need + kLeastFree) large = 1;
+        }
+    }
+    if (large > 1) {
         try {
             buffers((uint32_t)lanes_of());
         } catch (const CudaError& e) {
             if (e.code != cudaErrorMemoryAllocation) throw;
             drop_waves(x);                      // no room for them: give back what was taken, small batches
             large = 1;
-            cap = small_cap;
-            max_lanes = kWaveLanes;
         }
+    }
+    if (large == 1 && cap != small_cap) {
+        cap = small_cap;
+        max_lanes = kWaveLanes;
     }
     const int lanes = lanes_of();
     if (large == 1) buffers((uint32_t)lanes);
@@ -788,6 +803,12 @@ tr_status render_region(tr_ctx* x, uint32_t x0, uint32_t y0, uint32_t x1, uint32
     x->stats.paths += total_slots;
     x->stats.camera_samples += win_pix * ns_total;
     x->stats.render_ms = ms;
+    if (large > 1) {
+        // large batches are the pool's again between calls (small ones stay): contexts that render in turn
+        // share them, and a context made meanwhile finds their memory
+        drop_waves(x, strm);
+        TR_CUDA(cudaStreamSynchronize(strm));
+    }
     if (guided) return guide_end_render(x, strm);
     return TR_OK;
 }
@@ -912,7 +933,7 @@ tr_status tr_create(const tr_scene* s, const tr_camera* c, const tr_film* f, con
         size_t free_b = 0, total_b = 0;
         cudaMemGetInfo(&free_b, &total_b);
         free_b += tri::pool_idle_bytes(device);      // kept by the pool for reuse
-        if (free_b < ((size_t)2 << 30)) return refuse_film();
+        if (free_b < kLeastFree) return refuse_film();
 
         // BVH (replaces World::freeze -> rtcCommit): built on the device from the uploaded arrays,
         // nodes and leaf order left there; the host builder takes one-leaf scenes and names the

@@ -65,6 +65,7 @@ constexpr uint32_t kMaxBounces = 63;            // counters hold 64 depths
 constexpr uint32_t kDefaultCapacity = 1u << 21; // path slots per wavefront batch
 constexpr uint32_t kLargeCapacity = 1u << 23;   // of a large render's (render_region)
 constexpr size_t kLargeWaveBytes = (size_t)6 << 30;  // path state a large render's batches may take
+constexpr size_t kLeastFree = (size_t)2 << 30;  // device memory left for a new context's path state
 #ifndef TR_WAVE_LANES
 #define TR_WAVE_LANES 4
 #endif
@@ -234,13 +235,14 @@ struct tr_ctx {
         allocs.push_back({p, bytes - before});
         return p;
     }
-    // gives p's memory back and forgets the address, so that it is never freed or used again
+    // gives p's memory back and forgets the address, so that it is never freed or used again: in the order of
+    // the stream `after`, or at once, which waits for the device
     template <class T>
-    void drop(T*& p) {
+    void drop(T*& p, cudaStream_t after = nullptr) {
         if (!p) return;
         const auto it = std::find_if(allocs.begin(), allocs.end(), [&](const Alloc& a) { return a.p == p; });
         if (it != allocs.end()) {
-            tri::dfree(p);
+            if (!after || cudaFreeAsync(p, after) != cudaSuccess) tri::dfree(p);
             bytes -= it->bytes;
             allocs.erase(it);
         }
@@ -285,7 +287,7 @@ namespace tri {
 // pool allocation instead of fourteen): with w null the bytes it takes, else w's pointers into it.
 size_t carve_wave(trk::Wave* w, void* block, uint32_t capacity, size_t R, bool time_sampling);
 void ensure_wave(tr_ctx* x, uint32_t capacity);
-void drop_waves(tr_ctx* x);
+void drop_waves(tr_ctx* x, cudaStream_t after = nullptr);
 void ensure_lane_wave(tr_ctx* x, int k, uint32_t capacity);
 void ensure_lane_guided(tr_ctx* x, int k, uint32_t capacity);
 void ensure_guide_pools(tr_ctx* x);

@@ -137,3 +137,21 @@ def test_freed_memory_counts_as_free(gpu):
         for _ in range(3):                                   # 1.1 GB of the 3.2, of which 2.1 and 1.0 beside are left
             gpu.Context(scene(680)).close()
         assert abs(_free() - before) < 64 * MB
+def test_large_batches_are_given_back(gpu):
+    """Between its calls a context holds no more than small batches take, however large its renders were,
+    and contexts that render in turn share the memory of the large ones."""
+    sc = S.cornell(width=512, height=512, time_bins=8, exposure=0.64, max_bounces=6, sqrt_spp=8)
+    _abi.check(_abi.lib().tr_release_cached_memory(0))
+    with gpu.Context(sc) as a, gpu.Context(sc) as b, gpu.Context(sc) as c:
+        a.render(0, 31)                                      # 8.1 M paths: four batches of 2 M slots
+        small = a.stats()["device_bytes"]
+        b.render(0, 64)
+        free1 = _free()
+        assert b.stats()["device_bytes"] <= small
+        c.render(0, 64)
+        assert free1 - _free() < 256 * MB
+        for k in range(1, 4):
+            b.render(64 * k, 64)
+        assert b.stats()["device_bytes"] <= small
+        assert free1 - _free() < 256 * MB
+        assert (b.film()["weight"] == 256).all()
