@@ -150,6 +150,14 @@ size_t pool_idle_bytes(int device) {
     return reserved > used ? (size_t)(reserved - used) : 0;
 }
 
+// Memory kept by the pool goes back to the driver (nothing where there is no pool).
+static void trim_pool(int device) noexcept {
+    try {
+        cudaMemPoolTrimTo(device_pool(device), 0);
+    } catch (const CudaError&) {
+    }
+}
+
 void dfree(const std::vector<void*>& blocks) {
     cudaDeviceSynchronize();
     for (void* p : blocks)
@@ -872,22 +880,28 @@ tr_status tr_create(const tr_scene* s, const tr_camera* c, const tr_film* f, con
         // earlier context is reused whole instead of mapped again)
         const size_t nstreak = (size_t)f->width * f->height * f->time_bins * 3u;
         const size_t nb = f->bounce_films;
-        const std::string too_big = "streak film of " + std::to_string(nstreak * 8 >> 20) +
-                                    " MiB does not fit in free device memory";
+        // Refused unless it leaves the path state its share, before anything is taken.  The query takes
+        // 0.2 ms: left out where the pool alone holds all that, and put off for films below 32 MB (what the
+        // pool grows by anyway) until the scene's uploads are under way.
+        const size_t film_bytes = (1 + nb) * nstreak * sizeof(double);
         auto refuse_film = [&] {
+            const size_t idle = tri::pool_idle_bytes(device);      // kept by the pool for reuse
+            if (idle + x->bytes >= film_bytes + kLeastFree) return false;
+            size_t free_b = 0, total_b = 0;
+            cudaMemGetInfo(&free_b, &total_b);
+            return free_b + idle + x->bytes < film_bytes + kLeastFree;
+        };
+        auto refused = [&] {
             cudaStreamSynchronize(x->stream);
             x->release();
             delete x;
-            cudaMemPoolTrimTo(tri::device_pool(device), 0);     // not kept for a film that was refused
-            return fail(TR_ERR_OUT_OF_MEMORY, too_big);
+            return fail(TR_ERR_OUT_OF_MEMORY, "streak film of " + std::to_string(nstreak * 8 >> 20) +
+                                                  " MiB does not fit in free device memory");
         };
-        try {
-            x->d_streak = x->alloc<double>(nstreak);
-            if (nb) x->d_bstreak = x->alloc<double>(nb * nstreak);
-        } catch (const CudaError& e) {
-            if (e.code != cudaErrorMemoryAllocation) throw;
-            return refuse_film();
-        }
+        const bool check_late = film_bytes < ((size_t)32 << 20);
+        if (!check_late && refuse_film()) return refused();
+        x->d_streak = x->alloc<double>(nstreak);
+        if (nb) x->d_bstreak = x->alloc<double>(nb * nstreak);
         x->d_steady = x->alloc<double>((size_t)f->width * f->height * 3u);
         x->d_weight = x->alloc<double>((size_t)f->width * f->height);
         TR_CUDA(cudaMemsetAsync(x->d_streak, 0, nstreak * sizeof(double), x->stream));
@@ -928,12 +942,7 @@ tr_status tr_create(const tr_scene* s, const tr_camera* c, const tr_film* f, con
         TR_CUDA(cudaMemcpyAsync(d_t, s->triangles, sizeof(uint32_t) * 3 * ntri, cudaMemcpyHostToDevice, x->stream));
         TR_CUDA(cudaMemcpyAsync(d_m, s->triangle_material, sizeof(uint32_t) * ntri, cudaMemcpyHostToDevice, x->stream));
 
-        // 2 GiB have to be left for the path state (asked while the uploads are under way: the query
-        // takes 0.2 ms)
-        size_t free_b = 0, total_b = 0;
-        cudaMemGetInfo(&free_b, &total_b);
-        free_b += tri::pool_idle_bytes(device);      // kept by the pool for reuse
-        if (free_b < kLeastFree) return refuse_film();
+        if (check_late && refuse_film()) return refused();
 
         // BVH (replaces World::freeze -> rtcCommit): built on the device from the uploaded arrays,
         // nodes and leaf order left there; the host builder takes one-leaf scenes and names the
@@ -1073,6 +1082,7 @@ tr_status tr_create(const tr_scene* s, const tr_camera* c, const tr_film* f, con
     } catch (const CudaError& e) {
         x->release();
         delete x;
+        if (e.code == cudaErrorMemoryAllocation) trim_pool(device);     // what it took is not kept for it
         return fail(e.code == cudaErrorMemoryAllocation ? TR_ERR_OUT_OF_MEMORY : TR_ERR_CUDA, e.what());
     } catch (const std::bad_alloc&) {
         x->release();

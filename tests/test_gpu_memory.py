@@ -155,3 +155,19 @@ def test_large_batches_are_given_back(gpu):
         assert b.stats()["device_bytes"] <= small
         assert free1 - _free() < 256 * MB
         assert (b.film()["weight"] == 256).all()
+
+
+def test_refused_film_is_not_taken_first(gpu):
+    """A film that would leave less than 2 GiB is refused before anything is allocated: the memory that
+    destroyed contexts left in the pool stays there."""
+    small = S.cornell(width=256, height=256, time_bins=680, exposure=0.01, sqrt_spp=1, max_bounces=2)    # 1.07 GB
+    big = S.cornell(width=256, height=256, time_bins=1400, exposure=0.01, sqrt_spp=1, max_bounces=2)     # 2.2 GB
+    _abi.check(_abi.lib().tr_release_cached_memory(0))
+    gpu.Context(small).close()
+    with _only(2600 * MB, release=False):
+        before = _free()
+        with pytest.raises(gpu.TransientError, match="does not fit"):
+            gpu.Context(big)
+        assert abs(_free() - before) < 64 * MB
+        gpu.Context(small).close()                           # 1 GB of the pool, 2.6 GB beside it
+        assert abs(_free() - before) < 64 * MB
