@@ -1510,15 +1510,18 @@ extern "C" tr_status tr_render_region_noalloc(tr_ctx* x, uint32_t x0, uint32_t y
 // -----------------------------------------------------------------------------------------
 
 namespace tri {
-tr_status guide_check_err(tr_guide* g, cudaStream_t s) {
-    int e = 0;
-    TR_CUDA(cudaMemcpyAsync(&e, g->err, sizeof(int), cudaMemcpyDeviceToHost, s));
+tr_status guide_check(tr_guide* g, cudaStream_t s, bool infer, bool train) {
+    int h[tr_guide::kWords] = {};
+    TR_CUDA(cudaMemcpyAsync(h, g->status, sizeof(h), cudaMemcpyDeviceToHost, s));
     TR_CUDA(cudaStreamSynchronize(s));
-    if (e) {
-        TR_CUDA(cudaMemsetAsync(g->err, 0, sizeof(int), s));
-        return fail(TR_ERR_TIMEOUT, "tensor-core MMA completion wait timed out");
+    infer = infer && h[tr_guide::kInfer];
+    train = train && h[tr_guide::kTrain];
+    if (infer) TR_CUDA(cudaMemsetAsync(g->status + tr_guide::kInfer, 0, sizeof(int), s));
+    if (train) {
+        TR_CUDA(cudaMemsetAsync(g->status + tr_guide::kTrain, 0, sizeof(int), s));
+        g->step = (uint32_t)h[tr_guide::kSteps];
     }
-    return TR_OK;
+    return infer || train ? fail(TR_ERR_TIMEOUT, "tensor-core MMA completion wait timed out") : TR_OK;
 }
 }  // namespace tri
 
@@ -1552,7 +1555,7 @@ extern "C" tr_status tr_guide_create(int device, uint64_t seed, tr_guide** out) 
         g->m2 = g->alloc<float>(TR_GUIDE_PARAMS);
         g->w_fwd = g->alloc<uint8_t>(4 * 8192);
         g->w_bwd = g->alloc<uint8_t>(4 * 8192);
-        g->err = g->alloc<int>(1);
+        g->status = g->alloc<int>(tr_guide::kWords);
         g->scalars = g->alloc<float>(4);
         // He-uniform hidden layers; a small output layer so the first mixture is broad
         std::vector<float> p(TR_GUIDE_PARAMS, 0.0f);
@@ -1570,7 +1573,7 @@ extern "C" tr_status tr_guide_create(int device, uint64_t seed, tr_guide** out) 
         TR_CUDA(cudaMemsetAsync(g->m1, 0, sizeof(float) * TR_GUIDE_PARAMS, g->stream));
         TR_CUDA(cudaMemsetAsync(g->m2, 0, sizeof(float) * TR_GUIDE_PARAMS, g->stream));
         TR_CUDA(cudaMemsetAsync(g->grads, 0, sizeof(float) * TR_GUIDE_PARAMS, g->stream));
-        TR_CUDA(cudaMemsetAsync(g->err, 0, sizeof(int), g->stream));
+        TR_CUDA(cudaMemsetAsync(g->status, 0, tr_guide::kWords * sizeof(int), g->stream));
         TR_CUDA(trg::pack_weights(g->params, g->w_fwd, g->w_bwd, g->stream));
         TR_CUDA(cudaStreamSynchronize(g->stream));
     } catch (const CudaError& e) {
@@ -1626,8 +1629,8 @@ extern "C" tr_status tr_guide_forward(tr_guide* g, const uint16_t* d_features, u
     try {
         TR_CUDA(cudaSetDevice(g->device));
         cudaStream_t s = stream ? static_cast<cudaStream_t>(stream) : g->stream;
-        TR_CUDA(trg::mlp_forward(g->dev(), reinterpret_cast<const uint4*>(d_features), n, d_out, g->err, s));
-        return guide_check_err(g, s);
+        TR_CUDA(trg::mlp_forward(g->dev(), reinterpret_cast<const uint4*>(d_features), n, d_out, guide_err(g), s));
+        return guide_check(g, s, true, false);
     } catch (const CudaError& e) {
         return fail(TR_ERR_CUDA, e.what());
     }
@@ -1646,7 +1649,8 @@ void train_enqueue(tr_guide* g, const uint4* x, const float* d_dirs, const float
     a.scratch = g->scratch; a.loss = g->scalars + 1;
     a.params = g->params; a.grads = g->grads; a.m1 = g->m1; a.m2 = g->m2;
     a.w_fwd = g->w_fwd; a.w_bwd = g->w_bwd;
-    a.err = g->err;
+    a.err = g->status + tr_guide::kTrain;
+    a.steps = g->status + tr_guide::kSteps;
     a.lr = lr;
     a.step = g->step;
     TR_CUDA(trg::train_step(a, n, s));
@@ -1662,7 +1666,7 @@ extern "C" tr_status tr_guide_train_step(tr_guide* g, const uint16_t* d_features
         cudaStream_t s = stream ? static_cast<cudaStream_t>(stream) : g->stream;
         train_enqueue(g, reinterpret_cast<const uint4*>(d_features), d_dirs, d_weights, n, lr, s);
         if (loss) TR_CUDA(cudaMemcpyAsync(loss, g->scalars + 1, sizeof(float), cudaMemcpyDeviceToHost, s));
-        return guide_check_err(g, s);
+        return guide_check(g, s, false, true);
     } catch (const CudaError& e) {
         return fail(e.code == cudaErrorMemoryAllocation ? TR_ERR_OUT_OF_MEMORY : TR_ERR_CUDA, e.what());
     }
@@ -1686,19 +1690,19 @@ extern "C" tr_status tr_guide_destroy(tr_guide* g) {
 
 namespace tri {
 trg::GuideDev guide_dev(tr_guide* g) { return g->dev(); }
-int* guide_err(tr_guide* g) { return g->err; }
+int* guide_err(tr_guide* g) { return g->status + tr_guide::kInfer; }
 
 tr_status train_on_pool(tr_guide* g, const trk::GuideWave& gw, const uint32_t* pool_state, uint32_t pool, float lr,
                         cudaStream_t s, tr_stats& stats) {
     stats.train_steps = 0;
-    if (!pool) return guide_check_err(g, s);
+    if (!pool) return guide_check(g, s, true, false);
     // one synchronisation for the render's MMA status and the pool fill ...
     int e = 0;
     uint32_t fill = 0;
-    TR_CUDA(cudaMemcpyAsync(&e, g->err, sizeof(int), cudaMemcpyDeviceToHost, s));
+    TR_CUDA(cudaMemcpyAsync(&e, guide_err(g), sizeof(int), cudaMemcpyDeviceToHost, s));
     TR_CUDA(cudaMemcpyAsync(&fill, pool_state, sizeof(uint32_t), cudaMemcpyDeviceToHost, s));
     TR_CUDA(cudaStreamSynchronize(s));
-    if (e) return guide_check_err(g, s);
+    if (e) return guide_check(g, s, true, false);
     // ... the training steps are enqueued back to back, and one more for their status and loss
     const uint32_t n = std::min(fill, pool);
     try {
@@ -1712,7 +1716,7 @@ tr_status train_on_pool(tr_guide* g, const trk::GuideWave& gw, const uint32_t* p
     }
     if (stats.train_steps) {
         TR_CUDA(cudaMemcpyAsync(&stats.train_loss, g->scalars + 1, sizeof(float), cudaMemcpyDeviceToHost, s));
-        return guide_check_err(g, s);
+        return guide_check(g, s, false, true);
     }
     return TR_OK;
 }
@@ -1770,7 +1774,7 @@ tr_status guide_end_render(tr_ctx* x, cudaStream_t s) {
     std::swap(w.pool_meta, a.meta);
     std::swap(x->pool_state, a.state);
     x->pool_pending = std::min(fill, x->guide_pool);
-    return guide_check_err(g, g->stream);             // tensor-core timeouts of render or training
+    return guide_check(g, g->stream, true, true);     // tensor-core timeouts of render or training
 }
 }  // namespace
 

@@ -474,8 +474,9 @@ __global__ void __launch_bounds__(128) k_dw_tc(DwLayers L, uint32_t m, uint32_t 
 
 // The step's tail in one launch: every parameter's gradient as the sum of the CTAs' parts (four lanes
 // per parameter, a fixed order), the batch loss, and with lr > 0 Adam (Kingma & Ba 2015) on the FP32
-// master parameters and the repacked BF16 tiles.  After a wait that timed out (*err) the parts are not
-// complete and the parameters stay.
+// master parameters and the repacked BF16 tiles.  After a wait that timed out (*err, written by this step's
+// kernels before this one only, so every thread reads the same) the parts are not complete: parameters, moments
+// and the count of steps stay.
 __global__ void __launch_bounds__(256) k_update(UpdateArgs u) {
     const uint32_t t = blockIdx.x * blockDim.x + threadIdx.x, i = t >> 2, q = t & 3u;
     const bool bias = i >= 4u * 4096u;
@@ -513,7 +514,10 @@ __global__ void __launch_bounds__(256) k_update(UpdateArgs u) {
         for (int off = 16; off > 0; off >>= 1) loss += __shfl_xor_sync(0xffffffffu, loss, off);
         if ((threadIdx.x & 31u) == 0) s[threadIdx.x >> 5] = loss;
         __syncthreads();
-        if (threadIdx.x == 0) *u.loss = ((s[0] + s[1]) + (s[2] + s[3])) + ((s[4] + s[5]) + (s[6] + s[7]));
+        if (threadIdx.x == 0) {
+            *u.loss = ((s[0] + s[1]) + (s[2] + s[3])) + ((s[4] + s[5]) + (s[6] + s[7]));
+            if (u.lr > 0.0f && *u.err == 0) *u.steps += 1;
+        }
     }
 }
 
@@ -565,7 +569,8 @@ cudaError_t train_step(const TrainArgs& a, uint32_t m, cudaStream_t s) {
     L.part = part;
     k_dw_tc<<<dim3(parts, 4), 128, kDwSmemBytes, s>>>(L, m, (ktiles + parts - 1) / parts, a.net.spin, a.err);
     UpdateArgs u{};
-    u.part = part; u.nparts = parts; u.loss_part = loss_part; u.ntiles = tiles; u.err = a.err; u.loss = a.loss;
+    u.part = part; u.nparts = parts; u.loss_part = loss_part; u.ntiles = tiles; u.loss = a.loss;
+    u.err = a.err; u.steps = a.steps;
     u.params = a.params; u.grads = a.grads; u.m1 = a.m1; u.m2 = a.m2; u.w_fwd = a.w_fwd; u.w_bwd = a.w_bwd;
     u.lr = a.lr;
     u.c1 = 1.0f - powf(0.9f, (float)a.step);

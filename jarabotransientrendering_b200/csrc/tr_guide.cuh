@@ -49,6 +49,7 @@ struct UpdateArgs {
     const float *part, *loss_part;
     uint32_t nparts, ntiles;
     const int* err;
+    int* steps;
     float *loss, *params, *grads, *m1, *m2;
     uint8_t *w_fwd, *w_bwd;
     float lr, c1, c2;
@@ -63,7 +64,7 @@ struct TrainArgs {
     uint4 *act, *dy, *dh;
     float *scratch, *loss, *params, *grads, *m1, *m2;
     uint8_t *w_fwd, *w_bwd;
-    int* err;
+    int *err, *steps;          // set when a wait times out; counts the steps applied
     float lr;
     uint32_t step;
 };

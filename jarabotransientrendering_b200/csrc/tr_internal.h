@@ -89,14 +89,17 @@ struct tr_guide {
     float* m2 = nullptr;
     uint8_t* w_fwd = nullptr;  // packed BF16 tiles
     uint8_t* w_bwd = nullptr;
-    int* err = nullptr;
+    // device words: [kInfer] / [kTrain] a wait of inference / of a training step timed out, [kSteps] training
+    // steps applied.  Training runs beside renders that sample with the network, so each has its own word.
+    enum { kInfer = 0, kTrain = 1, kSteps = 2, kWords = 3 };
+    int* status = nullptr;
     float* scalars = nullptr;  // [0] weight sum, [1] loss
     uint32_t cap = 0;
     uint4* act = nullptr;
     float* scratch = nullptr;          // partial sums of a training step
     uint4* dy_bf = nullptr;
     uint4* dh = nullptr;       // BF16 hidden-layer gradients [3][n][64]
-    uint32_t step = 0;
+    uint32_t step = 0;                 // training steps enqueued; after one that timed out, those applied
     uint32_t spin = trg::kWaitPolls;   // mbarrier polls before a tensor-core wait times out
     template <class T>
     T* alloc(size_t n) {
@@ -295,7 +298,8 @@ void ensure_guided(tr_ctx* x, uint32_t capacity);
 trk::Params make_params(tr_ctx* x);
 trg::GuideDev guide_dev(tr_guide* g);
 int* guide_err(tr_guide* g);
-tr_status guide_check_err(tr_guide* g, cudaStream_t s);
+// waits for stream s and reports (and clears) waits that timed out in inference, in training steps or in either
+tr_status guide_check(tr_guide* g, cudaStream_t s, bool infer, bool train);
 // enqueues one training step of the proposal on stream s (no host synchronisation)
 void train_enqueue(tr_guide* g, const uint4* x, const float* d_dirs, const float* d_weights, uint32_t n, float lr,
                    cudaStream_t s);
