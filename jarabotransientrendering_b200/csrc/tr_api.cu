@@ -469,7 +469,7 @@ tr_status render_region(tr_ctx* x, uint32_t x0, uint32_t y0, uint32_t x1, uint32
     // not depend on the batch size).
     uint32_t large = 1;
     if (max_lanes > 1 && total_slots >= kLargeCapacity && !(sink && sink->type != TR_FILM_RGBE)) {
-        const int lanes = sink ? 3 : 2;
+        const int lanes = large_lanes(rgbe);
         const uint64_t slots = std::min<uint64_t>(sink ? kLargeCapacity / 2 : kLargeCapacity, total_slots / (uint64_t)lanes);
         const size_t per_slot = (guided ? 80u : 0u) +
             carve_wave(nullptr, nullptr, 1u << 16, std::max<uint32_t>(1u, x->integ.max_bounces), true) / (1u << 16);
@@ -666,13 +666,12 @@ tr_status render_region(tr_ctx* x, uint32_t x0, uint32_t y0, uint32_t x1, uint32
             cudaStream_t s_gen = nullptr, s_conn = nullptr;
             trk::Params pc = p;
             if (bidir && x->bd.nvert) {
-                if (!x->lane_stream[0]) TR_CUDA(cudaStreamCreateWithFlags(&x->lane_stream[0], cudaStreamNonBlocking));
-                if (!x->lane_shadow_stream[0])
-                    TR_CUDA(cudaStreamCreateWithFlags(&x->lane_shadow_stream[0], cudaStreamNonBlocking));
+                for (cudaStream_t& c : x->conn_stream)
+                    if (!c) TR_CUDA(cudaStreamCreateWithFlags(&c, cudaStreamNonBlocking));
                 for (cudaEvent_t& e : x->bd_free)
                     if (!e) TR_CUDA(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
-                s_gen = x->lane_stream[0];
-                s_conn = x->lane_shadow_stream[0];
+                s_gen = x->conn_stream[0];
+                s_conn = x->conn_stream[1];
                 const size_t R = (size_t)x->integ.max_bounces + x->bd.ncand;
                 TR_CUDA(cudaMemsetAsync(x->bd.valid, 0, R * x->wave.capacity, ls));
                 TR_CUDA(order(x->light_stream, s_gen));

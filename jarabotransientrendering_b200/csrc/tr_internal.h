@@ -70,6 +70,9 @@ constexpr size_t kLeastFree = (size_t)2 << 30;  // device memory left for a new 
 #define TR_WAVE_LANES 4
 #endif
 constexpr int kWaveLanes = TR_WAVE_LANES;        // wave buffer sets batches alternate between
+static_assert(kWaveLanes >= 1, "a render needs a wave");
+// lanes of a large render's batches (three with RGBE delivery), of those the build has
+constexpr int large_lanes(bool rgbe) { return std::min(rgbe ? 3 : 2, kWaveLanes); }
 // default roughness below which GGX vertices sample their BSDF instead of the learned proposal
 constexpr float kGuideMinAlpha = 0.5f;
 constexpr uint32_t kTrainBatch = 65536, kTrainLeast = 1024;     // samples of a training step: at most, at least
@@ -181,6 +184,7 @@ struct tr_ctx {
     cudaStream_t shadow_stream = nullptr;
     cudaStream_t lane_stream[tri::kWaveLanes - 1]{}, lane_shadow_stream[tri::kWaveLanes - 1]{};
     cudaStream_t light_stream = nullptr;    // light subpaths beside the eye walks (bidirectional)
+    cudaStream_t conn_stream[2]{};          // setting up and tracing their connections
     std::vector<cudaEvent_t> dep_events;    // ordering events (no timing), reused in turn
     size_t next_dep = 0;
     float* d_stage = nullptr;               // FP32 staging of one pixel batch's rows
@@ -267,6 +271,10 @@ struct tr_ctx {
             if (lane_stream[k]) cudaStreamDestroy(lane_stream[k]);
             if (lane_shadow_stream[k]) cudaStreamDestroy(lane_shadow_stream[k]);
             lane_stream[k] = lane_shadow_stream[k] = nullptr;
+        }
+        for (cudaStream_t& c : conn_stream) {
+            if (c) cudaStreamDestroy(c);
+            c = nullptr;
         }
         if (light_stream) cudaStreamDestroy(light_stream);
         shadow_stream = light_stream = nullptr;
