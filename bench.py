@@ -255,9 +255,15 @@ WORKLOAD_CONFIG = "icosphere subdiv 7 in Cornell box, 512x512, 2048 bins x 0.002
 
 def run_reference(args, rank, world):
     """The reference arm: the reference's own renderer (Embree backend, streak splat on) on all
-    host cores; rank 0 alone runs it under torchrun."""
+    host cores; rank 0 alone runs it under torchrun.  Where its program was not built the arm is
+    unavailable: nothing else stands in for it."""
     from jarabotransientrendering_b200 import scenes as S
+    from oracle import refscene
     if rank != 0:
+        return
+    if not os.path.exists(refscene.REF_BIN):
+        print(json.dumps({"impl": "reference", "unavailable": "the reference's program is not built "
+                          "(oracle/_ref/ref_render: needs the reference's sources at build time)"}), flush=True)
         return
     sc = S.WORKLOADS[WORKLOAD]()
     procs = max(1, min(host_cores(), sc.height))
