@@ -421,7 +421,9 @@ tr_status tr_set_stream(tr_ctx* ctx, void* stream);
  * when it ends (tr_stats: the last render's); 2 on, read out at the next tr_stats_get (tr_stats:
  * the sums over the renders since the previous read, or the previous sums again when no render
  * ran since), which keeps the read-out, about 1.5 us of
- * host time per timed launch, out of the renders.                                          */
+ * host time per timed launch, out of the renders.  With timing on, the launches that walk whole
+ * paths (small renders) or the last depths of a lone batch are replaced by the per-depth kernels
+ * whose times are asked for: such a render takes longer than without, its film is the same.  */
 tr_status tr_set_profiling(tr_ctx* ctx, int on);
 tr_status tr_destroy(tr_ctx* ctx);
 

@@ -1600,7 +1600,8 @@ __device__ float mis_quantity(const Params& p, uint32_t slot, uint32_t t, uint32
 // reference connects when World::intersects returns true, World.h:617-639 / 693-697).
 // A warp tests its slots' pairs light vertex by light vertex, one slot per lane, lists those that get
 // a ray in shared memory and sets up 32 of them at a time, one per lane; what is left over joins the
-// next slots' pairs.  Bound by issue: a slot has 0 to max_bounces - 1 pairs and fewer slots have an
+// next slots' pairs.  The eye walk goes on beside it: k_shade of the next depth may raise a slot's ne from ie + 1
+// to ie + 2 while it is read here, and either value says the same, that vertex ie is there.  Bound by issue: a slot has 0 to max_bounces - 1 pairs and fewer slots have an
 // eye vertex the deeper it is, so with one slot per thread 8 of 32 lanes were active (depth 8: 650 us
 // of launches for 480 k paths, in a render of 3.53 ms; now 3.34; depth 12, 1.2 M paths: 10.85 -> 9.9).
 // Grids of 2 or 16 blocks per SM are equal.
