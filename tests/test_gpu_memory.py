@@ -171,3 +171,18 @@ def test_refused_film_is_not_taken_first(gpu):
         assert abs(_free() - before) < 64 * MB
         gpu.Context(small).close()                           # 1 GB of the pool, 2.6 GB beside it
         assert abs(_free() - before) < 64 * MB
+
+
+def test_small_batches_where_the_large_ones_do_not_fit(gpu):
+    """With too little free memory for the two large batches of a render, eight small ones, and the large ones
+    again with memory there."""
+    sc = S.cornell(width=512, height=512, time_bins=4, exposure=1.28, max_bounces=3, sqrt_spp=8)
+    wave = 2 + 3 * 3
+    with gpu.Context(sc) as ctx:
+        ctx.render(0, 1)
+        # two batches of 8 M slots take 2.9 GB, four of 2 M slots 1.5 GB
+        for free, batches in ((2300, 8), (4000, 8), (6000, 2)):
+            with _only(free * MB):
+                ctx.render(0, 64)
+            assert ctx.stats()["kernel_launches"] == batches * wave
+        assert (ctx.film()["weight"] == 193).all()
