@@ -900,7 +900,7 @@ bool build_bvh_device(const float* d_v, uint32_t nv, const uint32_t* d_t, uint32
     TR_CUDA(cudaGetDevice(&dev));
     TR_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
     void* block = nullptr;
-    TR_CUDA(cudaMallocFromPoolAsync(&block, carve(nullptr), tri::device_pool(dev), s));
+    TR_CUDA(tri::pool_malloc(&block, carve(nullptr), s));
     struct Free { void* p; cudaStream_t s; ~Free() { cudaFreeAsync(p, s); } } release{block, s};
     carve(static_cast<char*>(block));
 

@@ -123,38 +123,52 @@ void upload(void* dst, const void* src, size_t bytes, cudaStream_t s) {
 
 namespace tri {
 
-cudaMemPool_t device_pool(int device) {
+cudaMemPool_t device_pool(int device, Pool which) {
     static std::mutex mu;
     static std::vector<cudaMemPool_t> pools;
     std::lock_guard<std::mutex> lock(mu);
     if (device < 0) throw CudaError(cudaErrorInvalidDevice, "device_pool");
-    if ((size_t)device >= pools.size()) pools.resize((size_t)device + 1, nullptr);
-    if (!pools[device]) {
+    const size_t at = 2 * (size_t)device + (which == Pool::kLarge ? 1u : 0u);
+    if (at >= pools.size()) pools.resize(at + 1, nullptr);
+    if (!pools[at]) {
         cudaMemPoolProps props{};
         props.allocType = cudaMemAllocationTypePinned;
         props.location.type = cudaMemLocationTypeDevice;
         props.location.id = device;
         cudaMemPool_t pool = nullptr;
         TR_CUDA(cudaMemPoolCreate(&pool, &props));
-        uint64_t keep = ~0ull;
+        uint64_t keep = which == Pool::kLarge ? (uint64_t)kLargeWaveBytes : ~0ull;
         TR_CUDA(cudaMemPoolSetAttribute(pool, cudaMemPoolAttrReleaseThreshold, &keep));
-        pools[device] = pool;
+        pools[at] = pool;
     }
-    return pools[device];
+    return pools[at];
 }
 
-size_t pool_idle_bytes(int device) {
+size_t pool_idle_bytes(int device, Pool which) {
     uint64_t reserved = 0, used = 0;
-    cudaMemPool_t pool = device_pool(device);
+    cudaMemPool_t pool = device_pool(device, which);
     if (cudaMemPoolGetAttribute(pool, cudaMemPoolAttrReservedMemCurrent, &reserved) != cudaSuccess) return 0;
     if (cudaMemPoolGetAttribute(pool, cudaMemPoolAttrUsedMemCurrent, &used) != cudaSuccess) return 0;
     return reserved > used ? (size_t)(reserved - used) : 0;
 }
 
-// Memory kept by the pool goes back to the driver (nothing where there is no pool).
-static void trim_pool(int device) noexcept {
+cudaError_t pool_malloc(void** p, size_t bytes, cudaStream_t s, Pool which) {
+    int dev = 0;
+    cudaError_t e = cudaGetDevice(&dev);
+    if (e != cudaSuccess) return e;
+    e = cudaMallocFromPoolAsync(p, bytes, device_pool(dev, which), s);
+    if (e == cudaErrorMemoryAllocation && which == Pool::kKept) {
+        cudaGetLastError();
+        cudaMemPoolTrimTo(device_pool(dev, Pool::kLarge), 0);       // what it keeps is free memory
+        e = cudaMallocFromPoolAsync(p, bytes, device_pool(dev, which), s);
+    }
+    return e;
+}
+
+// Memory kept by the pools goes back to the driver (nothing where there are none).
+static void trim_pools(int device) noexcept {
     try {
-        cudaMemPoolTrimTo(device_pool(device), 0);
+        for (Pool which : {Pool::kKept, Pool::kLarge}) cudaMemPoolTrimTo(device_pool(device, which), 0);
     } catch (const CudaError&) {
     }
 }
@@ -198,7 +212,7 @@ static void drop_first_wave(tr_ctx* x, cudaStream_t after = nullptr) {
     drop(bd.lvert, bd.evert, bd.nl, bd.ne, bd.L0, bd.co_o, bd.co_d, bd.co_L, bd.valid);
 }
 
-void ensure_wave(tr_ctx* x, uint32_t capacity) {
+void ensure_wave(tr_ctx* x, uint32_t capacity, Pool which) {
     if (x->wave.capacity >= capacity) return;
     // grow: drop the old buffers (they are only scratch between calls)
     drop_first_wave(x);
@@ -209,7 +223,7 @@ void ensure_wave(tr_ctx* x, uint32_t capacity) {
     if (x->integ.flags & TR_FLAG_BIDIRECTIONAL) R += R * (R - 1) / 2;
     const bool tsm = (x->integ.flags & TR_FLAG_TIME_SAMPLING) != 0;
     try {
-        w.block = x->alloc<unsigned char>(carve_wave(nullptr, nullptr, capacity, R, tsm));
+        w.block = x->alloc<unsigned char>(carve_wave(nullptr, nullptr, capacity, R, tsm), which);
         if (x->integ.flags & TR_FLAG_BIDIRECTIONAL) {
             // light wave (own rays, queues, counters; shares target and ray counts) and the
             // subpath vertex arrays
@@ -312,14 +326,14 @@ void drop_waves(tr_ctx* x, cudaStream_t after) {
 
 // Lane k + 1's buffers: the per-slot arrays of `capacity` slots, its own queue counters, the first
 // wave's statistics counters.
-void ensure_lane_wave(tr_ctx* x, int k, uint32_t capacity) {
+void ensure_lane_wave(tr_ctx* x, int k, uint32_t capacity, Pool which) {
     trk::Wave& w = x->lane_wave[k];
     if (w.capacity >= capacity && w.counters) return;
     x->drop(w.block);
     w.capacity = 0;
     const size_t R = std::max<uint32_t>(1u, x->integ.max_bounces);
     const bool tsm = (x->integ.flags & TR_FLAG_TIME_SAMPLING) != 0;
-    w.block = x->alloc<unsigned char>(carve_wave(nullptr, nullptr, capacity, R, tsm));
+    w.block = x->alloc<unsigned char>(carve_wave(nullptr, nullptr, capacity, R, tsm), which);
     if (!w.counters) w.counters = x->alloc<uint32_t>(trk::kCounters);
     w.stats = x->wave.stats;
     carve_wave(&w, w.block, capacity, R, tsm);
@@ -327,11 +341,11 @@ void ensure_lane_wave(tr_ctx* x, int k, uint32_t capacity) {
 
 // Lane k + 1's guided-vertex records (the training pool and its counters are shared: the
 // batches of all lanes fill it, each entry tagged with its batch).
-void ensure_lane_guided(tr_ctx* x, int k, uint32_t capacity) {
+void ensure_lane_guided(tr_ctx* x, int k, uint32_t capacity, Pool which) {
     if (x->lane_vrec_cap[k] >= capacity && x->lane_vrec[k]) return;
     x->drop(x->lane_vrec[k]);
     x->lane_vrec_cap[k] = 0;
-    x->lane_vrec[k] = x->alloc<uint4>((size_t)capacity * 5);
+    x->lane_vrec[k] = x->alloc<uint4>((size_t)capacity * 5, which);
     x->lane_vrec_cap[k] = capacity;
 }
 
@@ -364,11 +378,11 @@ void ensure_guide_pools(tr_ctx* x) {
 }
 
 // The first lane's guided-vertex records.
-void ensure_guided(tr_ctx* x, uint32_t capacity) {
+void ensure_guided(tr_ctx* x, uint32_t capacity, Pool which) {
     if (x->gw_capacity >= capacity) return;
     x->drop(x->gw.vrec);
     x->gw_capacity = 0;
-    x->gw.vrec = x->alloc<uint4>((size_t)capacity * 5);
+    x->gw.vrec = x->alloc<uint4>((size_t)capacity * 5, which);
     x->gw_capacity = capacity;
 }
 
@@ -479,11 +493,12 @@ tr_status render_region(tr_ctx* x, uint32_t x0, uint32_t y0, uint32_t x1, uint32
     }
     const uint32_t small_cap = cap;
     auto buffers = [&](uint32_t n_lanes) {
-        ensure_wave(x, cap);
-        if (guided) ensure_guided(x, cap);
+        const Pool which = large > 1 ? Pool::kLarge : Pool::kKept;
+        ensure_wave(x, cap, which);
+        if (guided) ensure_guided(x, cap, which);
         for (uint32_t k = 0; k + 1 < n_lanes; ++k) {
-            ensure_lane_wave(x, (int)k, cap);
-            if (guided) ensure_lane_guided(x, (int)k, cap);
+            ensure_lane_wave(x, (int)k, cap, which);
+            if (guided) ensure_lane_guided(x, (int)k, cap, which);
             if (!x->lane_stream[k]) TR_CUDA(cudaStreamCreateWithFlags(&x->lane_stream[k], cudaStreamNonBlocking));
             if (!x->lane_shadow_stream[k])
                 TR_CUDA(cudaStreamCreateWithFlags(&x->lane_shadow_stream[k], cudaStreamNonBlocking));
@@ -494,17 +509,17 @@ tr_status render_region(tr_ctx* x, uint32_t x0, uint32_t y0, uint32_t x1, uint32
         return (int)std::min<uint64_t>((uint64_t)max_lanes, (win_pix + ppb - 1) / ppb);
     };
     if (large > 1) {
-        // they may take what the pool holds, and of the rest what leaves a new context its share (the query
+        // they may take what their pool holds, and of the rest what leaves a new context its share (the query
         // takes 0.2 ms: asked only where the pool is short of them)
         cap = unit * large * ns_chunk * ninc;
         const size_t need = (size_t)lanes_of() *
             (carve_wave(nullptr, nullptr, cap, std::max<uint32_t>(1u, x->integ.max_bounces),
                         (x->integ.flags & TR_FLAG_TIME_SAMPLING) != 0) + (guided ? (size_t)cap * 5 * sizeof(uint4) : 0));
-        size_t room = pool_idle_bytes(x->device), free_b = 0, total_b = 0;
+        size_t room = pool_idle_bytes(x->device, Pool::kLarge), free_b = 0, total_b = 0;
         if (room < need) {
             TR_CUDA(cudaMemGetInfo(&free_b, &total_b));
             room += free_b;
-            if (room < need + kLeastFree) large = 1;
+            if (room < need || room - need + pool_idle_bytes(x->device, Pool::kKept) < kLeastFree) large = 1;
         }
     }
     if (large > 1) {
@@ -812,7 +827,7 @@ tr_status render_region(tr_ctx* x, uint32_t x0, uint32_t y0, uint32_t x1, uint32
     x->stats.camera_samples += win_pix * ns_total;
     x->stats.render_ms = ms;
     if (large > 1) {
-        // large batches are the pool's again between calls (small ones stay): contexts that render in turn
+        // large batches are their pool's again between calls (small ones stay): contexts that render in turn
         // share them, and a context made meanwhile finds their memory
         drop_waves(x, strm);
         TR_CUDA(cudaStreamSynchronize(strm));
@@ -885,7 +900,8 @@ tr_status tr_create(const tr_scene* s, const tr_camera* c, const tr_film* f, con
         // pool grows by anyway) until the scene's uploads are under way.
         const size_t film_bytes = (1 + nb) * nstreak * sizeof(double);
         auto refuse_film = [&] {
-            const size_t idle = tri::pool_idle_bytes(device);      // kept by the pool for reuse
+            // kept by the pools for reuse
+            const size_t idle = tri::pool_idle_bytes(device, Pool::kKept) + tri::pool_idle_bytes(device, Pool::kLarge);
             if (idle + x->bytes >= film_bytes + kLeastFree) return false;
             size_t free_b = 0, total_b = 0;
             cudaMemGetInfo(&free_b, &total_b);
@@ -1082,7 +1098,7 @@ tr_status tr_create(const tr_scene* s, const tr_camera* c, const tr_film* f, con
     } catch (const CudaError& e) {
         x->release();
         delete x;
-        if (e.code == cudaErrorMemoryAllocation) trim_pool(device);     // what it took is not kept for it
+        if (e.code == cudaErrorMemoryAllocation) trim_pools(device);     // what it took is not kept for it
         return fail(e.code == cudaErrorMemoryAllocation ? TR_ERR_OUT_OF_MEMORY : TR_ERR_CUDA, e.what());
     } catch (const std::bad_alloc&) {
         x->release();
@@ -1111,7 +1127,7 @@ tr_status tr_release_cached_memory(int device) {
         if (device < 0 || device >= n) return fail(TR_ERR_INVALID_ARGUMENT, "no such device");
         TR_CUDA(cudaSetDevice(device));
         TR_CUDA(cudaDeviceSynchronize());
-        TR_CUDA(cudaMemPoolTrimTo(tri::device_pool(device), 0));
+        for (Pool which : {Pool::kKept, Pool::kLarge}) TR_CUDA(cudaMemPoolTrimTo(tri::device_pool(device, which), 0));
     } catch (const CudaError& e) {
         return fail(TR_ERR_CUDA, e.what());
     }

@@ -37,25 +37,29 @@ struct CudaError : std::runtime_error {
 // Device memory of contexts, guides and batches comes from one stream-ordered pool per device
 // that keeps freed memory for the next allocations (release threshold unlimited), so creating
 // and destroying contexts does not map and unmap gigabytes each time; memory goes back to the
-// driver only through tr_release_cached_memory or at exit.
-cudaMemPool_t device_pool(int device);
+// driver only through tr_release_cached_memory or at exit.  A large render's batches come and go with
+// each call; they have a pool of their own, or what other contexts keep would be carved from their blocks and the
+// next large render would have to map new ones (13 to 20 ms).  That pool keeps at most kLargeWaveBytes, which
+// the other gets when it finds no memory.
+enum class Pool { kKept, kLarge };
+cudaMemPool_t device_pool(int device, Pool which = Pool::kKept);
 // pool memory of `device` reserved but not in use (free for the next allocations)
-size_t pool_idle_bytes(int device);
+size_t pool_idle_bytes(int device, Pool which);
+// cudaMallocFromPoolAsync on stream s, from the current device's pool
+cudaError_t pool_malloc(void** p, size_t bytes, cudaStream_t s, Pool which = Pool::kKept);
 
 template <class T>
-T* dalloc(size_t count, size_t& total) {
+T* dalloc(size_t count, size_t& total, Pool which = Pool::kKept) {
     if (count == 0) count = 1;
-    int dev = 0;
-    cudaError_t e = cudaGetDevice(&dev);
     void* p = nullptr;
-    if (e == cudaSuccess) e = cudaMallocFromPoolAsync(&p, count * sizeof(T), device_pool(dev), 0);
+    cudaError_t e = pool_malloc(&p, count * sizeof(T), 0, which);
     if (e == cudaSuccess) e = cudaStreamSynchronize(0);     // usable from every stream
     if (e != cudaSuccess) throw CudaError(e, "device allocation");
     total += count * sizeof(T);
     return static_cast<T*>(p);
 }
 
-// Gives memory of the current device back to its pool once the device is idle (any stream may have used it).
+// Gives memory of the current device back to the pool it came from once the device is idle (any stream may have used it).
 // In stream order, not by cudaFree: what that returns the pool can hand out again but goes on counting as used,
 // and pool_idle_bytes would miss it.
 void dfree(const std::vector<void*>& blocks);
@@ -236,9 +240,9 @@ struct tr_ctx {
     cudaStream_t s() const { return user_stream ? user_stream : stream; }
 
     template <class T>
-    T* alloc(size_t n) {
+    T* alloc(size_t n, tri::Pool which = tri::Pool::kKept) {
         const size_t before = bytes;
-        T* p = tri::dalloc<T>(n, bytes);
+        T* p = tri::dalloc<T>(n, bytes, which);
         allocs.push_back({p, bytes - before});
         return p;
     }
@@ -297,12 +301,12 @@ namespace tri {
 // Per-slot arrays of a wave of `capacity` slots with R records each, carved from one block (one
 // pool allocation instead of fourteen): with w null the bytes it takes, else w's pointers into it.
 size_t carve_wave(trk::Wave* w, void* block, uint32_t capacity, size_t R, bool time_sampling);
-void ensure_wave(tr_ctx* x, uint32_t capacity);
+void ensure_wave(tr_ctx* x, uint32_t capacity, Pool which = Pool::kKept);
 void drop_waves(tr_ctx* x, cudaStream_t after = nullptr);
-void ensure_lane_wave(tr_ctx* x, int k, uint32_t capacity);
-void ensure_lane_guided(tr_ctx* x, int k, uint32_t capacity);
+void ensure_lane_wave(tr_ctx* x, int k, uint32_t capacity, Pool which);
+void ensure_lane_guided(tr_ctx* x, int k, uint32_t capacity, Pool which);
 void ensure_guide_pools(tr_ctx* x);
-void ensure_guided(tr_ctx* x, uint32_t capacity);
+void ensure_guided(tr_ctx* x, uint32_t capacity, Pool which);
 trk::Params make_params(tr_ctx* x);
 trg::GuideDev guide_dev(tr_guide* g);
 int* guide_err(tr_guide* g);

@@ -186,3 +186,32 @@ def test_small_batches_where_the_large_ones_do_not_fit(gpu):
                 ctx.render(0, 64)
             assert ctx.stats()["kernel_launches"] == batches * wave
         assert (ctx.film()["weight"] == 193).all()
+
+
+def test_large_batches_are_not_carved_up(gpu):
+    """What other contexts keep is not taken out of the large batches' memory while that is idle: a large render
+    after them maps nothing new."""
+    sc = S.cornell(width=512, height=512, time_bins=8, exposure=0.64, max_bounces=6, sqrt_spp=8)
+    _abi.check(_abi.lib().tr_release_cached_memory(0))
+    with gpu.Context(sc) as a, gpu.Context(sc) as b, gpu.Context(sc) as c:
+        a.render(0, 64)
+        for x in (b, c):
+            x.render(0, 31)                                  # four batches of 2 M slots each, kept
+        before = _free()
+        a.render(64, 64)
+        assert before - _free() < 64 * MB
+
+
+def test_idle_large_batches_count_as_free(gpu):
+    """Memory that large renders left idle is there for a film that needs it."""
+    sc = S.cornell(width=512, height=512, time_bins=8, exposure=0.64, max_bounces=6, sqrt_spp=8)
+    film = S.cornell(width=256, height=256, time_bins=1400, exposure=0.01, sqrt_spp=1, max_bounces=2)    # 2.2 GB
+    _abi.check(_abi.lib().tr_release_cached_memory(0))
+    with gpu.Context(sc) as a:
+        a.render(0, 64)                                      # two batches of 8 M slots: 3.7 GB
+        with _only(1000 * MB, release=False):
+            with gpu.Context(film) as ctx:
+                ctx.render(0, 1)
+                assert (ctx.film(streak=False)["weight"] == 1).all()
+        a.render(64, 64)
+        assert (a.film()["weight"] == 128).all()
