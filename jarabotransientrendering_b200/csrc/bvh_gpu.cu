@@ -901,7 +901,7 @@ bool build_bvh_device(const float* d_v, uint32_t nv, const uint32_t* d_t, uint32
     TR_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
     void* block = nullptr;
     TR_CUDA(tri::pool_malloc(&block, carve(nullptr), s));
-    struct Free { void* p; cudaStream_t s; ~Free() { cudaFreeAsync(p, s); } } release{block, s};
+    struct Free { void* p; cudaStream_t s; ~Free() { tri::pool_free_after(p, s); } } release{block, s};
     carve(static_cast<char*>(block));
 
     uint32_t h[kCounters];

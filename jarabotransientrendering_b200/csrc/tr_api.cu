@@ -14,6 +14,7 @@
 #include <new>
 #include <stdexcept>
 #include <string>
+#include <unordered_map>
 #include <vector>
 
 #include "bvh_build.h"
@@ -123,12 +124,14 @@ void upload(void* dst, const void* src, size_t bytes, cudaStream_t s) {
 
 namespace tri {
 
+static size_t pool_index(int device, Pool which) { return 2 * (size_t)device + (which == Pool::kLarge ? 1u : 0u); }
+
 cudaMemPool_t device_pool(int device, Pool which) {
     static std::mutex mu;
     static std::vector<cudaMemPool_t> pools;
     std::lock_guard<std::mutex> lock(mu);
     if (device < 0) throw CudaError(cudaErrorInvalidDevice, "device_pool");
-    const size_t at = 2 * (size_t)device + (which == Pool::kLarge ? 1u : 0u);
+    const size_t at = pool_index(device, which);
     if (at >= pools.size()) pools.resize(at + 1, nullptr);
     if (!pools[at]) {
         cudaMemPoolProps props{};
@@ -144,12 +147,38 @@ cudaMemPool_t device_pool(int device, Pool which) {
     return pools[at];
 }
 
+namespace {
+// blocks of the pools in use, and their bytes per pool (pool_index); never destroyed: contexts that a program
+// keeps to its end are
+struct Blocks {
+    struct Block { size_t bytes, pool; };
+    std::mutex mu;
+    std::unordered_map<void*, Block> at;
+    std::vector<size_t> in_use;
+};
+Blocks& blocks() {
+    static Blocks* const b = new Blocks;
+    return *b;
+}
+
+void forget_block(void* p) {
+    Blocks& b = blocks();
+    std::lock_guard<std::mutex> lock(b.mu);
+    const auto it = b.at.find(p);
+    if (it == b.at.end()) return;
+    b.in_use[it->second.pool] -= it->second.bytes;
+    b.at.erase(it);
+}
+}  // namespace
+
 size_t pool_idle_bytes(int device, Pool which) {
-    uint64_t reserved = 0, used = 0;
-    cudaMemPool_t pool = device_pool(device, which);
-    if (cudaMemPoolGetAttribute(pool, cudaMemPoolAttrReservedMemCurrent, &reserved) != cudaSuccess) return 0;
-    if (cudaMemPoolGetAttribute(pool, cudaMemPoolAttrUsedMemCurrent, &used) != cudaSuccess) return 0;
-    return reserved > used ? (size_t)(reserved - used) : 0;
+    uint64_t reserved = 0;
+    if (cudaMemPoolGetAttribute(device_pool(device, which), cudaMemPoolAttrReservedMemCurrent, &reserved) != cudaSuccess) return 0;
+    const size_t at = pool_index(device, which);
+    Blocks& b = blocks();
+    std::lock_guard<std::mutex> lock(b.mu);
+    const size_t used = at < b.in_use.size() ? b.in_use[at] : 0;
+    return reserved > used ? (size_t)reserved - used : 0;
 }
 
 cudaError_t pool_malloc(void** p, size_t bytes, cudaStream_t s, Pool which) {
@@ -162,7 +191,26 @@ cudaError_t pool_malloc(void** p, size_t bytes, cudaStream_t s, Pool which) {
         cudaMemPoolTrimTo(device_pool(dev, Pool::kLarge), 0);       // what it keeps is free memory
         e = cudaMallocFromPoolAsync(p, bytes, device_pool(dev, which), s);
     }
+    if (e != cudaSuccess) return e;
+    const size_t at = pool_index(dev, which);
+    Blocks& b = blocks();
+    std::lock_guard<std::mutex> lock(b.mu);
+    if (at >= b.in_use.size()) b.in_use.resize(at + 1, 0);
+    b.in_use[at] += bytes;
+    b.at[*p] = {bytes, at};
     return e;
+}
+
+void pool_free(void* p) {
+    if (!p) return;
+    forget_block(p);                             // before another thread can be given the address
+    cudaFree(p);
+}
+
+void pool_free_after(void* p, cudaStream_t s) {
+    if (!p) return;
+    forget_block(p);
+    if (cudaFreeAsync(p, s) != cudaSuccess) cudaFree(p);
 }
 
 // Memory kept by the pools goes back to the driver (nothing where there are none).
@@ -171,13 +219,6 @@ static void trim_pools(int device) noexcept {
         for (Pool which : {Pool::kKept, Pool::kLarge}) cudaMemPoolTrimTo(device_pool(device, which), 0);
     } catch (const CudaError&) {
     }
-}
-
-void dfree(const std::vector<void*>& blocks) {
-    cudaDeviceSynchronize();
-    for (void* p : blocks)
-        if (p) cudaFreeAsync(p, 0);
-    cudaStreamSynchronize(0);                    // back in the pool, for every stream
 }
 
 size_t carve_wave(trk::Wave* w, void* block, uint32_t capacity, size_t R, bool time_sampling) {
@@ -1619,7 +1660,7 @@ extern "C" tr_status tr_guide_create(int device, uint64_t seed, tr_guide** out) 
         TR_CUDA(trg::pack_weights(g->params, g->w_fwd, g->w_bwd, g->stream));
         TR_CUDA(cudaStreamSynchronize(g->stream));
     } catch (const CudaError& e) {
-        dfree(g->allocs);
+        for (void* q : g->allocs) pool_free(q);
         delete g;
         return fail(TR_ERR_CUDA, e.what());
     }
@@ -1724,7 +1765,7 @@ extern "C" tr_status tr_guide_destroy(tr_guide* g) {
     if (!g) return TR_OK;
     cudaSetDevice(g->device);
     if (g->stream) cudaStreamSynchronize(g->stream);
-    dfree(g->allocs);
+    for (void* q : g->allocs) pool_free(q);
     if (g->stream) cudaStreamDestroy(g->stream);
     delete g;
     return TR_OK;

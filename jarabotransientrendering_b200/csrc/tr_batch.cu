@@ -77,7 +77,7 @@ struct tr_batch {
     template <class T>
     void drop(T*& p) {
         if (!p) return;
-        tri::dfree(p);
+        tri::pool_free(p);
         allocs.erase(std::remove(allocs.begin(), allocs.end(), (void*)p), allocs.end());
         p = nullptr;
     }
@@ -446,7 +446,7 @@ tr_status tr_batch_create(tr_ctx* const* contexts, uint32_t n, tr_batch** out) {
         b->trace_grid = trk::trace_grid_size(b->device, b->bvh_depth, true);
         b->stats.device_bytes = b->bytes;
     } catch (const CudaError& e) {
-        dfree(b->allocs);
+        for (void* p : b->allocs) pool_free(p);
         for (cudaEvent_t e : b->dep)
             if (e) cudaEventDestroy(e);
         if (b->shadow_stream) cudaStreamDestroy(b->shadow_stream);
@@ -586,7 +586,7 @@ tr_status tr_batch_destroy(tr_batch* b) {
     cudaSetDevice(b->device);
     if (b->stream) cudaStreamSynchronize(b->stream);
     b->drop_graph();
-    dfree(b->allocs);
+    for (void* p : b->allocs) pool_free(p);
     if (b->ev0) cudaEventDestroy(b->ev0);
     if (b->ev1) cudaEventDestroy(b->ev1);
     for (cudaEvent_t e : b->dep)

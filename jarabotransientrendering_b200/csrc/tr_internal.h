@@ -47,6 +47,11 @@ cudaMemPool_t device_pool(int device, Pool which = Pool::kKept);
 size_t pool_idle_bytes(int device, Pool which);
 // cudaMallocFromPoolAsync on stream s, from the current device's pool
 cudaError_t pool_malloc(void** p, size_t bytes, cudaStream_t s, Pool which = Pool::kKept);
+// Gives p back to its pool: by cudaFree, which waits for the device (any stream may have used it), or in the order
+// of stream s.  Both keep the count of what is in use: the pool's own goes on counting what cudaFree returned
+// (and freeing in stream order after a wait for the device would end the graph captures of other threads).
+void pool_free(void* p);
+void pool_free_after(void* p, cudaStream_t s);
 
 template <class T>
 T* dalloc(size_t count, size_t& total, Pool which = Pool::kKept) {
@@ -58,12 +63,6 @@ T* dalloc(size_t count, size_t& total, Pool which = Pool::kKept) {
     total += count * sizeof(T);
     return static_cast<T*>(p);
 }
-
-// Gives memory of the current device back to the pool it came from once the device is idle (any stream may have used it).
-// In stream order, not by cudaFree: what that returns the pool can hand out again but goes on counting as used,
-// and pool_idle_bytes would miss it.
-void dfree(const std::vector<void*>& blocks);
-inline void dfree(void* p) { dfree(std::vector<void*>{p}); }
 
 constexpr uint32_t kMaxBounces = 63;            // counters hold 64 depths
 constexpr uint32_t kDefaultCapacity = 1u << 21; // path slots per wavefront batch
@@ -116,7 +115,7 @@ struct tr_guide {
     }
     void drop(void* p) {
         if (!p) return;
-        tri::dfree(p);
+        tri::pool_free(p);
         allocs.erase(std::remove(allocs.begin(), allocs.end(), p), allocs.end());
     }
     trg::GuideDev dev() const {
@@ -253,7 +252,8 @@ struct tr_ctx {
         if (!p) return;
         const auto it = std::find_if(allocs.begin(), allocs.end(), [&](const Alloc& a) { return a.p == p; });
         if (it != allocs.end()) {
-            if (!after || cudaFreeAsync(p, after) != cudaSuccess) tri::dfree(p);
+            if (after) tri::pool_free_after(p, after);
+            else tri::pool_free(p);
             bytes -= it->bytes;
             allocs.erase(it);
         }
@@ -282,9 +282,7 @@ struct tr_ctx {
         }
         if (light_stream) cudaStreamDestroy(light_stream);
         shadow_stream = light_stream = nullptr;
-        std::vector<void*> blocks;
-        for (const Alloc& a : allocs) blocks.push_back(a.p);
-        tri::dfree(blocks);
+        for (const Alloc& a : allocs) tri::pool_free(a.p);
         allocs.clear();
         if (ev0) cudaEventDestroy(ev0);
         if (ev1) cudaEventDestroy(ev1);

@@ -215,3 +215,32 @@ def test_idle_large_batches_count_as_free(gpu):
                 assert (ctx.film(streak=False)["weight"] == 1).all()
         a.render(64, 64)
         assert (a.film()["weight"] == 128).all()
+
+
+def test_contexts_are_destroyed_while_another_thread_captures(gpu):
+    """Giving memory back waits for the device without disturbing a graph that another thread is capturing."""
+    import threading
+    import torch
+    sc = S.cornell(width=64, height=64, time_bins=64, exposure=0.08, max_bounces=3, sqrt_spp=4)
+    g, x = R.Guide(device=0, seed=1), torch.zeros(1024, device="cuda")
+    ctx = gpu.Context(sc)
+    ctx.render(0, sc.spp)
+    torch.cuda.synchronize()
+    graph, side = torch.cuda.CUDAGraph(), torch.cuda.Stream()
+
+    def destroy():
+        ctx.close()
+        g.close()
+
+    with torch.cuda.stream(side):
+        graph.capture_begin(capture_error_mode="thread_local")
+        x += 1
+        t = threading.Thread(target=destroy)
+        t.start()
+        t.join()
+        x += 1
+        graph.capture_end()
+    for _ in range(3):
+        graph.replay()
+    torch.cuda.synchronize()
+    assert (x == 6).all()
