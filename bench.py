@@ -28,13 +28,13 @@ sys.path.insert(0, ROOT)
 B_CLOSEST = 48 + 64 * 19.397909840536915 + 48 * 8.579641797558255     # 1701.3 B
 B_SHADOW = 48 + 64 * 16.98375084460311 + 48 * 6.767252594318216       # 1459.8 B
 # DRAM bytes per closest-hit query of k_extend, from one ncu capture of all eight k_extend
-# launches of the 2M-path icosphere case (same 2^21-slot batches as this workload):
-# (425,001,984 B read + 36,808,704 B written) / 4,550,499 queries -- the BVH stays in L2, DRAM
-# carries the ray records.  Scaled to this workload's mean launch for roofline.traffic.
-DRAM_BYTES_PER_CLOSEST_QUERY = (425001984 + 36808704) / 4550499
-# The same for k_shadow (all eight launches of the same case): (234,519,552 B read + 23,867,904 B
+# launches of the 2M-path icosphere case: (409,113,856 B read + 11,821,824 B written) / 4,550,499
+# queries -- the BVH stays in L2, DRAM carries the ray records.  Scaled to this workload's mean
+# launch (batches of 2^23 slots, whose records stay in L2 no better) for roofline.traffic.
+DRAM_BYTES_PER_CLOSEST_QUERY = (409113856 + 11821824) / 4550499
+# The same for k_shadow (all eight launches of the same case): (232,784,384 B read + 18,305,536 B
 # written) / 3,177,936 any-hit queries.
-DRAM_BYTES_PER_SHADOW_QUERY = (234519552 + 23867904) / 3177936
+DRAM_BYTES_PER_SHADOW_QUERY = (232784384 + 18305536) / 3177936
 
 WORKLOAD = "icosphere"
 # throughput (value, paths/s) plus the "convergence" object: time to 5% rel-L2, guided vs plain
@@ -65,6 +65,8 @@ def parse():
     ap.add_argument("--case-repeat", type=int, default=1)
     ap.add_argument("--case-width", type=int, default=0)
     ap.add_argument("--case-height", type=int, default=0)
+    ap.add_argument("--case-apart", action="store_true",
+                    help="per-kernel timing on: the per-depth kernels also where one launch walks whole paths")
     ap.add_argument("--case-guided", action="store_true")
     ap.add_argument("--case-mix", type=float, default=0.7)
     ap.add_argument("--case-train-pool", type=int, default=0)
@@ -82,7 +84,7 @@ def profile_case(a):
     (8192 pixels x 256 paths) and a 0.4 GB film.  `--case-guided` attaches a learned proposal
     (orthonormal shading frames, mixture probability `--case-mix`); with `--case-train-pool 0`
     the network stays at its seeded initialisation, otherwise it trains after every pass."""
-    from jarabotransientrendering_b200 import scenes as S
+    from jarabotransientrendering_b200 import _abi, scenes as S
     from jarabotransientrendering_b200.renderer import Context, Guide
     sc = S.WORKLOADS[a.case]()
     sc.exposure = sc.exposure * sc.time_bins / a.case_bins
@@ -96,6 +98,8 @@ def profile_case(a):
         sc.flags |= S.FLAG_ORTHONORMAL_FRAME
         guide = Guide(seed=1)
     with Context(sc) as ctx:
+        if a.case_apart:
+            _abi.check(_abi.lib().tr_set_profiling(ctx.h, 1))
         if guide is not None:
             ctx.set_guide(guide, mix_prob=a.case_mix, learning_rate=3e-3, train_pool=a.case_train_pool)
         for r in range(a.case_repeat):
