@@ -244,3 +244,34 @@ def test_contexts_are_destroyed_while_another_thread_captures(gpu):
         graph.replay()
     torch.cuda.synchronize()
     assert (x == 6).all()
+
+
+def test_large_renders_of_several_threads(gpu):
+    """Threads whose contexts take and return large batches at once, one on a stream of its caller's, with small
+    renders between: the films of the same renders one after another."""
+    import threading
+    import torch
+    scenes = [S.cornell(width=512, height=512, time_bins=8, exposure=0.64, max_bounces=3, sqrt_spp=8, seed=k + 1)
+              for k in range(3)]
+
+    def work(k, films, stream=None):
+        with gpu.Context(scenes[k]) as ctx:
+            if stream is not None:
+                _abi.check(_abi.lib().tr_set_stream(ctx.h, stream.cuda_stream))
+            for first, count in ((0, 32), (32, 2), (34, 64), (98, 1)):
+                ctx.render(first, count)
+            films[k] = ctx.film()
+
+    one, many = [None] * 3, [None] * 3
+    for k in range(3):
+        work(k, one)
+    side = torch.cuda.Stream()
+    threads = [threading.Thread(target=work, args=(k, many, side if k == 1 else None)) for k in range(3)]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    for a, b in zip(one, many):
+        assert (a["weight"] == 99).all() and (b["weight"] == 99).all()
+        for k in a:
+            assert np.allclose(a[k], b[k], rtol=1e-12, atol=0.0), k
