@@ -936,9 +936,10 @@ tr_status tr_create(const tr_scene* s, const tr_camera* c, const tr_film* f, con
         // earlier context is reused whole instead of mapped again)
         const size_t nstreak = (size_t)f->width * f->height * f->time_bins * 3u;
         const size_t nb = f->bounce_films;
-        // Refused unless it leaves the path state its share, before anything is taken.  The query takes
-        // 0.2 ms: left out where the pool alone holds all that, and put off for films below 32 MB (what the
-        // pool grows by anyway) until the scene's uploads are under way.
+        // Refused unless it leaves the path state its share, before anything is taken of the device's free
+        // memory.  The query takes 0.2 ms: left out where the pool alone holds film and share, and put off until
+        // the film is being cleared and the scene uploaded where the pool holds the film (0.4 GB 550 -> 520 us,
+        // 0.8 GB 620 -> 540) or it is below 32 MB, what the pool grows by anyway.
         const size_t film_bytes = (1 + nb) * nstreak * sizeof(double);
         auto refuse_film = [&] {
             // kept by the pools for reuse
@@ -955,7 +956,7 @@ tr_status tr_create(const tr_scene* s, const tr_camera* c, const tr_film* f, con
             return fail(TR_ERR_OUT_OF_MEMORY, "streak film of " + std::to_string(nstreak * 8 >> 20) +
                                                   " MiB does not fit in free device memory");
         };
-        const bool check_late = film_bytes < ((size_t)32 << 20);
+        const bool check_late = film_bytes < std::max((size_t)32 << 20, tri::pool_idle_bytes(device, Pool::kKept));
         if (!check_late && refuse_film()) return refused();
         x->d_streak = x->alloc<double>(nstreak);
         if (nb) x->d_bstreak = x->alloc<double>(nb * nstreak);
